@@ -1,0 +1,280 @@
+// attn_tiles.cuh -- attention of many query rows (prompts and long portions) in f32 on CUDA cores, as two register-tiled
+// products per key tile.  Same parameters and arithmetic rules as attn_rows_kernel (dense_ops.cuh), which serves steps of one
+// or a few rows.
+#pragma once
+#include "dense_ops.cuh"
+
+namespace lmrs {
+namespace dense {
+
+// What bounds it: the FMA pipe and the issue slots.  A (query row, key) pair costs dk + dv multiply-adds and nothing else of that
+// size; at 148 SMs x 128 lanes a prompt of 2048 tokens with 24 heads of 128 cannot take less than 346 us.  attn_rows_kernel gives a
+// lane two keys and a warp 4 or 8 rows, so that every 16 bytes it reads from shared memory feed few multiply-adds: 1731 us there, 830
+// here (512 tokens, 32 heads of 64: 142 us and 74).  What is left is latency: registers allow two or three warps per scheduler.
+// Here a CTA owns 64 rows (tokens x grouped heads of one KV head) against 64 keys, a warp 16 of the rows,
+// and a thread 4 rows x 8 keys of the scores, then 4 rows x 8 NV columns of the output: a 16-byte read of q or k feeds 16 or 32
+// multiply-adds.  (8 rows x 4 keys costs as many reads but leaves a row to 16 lanes instead of 8, twice the work per row:
+// 953 us against 877 us.)
+//   scores   packed f32x2 multiply-adds over (even, odd) positions of the head dimension -- both operands are pairs as they lie in
+//            shared memory -- which also halves the issue slots, leaving room for the loads and the softmax of the other warps
+//            (scalar multiply-adds: 949 us)
+//   weights  in powers of two: scores are scaled by log2(e) with the scale itself
+//   values   packed over two neighbouring output columns, the probability duplicated into a pair (scalar: 1013 us)
+// Shared memory holds q, k and probability rows unpadded, 16-byte pieces rotated by the row (xor with row & 7): the lanes that
+// read 8 key rows, or 4 query rows, at the same dimension meet no bank twice.  Unpadded rows are what lets two
+// CTAs with 128-wide heads share an SM (114,688 bytes each); with 64-wide heads it is three.  K of the next tile is
+// copied while this tile's values are summed, V while the scores are.  A warp's rows belong to it alone, so the
+// probabilities need no barrier of their own.
+constexpr int TA_ROWS = 64, TA_KEYS = 64, TA_THREADS = 128;
+inline int attn_tile_pitch(int dk) { return (dk + 31) & ~31; }
+inline size_t attn_tile_smem(int dk, int dv, bool v_in_k) {
+    const size_t qs = attn_tile_pitch(dk), vs = v_in_k ? 0 : (dv <= 64 ? 64 : 128);
+    return ((size_t)TA_ROWS * qs + (size_t)TA_KEYS * (qs + vs) + (size_t)TA_ROWS * TA_KEYS) * 4;
+}
+typedef unsigned long long f32pair;
+DN_DEVINL void fma2(f32pair& acc, f32pair a, f32pair b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
+DN_DEVINL f32pair mul2(f32pair a, f32pair b) { f32pair r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+DN_DEVINL f32pair dup2(float v) { f32pair r; asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v)); return r; }
+DN_DEVINL float2 unpack2(f32pair v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
+DN_DEVINL float ex2(float v) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v)); return r; }
+DN_DEVINL float lg2(float v) { float r; asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v)); return r; }
+
+// NV: 64-column blocks of the values.  SIG: sigmoid weights (attn_rows_kernel).  VK: the values are the first dv entries of the K
+// rows (p.v_in_k): no V tile, and the next K tile is copied after the values instead of under them.  QS: the pitch of the q and k
+// rows in shared memory (0: any, from dk; a pitch known here leaves the inner loop without address arithmetic).
+template <typename AT, int NV, int QS, bool SIG, bool VK>
+static __global__ void __launch_bounds__(TA_THREADS, NV == 1 ? 3 : 2) attn_tile_kernel(const AttnRowsParams<AT> p) {
+    extern __shared__ __align__(16) float ta_sm[];
+    constexpr int VS = 64 * NV;
+    const int qs = QS ? QS : (p.dk + 31) & ~31, d4 = (p.dk + 3) & ~3;
+    float* Qs = ta_sm;                       // [64][qs]
+    float* Ks = Qs + TA_ROWS * qs;           // [64][qs]
+    float* Vs = Ks + TA_KEYS * qs;           // [64][VS], not rotated
+    float* Ps = VK ? Vs : Vs + TA_KEYS * VS; // [64][64]
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int cg = lane & 7, rq = lane >> 3, rg = warp * 16 + rq;   // this thread's keys cg + 8 j, its rows rg + 4 i
+    const int kv_mul = p.H / p.G, chunks = (kv_mul + p.HC - 1) / p.HC;
+    const int g = blockIdx.x / chunks, h0 = (blockIdx.x % chunks) * p.HC;
+    const int t0 = (int)(gridDim.y - 1 - blockIdx.y) * p.TQ;   // late query tiles see the most keys: they are scheduled first
+    const uint32_t pos0 = pos_of(p.ps);
+    const int t_last = min(p.T, t0 + p.TQ) - 1;
+    const int n_keys = (int)pos0 + t_last + 1;
+    // the walk over the key tiles: as in attn_rows_kernel
+    const int n_tiles = (n_keys + TA_KEYS - 1) / TA_KEYS;
+    const int first_tile = p.window > 0 ? max(0, (int)pos0 + t0 - p.window + 1) / TA_KEYS
+                           : p.chunk > 0 ? ((int)pos0 + t0) / p.chunk * p.chunk / TA_KEYS : 0;
+    const int kf_tiles = p.window > 0 && p.keep_first > 0 ? min(first_tile, (p.keep_first + TA_KEYS - 1) / TA_KEYS) : 0;
+    const int n_walk = kf_tiles + n_tiles - first_tile;
+    auto tile_of = [&](int u) { return u < kf_tiles ? u : first_tile + (u - kf_tiles); };
+
+    // 64 rows of `cols` floats (a last partial 16-byte piece is filled with zeros; rows >= valid are zeros), `ld` floats apart, into
+    // shared memory; a thread's pieces are 128 apart
+    auto copy_rows = [&](float* dst, int pitch, int rot, int cols, const float* src, int ld, int valid) {
+        const int pieces = (cols + 3) >> 2, dr = TA_THREADS / pieces, dc = TA_THREADS - dr * pieces;
+        int r = (int)threadIdx.x / pieces, c = (int)threadIdx.x - r * pieces;
+        src += (size_t)r * ld;
+        while (r < 64) {
+            float* d = dst + r * pitch + ((c ^ (r & rot)) << 2);
+            if (p.async) {
+                cp_async16_zfill(d, r < valid ? src + 4 * c : p.kcache, r < valid);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; e++) d[e] = r < valid && 4 * c + e < cols ? src[4 * c + e] : 0.0f;
+            }
+            r += dr; c += dc; src += (size_t)dr * ld;
+            if (c >= pieces) { c -= pieces; r++; src += ld; }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto load_k = [&](int tile) {
+        const int j0 = tile * TA_KEYS;
+        copy_rows(Ks, qs, 7, p.dk, p.kcache + (size_t)j0 * p.k_ld + (size_t)g * p.dk, p.k_ld, n_keys - j0);
+    };
+    auto load_v = [&](int tile) {
+        const int j0 = tile * TA_KEYS;
+        copy_rows(Vs, VS, 0, p.dv, p.vcache + (size_t)j0 * p.v_ld + (size_t)g * p.dv, p.v_ld, n_keys - j0);
+    };
+    pdl_launch();
+    pdl_wait();
+    for (int e = threadIdx.x; e < TA_ROWS * (d4 >> 2); e += TA_THREADS) {
+        const int r = e / (d4 >> 2), c = e - r * (d4 >> 2);
+        const int t = t0 + r / p.HC, hl = h0 + r % p.HC;
+        const bool ok = r / p.HC < p.TQ && t < p.T && hl < kv_mul;
+        const float* src = p.q + ((size_t)t * p.H + g * kv_mul + hl) * p.dk + 4 * c;
+        float* d = Qs + r * qs + ((c ^ (r & 7)) << 2);
+        if (p.async) {
+            cp_async16_zfill(d, ok ? src : p.q, ok);
+        } else {
+            for (int x = 0; x < 4; x++) d[x] = ok && 4 * c + x < p.dk ? src[x] : 0.0f;
+        }
+    }
+    load_k(tile_of(0));
+    if (!VK) {   // value columns beyond dv take part in the sums (their results are not stored): zero once
+        const int v4 = (p.dv + 3) & ~3;
+        for (int e = threadIdx.x; e < TA_KEYS * (VS - v4); e += TA_THREADS) Vs[(e / (VS - v4)) * VS + v4 + e % (VS - v4)] = 0.0f;
+    }
+
+    constexpr float LOG2E = 1.4426950408889634f;
+    float m[4], l[4];   // running maximum (of scores * log2(e)) and this lane's share of the sum
+    f32pair o[4][4 * NV];
+    int last[4];        // last visible key of row i (-1: no such row)
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int r = rg + 4 * i, t = t0 + r / p.HC, hl = h0 + r % p.HC;
+        const bool ok = r / p.HC < p.TQ && t < p.T && hl < kv_mul;
+        last[i] = ok ? (int)pos0 + t : -1;
+        m[i] = !SIG && p.sink && ok ? p.sink[g * kv_mul + hl] * LOG2E : -1e30f;
+        l[i] = (SIG || (p.sink && ok)) && cg == 0 ? 1.0f : 0.0f;
+#pragma unroll
+        for (int c = 0; c < 4 * NV; c++) o[i][c] = 0ull;
+    }
+    const float scale2 = p.scale * LOG2E, cap2 = p.softcap * LOG2E;
+    const float to_cap = p.softcap > 0.0f ? 2.0f / p.softcap * scale2 : 0.0f;   // e^(2 s scale / cap) as a power of two
+    const int t_first_last = (int)pos0 + t0, t_last_last = (int)pos0 + t_last;   // last visible keys of the CTA's first and last row
+
+    for (int u = 0; u < n_walk; u++) {
+        const int j0 = tile_of(u) * TA_KEYS;
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();   // K (and Q) of this tile are here; everyone is done with the previous V tile
+        if (!VK) load_v(tile_of(u));
+        // ---- scores
+        f32pair s2[4][8];
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 8; j++) s2[i][j] = 0ull;
+        {
+            const float* qp = Qs + rg * qs;
+            const float* kp = Ks + cg * qs;
+#pragma unroll 1
+            for (int d = 0; d < d4; d += 4) {
+                const int dq = d ^ (rq << 2), dk = d ^ (cg << 2);
+                ulonglong2 kv[8], qv[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) qv[i] = *reinterpret_cast<const ulonglong2*>(qp + i * 4 * qs + (i & 1 ? dq ^ 16 : dq));
+#pragma unroll
+                for (int j = 0; j < 8; j++) kv[j] = *reinterpret_cast<const ulonglong2*>(kp + j * 8 * qs + dk);
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+#pragma unroll
+                    for (int i = 0; i < 4; i++) fma2(s2[i][j], qv[i].x, kv[j].x);
+#pragma unroll
+                    for (int i = 0; i < 4; i++) fma2(s2[i][j], qv[i].y, kv[j].y);
+                }
+            }
+        }
+        // ---- weights
+        // every row sees every key of the tile? (rows that do not exist score zeros and are never stored)
+        const bool full = j0 + TA_KEYS - 1 <= t_first_last && (p.window <= 0 || t_last_last - j0 < p.window) && (p.chunk <= 0 || j0 >= t_last_last / p.chunk * p.chunk);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int r = rg + 4 * i;
+            float* prow = Ps + r * TA_KEYS + (cg & 3);
+            float a[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) { const float2 s = unpack2(s2[i][j]); a[j] = s.x + s.y; }
+            if (SIG) {
+                const float b = last[i] >= 0 ? p.wbias[g * kv_mul + h0 + r % p.HC] : 0.0f;
+#pragma unroll
+                for (int j = 0; j < 8; j++) a[j] = att_sigmoid(a[j] * p.scale + b);
+            } else {
+                if (p.softcap > 0.0f) {
+#pragma unroll
+                    for (int j = 0; j < 8; j++) a[j] = fmaf(-2.0f * cap2, __fdividef(1.0f, ex2(a[j] * to_cap) + 1.0f), cap2);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 8; j++) a[j] *= scale2;
+                }
+                if (p.r1) {
+                    const int h = g * kv_mul + min(h0 + r % p.HC, kv_mul - 1);
+                    const float p1 = p.r1[h], p2 = p.r2[h];
+#pragma unroll
+                    for (int j = 0; j < 8; j++) a[j] -= p1 * lg2(1.0f + p2 * (float)max(last[i] - (j0 + cg + 8 * j), 0));
+                }
+            }
+            uint32_t hidden = 0;   // bit j: key cg + 8 j is not visible to this row
+            if (!full) {
+                const int first = p.chunk > 0 ? last[i] / p.chunk * p.chunk : 0;
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const int key = j0 + cg + 8 * j, dist = last[i] - key;
+                    const bool vis = dist >= 0 && key >= first && (p.window <= 0 || dist < p.window || key < p.keep_first);
+                    if (!vis) { hidden |= 1u << j; a[j] = SIG ? 0.0f : -1e30f; }
+                }
+            }
+            if (!SIG) {
+                float mt = fmaxf(fmaxf(fmaxf(a[0], a[1]), fmaxf(a[2], a[3])), fmaxf(fmaxf(a[4], a[5]), fmaxf(a[6], a[7])));
+#pragma unroll
+                for (int x = 4; x > 0; x >>= 1) mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, x));
+                const float mn = fmaxf(m[i], mt);
+#pragma unroll
+                for (int j = 0; j < 8; j++) a[j] = ex2(a[j] - mn);
+                if (!full)   // a row that has not met a visible key yet: its hidden keys score the maximum
+#pragma unroll
+                    for (int j = 0; j < 8; j++) a[j] = hidden >> j & 1 ? 0.0f : a[j];
+                const float corr = ex2(m[i] - mn);
+                l[i] = l[i] * corr + (((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7])));
+                m[i] = mn;
+                const f32pair c2 = dup2(corr);
+#pragma unroll
+                for (int c = 0; c < 4 * NV; c++) o[i][c] = mul2(o[i][c], c2);
+            }
+#pragma unroll
+            for (int j = 0; j < 8; j++) prow[(((cg >> 2) + 2 * j) ^ (r & 7)) << 2] = a[j];
+        }
+        if (!VK) {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncthreads();   // V is here; everyone is done with K
+            if (u + 1 < n_walk) load_k(tile_of(u + 1));
+        } else {
+            __syncwarp();
+        }
+        // ---- values: columns 4 cg .. 4 cg + 3 of every 32-column block
+        const float* pp = Ps + rg * TA_KEYS;
+#pragma unroll 1
+        for (int j = 0; j < TA_KEYS; j += 4) {
+            float4 pv[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) pv[i] = *reinterpret_cast<const float4*>(pp + i * 4 * TA_KEYS + (j ^ ((i & 1 ? rq ^ 4 : rq) << 2)));
+#pragma unroll
+            for (int jj = 0; jj < 4; jj++) {
+                ulonglong2 vv[2 * NV];
+#pragma unroll
+                for (int b = 0; b < 2 * NV; b++)
+                    vv[b] = VK ? *reinterpret_cast<const ulonglong2*>(Ks + (j + jj) * qs + (((8 * b + cg) ^ ((j + jj) & 7)) << 2))
+                               : *reinterpret_cast<const ulonglong2*>(Vs + (j + jj) * VS + 32 * b + 4 * cg);
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const f32pair p2 = dup2(jj == 0 ? pv[i].x : jj == 1 ? pv[i].y : jj == 2 ? pv[i].z : pv[i].w);
+#pragma unroll
+                    for (int b = 0; b < 2 * NV; b++) { fma2(o[i][2 * b], p2, vv[b].x); fma2(o[i][2 * b + 1], p2, vv[b].y); }
+                }
+            }
+        }
+        if (VK) {
+            __syncthreads();   // everyone is done with K
+            if (u + 1 < n_walk) load_k(tile_of(u + 1));
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        float ls = l[i];
+#pragma unroll
+        for (int x = 4; x > 0; x >>= 1) ls += __shfl_xor_sync(0xffffffffu, ls, x);
+        if (last[i] < 0) continue;
+        const int r = rg + 4 * i, t = t0 + r / p.HC, h = g * kv_mul + h0 + r % p.HC;
+        const float inv = (p.gate ? p.gate[(size_t)t * p.H + h] : 1.0f) * p.out_scale / ls;
+        AT* dst = p.out + (size_t)t * p.out_ld + (size_t)h * p.dv;
+        const float* gl = p.gate_logits ? p.gate_logits + (size_t)t * p.gate_ld + (size_t)h * p.dv : nullptr;
+#pragma unroll
+        for (int c = 0; c < 4 * NV; c++) {
+            const float2 v = unpack2(o[i][c]);
+            const int col = 32 * (c >> 1) + 4 * cg + 2 * (c & 1);
+            if (col < p.dv) from_f(dst[col], gl ? v.x * inv / (1.0f + expf(-gl[col])) : v.x * inv);
+            if (col + 1 < p.dv) from_f(dst[col + 1], gl ? v.y * inv / (1.0f + expf(-gl[col + 1])) : v.y * inv);
+        }
+    }
+}
+
+}  // namespace dense
+}  // namespace lmrs

@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "arch.h"
+#include "attn_tiles.cuh"
 #include "dense_gemm.cuh"
 #include "dense_ops.cuh"
 #include "safetensors.h"
@@ -349,15 +350,22 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
         if (ni <= 1) return launch_attn_t<RW, 1, SIG>(st, p, gx, gy);
         if (ni <= 2) return launch_attn_t<RW, 2, SIG>(st, p, gx, gy);
         if (ni <= 4) return launch_attn_t<RW, 4, SIG>(st, p, gx, gy);
-        if constexpr (RW <= 4) {
-            if constexpr (!SIG) {
-                if (ni > 8) return launch_attn_t<RW, 16, SIG>(st, p, gx, gy);   // only a shared latent head is as wide
-            }
-            return launch_attn_t<RW, 8, SIG>(st, p, gx, gy);
-        } else {
-            error = "attention: no wide-tile kernel for this value size";
-            return 1;
+        if constexpr (!SIG) {
+            if (ni > 8) return launch_attn_t<RW, 16, SIG>(st, p, gx, gy);   // only a shared latent head is as wide
         }
+        return launch_attn_t<RW, 8, SIG>(st, p, gx, gy);
+    }
+    template <bool SIG> int launch_attn_tiles(cudaStream_t st, AttnRowsParams<AT> p, int gx) {
+        p.async = p.dk % 4 == 0 && p.dv % 4 == 0 && p.k_ld % 4 == 0 && p.v_ld % 4 == 0;
+        const size_t smem = attn_tile_smem(p.dk, p.dv, p.v_in_k);
+        const dim3 grid(gx, (p.T + p.TQ - 1) / p.TQ);
+        auto go = [&](auto kernel) { return optin(kernel, smem) || launch_k("attn_tile_kernel", st, pdl_now, kernel, grid, dim3(TA_THREADS), smem, p); };
+        if constexpr (!SIG) {
+            if (p.v_in_k) return p.dv <= 64 ? go(attn_tile_kernel<AT, 1, 0, SIG, true>) : go(attn_tile_kernel<AT, 2, 0, SIG, true>);
+        }
+        const int pitch = attn_tile_pitch(p.dk);
+        if (p.dv <= 64) return pitch == 64 ? go(attn_tile_kernel<AT, 1, 64, SIG, false>) : pitch == 128 ? go(attn_tile_kernel<AT, 1, 128, SIG, false>) : go(attn_tile_kernel<AT, 1, 0, SIG, false>);
+        return pitch == 128 ? go(attn_tile_kernel<AT, 2, 128, SIG, false>) : pitch == 96 ? go(attn_tile_kernel<AT, 2, 96, SIG, false>) : go(attn_tile_kernel<AT, 2, 0, SIG, false>);
     }
     // attention over T query rows: the caller fills the tensors, head geometry, pitches, scale, soft-cap, window, kept first keys,
     // sink, gates and penalty;
@@ -377,12 +385,13 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
         // a one-row step over few KV heads: fewer query heads per CTA, so that more SMs share the keys
         while (T == 1 && p.HC > 4 && p.G * ((kv_mul + p.HC - 1) / p.HC) * tiles < sms) p.HC /= 2;
         const int chunks = (kv_mul + p.HC - 1) / p.HC;
-        int rw = 4;
-        if (T == 1) rw = p.HC <= 4 ? 1 : (p.HC <= 8 ? 2 : 4);
-        // long portions: eight rows per warp share each read of a key, when two CTAs still fit an SM and every SM gets two
-        else if (p.dv <= 128 && attn_smem_bytes<8, 4>(p.dk, p.dv, 1) <= 112 * 1024 &&
-                 (long long)((T * p.HC + 8 * ATT_WARPS - 1) / (8 * ATT_WARPS)) * p.G * chunks >= 2 * sms)
-            rw = 8;
+        // Prompts and long portions: the register-tiled kernel, from one whole tile of rows on (the values in one or two 64-column
+        // blocks).  Fewer rows spread better over the 16-row tiles of attn_rows_kernel.
+        if (T > 1 && (long long)T * p.HC >= TA_ROWS && p.dv <= 128 && attn_tile_smem(p.dk, p.dv, p.v_in_k) <= 227 * 1024) {
+            p.TQ = std::max(1, TA_ROWS / p.HC);
+            if ((T + p.TQ - 1) / p.TQ <= 65535) return launch_attn_tiles<SIG>(st, p, p.G * chunks);
+        }
+        const int rw = T > 1 ? 4 : p.HC <= 4 ? 1 : p.HC <= 8 ? 2 : 4;
         p.TQ = std::max(1, rw * ATT_WARPS / p.HC);
         p.nsplit = 1;
         if (T == 1) {   // decode: split the keys so that the GPU has enough CTAs
@@ -391,8 +400,7 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
         const int gx = (T + p.TQ - 1) / p.TQ, gy = p.G * chunks;
         int rc = rw == 1   ? launch_attn_rw<1, SIG>(st, p, gx, gy)
                  : rw == 2 ? launch_attn_rw<2, SIG>(st, p, gx, gy)
-                 : rw == 4 ? launch_attn_rw<4, SIG>(st, p, gx, gy)
-                           : launch_attn_rw<8, SIG>(st, p, gx, gy);
+                           : launch_attn_rw<4, SIG>(st, p, gx, gy);
         if (rc) return rc;
         if (p.nsplit > 1) {
             AttnCombineParams<AT> cp{};

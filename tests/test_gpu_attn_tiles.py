@@ -1,0 +1,37 @@
+"""The register-tiled prompt attention (csrc/attn_tiles.cuh) where its tiles end: head sizes of every shared-memory pitch and
+value width, query rows and keys around whole tiles of 64, grouped heads that do not divide a tile, prompts cut in portions.
+One-layer Genetar models in float32 against the float64 implementation, held to that mode's 2e-4 of the logits' root mean square
+(test_gpu_genetar.py); the windowed, chunked, penalised, sink and latent forms run in the test files of their models."""
+import numpy as np
+import pytest
+
+import genetar_oracle as G
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,n", [
+    (4, 1, 64, 64, 16),     # exactly one tile of rows
+    (4, 1, 64, 64, 17),     # one row more
+    (4, 2, 64, 64, 129),    # key tiles: two whole ones and one key
+    (3, 1, 128, 128, 64),   # 21 tokens x 3 heads in a tile of 64 rows
+    (2, 2, 128, 64, 65),    # an ungrouped head of latent attention's shape
+    (2, 2, 96, 96, 127),    # pitch 96, value columns beyond 96 unused
+    (2, 1, 72, 72, 70),     # pitch 96, partial pieces at the end of a row
+    (2, 1, 160, 128, 66),   # pitch 160
+    (2, 1, 20, 4, 90),      # one piece of values
+    (2, 1, 10, 6, 80),      # sizes that are not whole 16-byte pieces
+    (20, 1, 32, 32, 9),     # more grouped heads than a tile takes at once
+])
+def test_tile_edges(gpu_lib, tmp_path, heads, kv_heads, dim, vdim, n):
+    cfg = G.make_config([G.attention_layer("attention_2", heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, ff=0, v_mix=False, scale=0.3, rot_dims=4)])
+    W = G.random_weights(cfg, seed=dim + n, qk_gain=2.0)
+    toks = np.random.default_rng(n).integers(0, cfg["vocab"], n).tolist()
+    want, _ = G.forward(cfg, W, toks)
+    m = gpu_lib.Transformer.open(G.write_model(str(tmp_path / "m"), cfg, W), dtype="float32", max_tokens=160)
+    whole = m.forward_tokens(toks, 0, list(range(n)))
+    assert G.rel_rms(whole, want) < 2e-4
+    cut = max(1, n // 2 - 3)   # a portion that starts inside a tile
+    parts = np.concatenate([m.forward_tokens(toks[:cut], 0, list(range(cut))), m.forward_tokens(toks[cut:], cut, list(range(n - cut)))])
+    assert G.rel_rms(parts, want) < 2e-4
+    m.close()
