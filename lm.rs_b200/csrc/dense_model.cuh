@@ -20,6 +20,7 @@
 #include "arch.h"
 #include "attn_tiles.cuh"
 #include "dense_gemm.cuh"
+#include "dense_gemm_f32.cuh"
 #include "dense_ops.cuh"
 #include "safetensors.h"
 
@@ -277,6 +278,18 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
         return 0;
     }
 
+    // a many-row product on CUDA cores: `rows` bounds the rows of one batch entry or group
+    template <int EPI> int launch_gemm_cores(cudaStream_t st, const GemmTiledParams<AT, WT>& p, int rows, int nb) {
+        if constexpr (std::is_same<AT, float>::value && std::is_same<WT, float>::value) {
+            if (gemm_f32_usable(p)) {
+                constexpr int cols = EPI == EPI_GLU ? FG_N / 2 : FG_N;
+                return optin(gemm_f32_kernel<EPI>, FG_SMEM) ||
+                       launch_k("gemm_f32_kernel", st, false, gemm_f32_kernel<EPI>, dim3((p.O + cols - 1) / cols, (rows + FG_M - 1) / FG_M, nb), dim3(FG_THREADS), FG_SMEM, p);
+            }
+        }
+        gemm_tiled_kernel<AT, WT, EPI><<<dim3((p.O + 63) / 64, (rows + 63) / 64, nb), 256, 0, st>>>(p);
+        return check_launch("gemm_tiled_kernel");
+    }
     // out = a . w^T with an epilogue; T rows.  One row: the streaming kernel; many rows: tensor cores when the shape
     // allows, else CUDA cores.
     template <int EPI> int matmul(cudaStream_t st, int T, const AT* a, int lda, const WT* w, const WT* w2, int K, int O, const EpiParams<AT>& e) {
@@ -291,8 +304,7 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
         }
         GemmTiledParams<AT, WT> p{};
         p.a = a; p.lda = lda; p.w = w; p.w2 = w2; p.T = T; p.K = K; p.O = O; p.e = e;
-        gemm_tiled_kernel<AT, WT, EPI><<<dim3((O + 63) / 64, (T + 63) / 64), 256, 0, st>>>(p);
-        return check_launch("gemm_tiled_kernel");
+        return launch_gemm_cores<EPI>(st, p, T, 1);
     }
     // nb products at once, one matrix per batch entry z (a head): out[:, z*o_bs ..] = a[:, z*a_bs ..] . (w + z*w_bs)^T.  The
     // matrices are small (a head's share of a projection), so the CUDA-core kernels serve both operand types.
@@ -305,8 +317,7 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
         }
         GemmTiledParams<AT, WT> p{};
         p.a = a; p.lda = lda; p.w = w; p.T = T; p.K = K; p.O = O; p.e = e; p.a_bs = a_bs; p.w_bs = w_bs; p.o_bs = o_bs;
-        gemm_tiled_kernel<AT, WT, EPI><<<dim3((O + 63) / 64, (T + 63) / 64, nb), 256, 0, st>>>(p);
-        return check_launch("gemm_tiled_kernel");
+        return launch_gemm_cores<EPI>(st, p, T, nb);
     }
     // rows sorted by group (expert): group z owns rows grp[z] .. grp[z+1] (device) and matrix w + z*O*K; T rows in all, no
     // group has more than max_group_rows
@@ -318,8 +329,7 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
         }
         GemmTiledParams<AT, WT> p{};
         p.a = a; p.lda = lda; p.w = w; p.w2 = w2; p.T = T; p.K = K; p.O = O; p.e = e; p.grp = grp; p.w_bs = (long long)O * K;
-        gemm_tiled_kernel<AT, WT, EPI><<<dim3((O + 63) / 64, (std::min(T, max_group_rows) + 63) / 64, n_groups), 256, 0, st>>>(p);
-        return check_launch("gemm_tiled_kernel");
+        return launch_gemm_cores<EPI>(st, p, std::min(T, max_group_rows), n_groups);
     }
     template <int EPI, int NORM> int launch_gemv(cudaStream_t st, GemvRowsParams<AT, WT> p, int nb = 1) {
         const int K = std::max(p.K, p.extra.w ? p.extra.K : 0), O = std::max(p.O, p.extra.w ? p.extra.O : 0);
