@@ -333,16 +333,18 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
     }
     template <int EPI, int NORM> int launch_gemv(cudaStream_t st, GemvRowsParams<AT, WT> p, int nb = 1) {
         const int K = std::max(p.K, p.extra.w ? p.extra.K : 0), O = std::max(p.O, p.extra.w ? p.extra.O : 0);
-        const size_t smem = ((size_t)((K + 3) & ~3) + 36 + 2 * 8 + 4) * 4;
+        auto aligned = [](const void* a, long long stride) { return (reinterpret_cast<uintptr_t>(a) & 15) == 0 && stride * (long long)sizeof(AT) % 16 == 0; };
+        p.staged = NORM != NORM_NONE || !aligned(p.a, nb > 1 || p.bidx ? p.a_bs : 0) || !aligned(p.extra.a, 0);
+        const size_t smem = p.staged ? ((size_t)K * sizeof(AT) + 15) & ~(size_t)15 : 0;
         if (optin(gemv_rows_kernel<AT, WT, EPI, NORM>, smem)) return 1;
-        const int rows_per_cta = EPI == EPI_GLU ? 8 : 16;
-        int grid = (O + rows_per_cta - 1) / rows_per_cta;
-        // few rows: the warps of a CTA split K instead (two row pairs per CTA)
-        p.ksplit = EPI != EPI_GLU && grid < 2 * sms && p.K % Vec16<WT>::N == 0 && p.K >= 1024;
-        if (p.ksplit) grid = (O + 3) / 4;
-        p.pdl = pdl_now ? 1 : 0;
-        grid = std::max(1, std::min(grid, sms * 4));
-        return launch_k("gemv_rows_kernel", st, pdl_now, gemv_rows_kernel<AT, WT, EPI, NORM>, dim3(grid, nb), dim3(256), smem, p);
+        // few rows: warps split K until every SM has about two CTAs' warps at work, down to two pieces per lane (2048 x 8192 bf16 without the
+        // split: 512 tasks for 2368 warps)
+        const int out = EPI == EPI_GLU ? GV_ROWS / 2 : GV_ROWS, groups = (O + out - 1) / out, pieces = K / Vec16<WT>::N;
+        p.ks = 1;
+        while (p.ks < 8 && (long long)groups * nb * p.ks < 16LL * sms && pieces >= 128 * p.ks) p.ks *= 2;
+        const int gpc = 8 / p.ks, tasks = (groups + gpc - 1) / gpc, cap_x = std::max(1, 2 * sms / nb);
+        const int rounds = (tasks + cap_x - 1) / cap_x;
+        return launch_k("gemv_rows_kernel", st, pdl_now, gemv_rows_kernel<AT, WT, EPI, NORM>, dim3((tasks + rounds - 1) / rounds, nb), dim3(GV_THREADS), smem, p);
     }
 
     template <int RW, int NI, bool SIG> int launch_attn_t(cudaStream_t st, AttnRowsParams<AT> p, int grid_x, int grid_y) {

@@ -31,6 +31,8 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "step_params.h"
 
 namespace lmrs {
@@ -565,7 +567,15 @@ template <int EPI, typename AT> DN_DEVINL void epi_apply(const EpiParams<AT>& e,
 }
 
 // ---- one row times a matrix: W [O][K] streamed once ----------------------------------------------------------------------
-// A warp owns output rows o = warp, warp + nwarps, ...; lanes walk K in 16-byte pieces, four pieces in flight per lane.
+// Bound by HBM for large matrices and by latency for all of them: a decode step is a chain of such products of 8 to 70 MB, 1 to 10 us
+// each at full bandwidth.  So every lane has 16 loads of 16 bytes in flight (256 threads, two CTAs per SM: 19 MB over the chip), the
+// first of them issued before the input is waited for or normalised, and every register is loaded again as soon as it has been
+// used, across task borders.  A task is GV_ROWS weight rows (EPI_GLU: two gate rows and the same two up rows) times one of `ks` slices of
+// K, one per warp; the warps of a CTA that share rows add their slices in a fixed order.  The grid is persistent.  (Two rows per warp, 4
+// loads in flight, the input staged in f32 before the first of them, up to four CTAs per SM: 23.6 us for the 67 MB of a gate/up
+// product at width 2048 and 18.4 us on average for the output and down projections, against 18.2 and 9.4; cold, ncu.)
+// The input row is read in the operand type: straight from memory by the lanes that need it, or, normalised here (or misaligned),
+// from shared memory.
 // NORM: the input row is the f32 residual, normalised here and rounded to the operand type exactly as the row kernels
 // (rmsnorm_rows_kernel, tanhnorm_rows_kernel) do, so both routes feed the product the same numbers.
 //   NORM_RMS   x * rsqrt(mean x^2 + eps) * nw          NORM_TANH   tanh(alpha x) w + b
@@ -595,8 +605,8 @@ template <typename AT, typename WT> struct GemvRowsParams {
     TanhNorm tn;                                  // NORM_TANH
     const WT* w; const WT* w2;   // [O][K]; w2: the "up" matrix of EPI_GLU
     int K, O;
-    int ksplit;               // 1: the warps of a CTA split K of one row pair (few rows), 0: a warp per row pair
-    int pdl;                  // launched with programmatic dependent launch: prefetch weights before waiting for the input
+    int ks;                   // slices of K that the warps of a CTA share (1, 2, 4 or 8)
+    int staged;               // the input row goes through shared memory (always with a norm; otherwise when it is not 16-byte aligned)
     EpiParams<AT> e;
     const int* bidx; long long a_bs, w_bs, o_bs;
     int n_mats;
@@ -606,76 +616,28 @@ template <typename AT, typename WT> struct GemvRowsParams {
 template <typename WT> struct Vec16;
 template <> struct Vec16<float> { static constexpr int N = 4; };
 template <> struct Vec16<__nv_bfloat16> { static constexpr int N = 8; };
-template <typename WT> DN_DEVINL void load16(const WT* p, float (&v)[Vec16<WT>::N]);
-template <> DN_DEVINL void load16<float>(const float* p, float (&v)[4]) {
-    const float4 q = __ldcs(reinterpret_cast<const float4*>(p));
-    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+DN_DEVINL uint4 ldcs16(const void* p) { return __ldcs(reinterpret_cast<const uint4*>(p)); }
+DN_DEVINL void widen16(const uint4& q, float (&v)[4], const float*) {
+    v[0] = __uint_as_float(q.x); v[1] = __uint_as_float(q.y); v[2] = __uint_as_float(q.z); v[3] = __uint_as_float(q.w);
 }
-template <> DN_DEVINL void load16<__nv_bfloat16>(const __nv_bfloat16* p, float (&v)[8]) {
-    const uint4 q = __ldcs(reinterpret_cast<const uint4*>(p));
+DN_DEVINL void widen16(const uint4& q, float (&v)[8], const __nv_bfloat16*) {
     const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
     for (int i = 0; i < 4; i++) { v[2 * i] = __uint_as_float(w[i] << 16); v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
 }
-// NR weight rows against the same input row: the shared-memory reads of the input are paid once for NR rows
-template <typename WT, int NR>
-DN_DEVINL void dot_rows(const WT* const (&w)[NR], const float* __restrict__ xs, int K, int lane, bool vec, float (&out)[NR]) {
-    constexpr int N = Vec16<WT>::N;
-    float acc[NR];
-#pragma unroll
-    for (int r = 0; r < NR; r++) acc[r] = 0.0f;
-    if (vec) {
-        const int pieces = K / N;
-        int i = lane;
-        for (; i + 32 < pieces; i += 64) {
-            float v[NR][2][N];
-#pragma unroll
-            for (int r = 0; r < NR; r++) { load16<WT>(w[r] + (size_t)i * N, v[r][0]); load16<WT>(w[r] + (size_t)(i + 32) * N, v[r][1]); }
-#pragma unroll
-            for (int u = 0; u < 2; u++) {
-                float xv[N];
-#pragma unroll
-                for (int j = 0; j < N; j += 4) {
-                    const float4 x4 = *reinterpret_cast<const float4*>(xs + (size_t)(i + 32 * u) * N + j);
-                    xv[j] = x4.x; xv[j + 1] = x4.y; xv[j + 2] = x4.z; xv[j + 3] = x4.w;
-                }
-#pragma unroll
-                for (int r = 0; r < NR; r++)
-#pragma unroll
-                    for (int j = 0; j < N; j++) acc[r] = fmaf(v[r][u][j], xv[j], acc[r]);
-            }
-        }
-        for (; i < pieces; i += 32) {
-            float xv[N];
-#pragma unroll
-            for (int j = 0; j < N; j += 4) {
-                const float4 x4 = *reinterpret_cast<const float4*>(xs + (size_t)i * N + j);
-                xv[j] = x4.x; xv[j + 1] = x4.y; xv[j + 2] = x4.z; xv[j + 3] = x4.w;
-            }
-#pragma unroll
-            for (int r = 0; r < NR; r++) {
-                float v0[N];
-                load16<WT>(w[r] + (size_t)i * N, v0);
-#pragma unroll
-                for (int j = 0; j < N; j++) acc[r] = fmaf(v0[j], xv[j], acc[r]);
-            }
-        }
-    } else {
-        for (int k = lane; k < K; k += 32)
-#pragma unroll
-            for (int r = 0; r < NR; r++) acc[r] = fmaf(to_f(w[r][k]), xs[k], acc[r]);
-    }
-#pragma unroll
-    for (int r = 0; r < NR; r++) out[r] = warp_sum(acc[r]);
-}
+template <typename WT> DN_DEVINL void load16(const WT* p, float (&v)[Vec16<WT>::N]) { widen16(ldcs16(p), v, p); }
+constexpr int GV_ROWS = 4, GV_PIECES = 4, GV_THREADS = 256;   // weight rows of a task, 16-byte pieces of each a lane has in flight
 template <typename AT, typename WT, int EPI, int NORM>
-static __global__ void __launch_bounds__(256) gemv_rows_kernel(const GemvRowsParams<AT, WT> pp) {
-    extern __shared__ __align__(16) float gv_xs[];   // [K rounded up to 4] the input row as f32, then reduction slots
+static __global__ void __launch_bounds__(GV_THREADS, 2) gemv_rows_kernel(const GemvRowsParams<AT, WT> pp) {
+    static_assert(std::is_same<AT, WT>::value, "the input row has the weights' type");
+    extern __shared__ __align__(16) unsigned char gv_sm[];   // the staged input row
+    constexpr int N = Vec16<WT>::N, R = GV_ROWS, U = GV_PIECES, OUT = EPI == EPI_GLU ? R / 2 : R, NW = GV_THREADS / 32;
+    __shared__ float red[36];
+    __shared__ float part[2][NW][R];
     GemvRowsParams<AT, WT> p = pp;
     pdl_launch();
     if (p.extra.w && blockIdx.y == gridDim.y - 1) {
         p.a = p.extra.a; p.w = p.extra.w; p.w2 = p.extra.w2; p.K = p.extra.K; p.O = p.extra.O; p.e.out = p.extra.out; p.e.act = p.extra.act;
-        p.ksplit = p.ksplit && p.K % Vec16<WT>::N == 0;
     } else if (gridDim.y > 1 || p.bidx) {   // the expert list is written by the step's router kernel: read it after the wait
         if (p.bidx) pdl_wait();
         const long long by = blockIdx.y, bw = p.bidx ? p.bidx[by] : by;
@@ -686,84 +648,120 @@ static __global__ void __launch_bounds__(256) gemv_rows_kernel(const GemvRowsPar
         if (p.e.out) p.e.out += by * p.o_bs;
         if (p.e.act) p.e.act += by * p.o_bs;
     }
-    float* red = gv_xs + ((p.K + 3) & ~3);
-    if (p.pdl) {   // weights do not depend on the predecessor: ask L2 for this warp's first rows while waiting for it
-        const int w0 = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
-        const int o = p.ksplit ? 2 * (int)blockIdx.x : (EPI == EPI_GLU ? w0 : 2 * w0);
-        if (o < p.O) {
-            const char* base = reinterpret_cast<const char*>(p.w + (size_t)o * p.K);
-            const size_t bytes = (size_t)p.K * sizeof(WT) * (EPI == EPI_GLU ? 1 : (o + 1 < p.O ? 2 : 1));
-            const size_t lo = p.ksplit ? bytes * (threadIdx.x >> 5) / (blockDim.x >> 5) : 0;
-            const size_t hi = p.ksplit ? bytes * ((threadIdx.x >> 5) + 1) / (blockDim.x >> 5) : bytes;
-            for (size_t b = lo + (size_t)(threadIdx.x & 31) * 128; b < hi && b < lo + 8192; b += 32 * 128)
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(base + b));
-            if (EPI == EPI_GLU) {
-                const char* base2 = reinterpret_cast<const char*>(p.w2 + (size_t)o * p.K);
-                for (size_t b = (size_t)(threadIdx.x & 31) * 128; b < bytes && b < 8192; b += 32 * 128)
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(base2 + b));
-            }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool vec = p.K % N == 0;   // every weight row then starts on a 16-byte boundary
+    const int ks = p.ks, gpc = NW / ks, slice = warp % ks;
+    const int units = vec ? p.K / N : p.K, per = (units + ks - 1) / ks;        // pieces, or elements
+    const int s0 = min(units, slice * per), s1 = min(units, s0 + per);
+    const int n_batch = max(1, (per + 32 * U - 1) / (32 * U));                  // uniform over the CTA
+    const int n_groups = (p.O + OUT - 1) / OUT, stride = gridDim.x * gpc;
+    const int g0 = blockIdx.x * gpc + warp / ks;
+    // the rows of task group g (rows past the end repeat the last one: their sums are dropped)
+    const WT* rows[R];
+    auto set_rows = [&](int g) {
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const int o = min(g * OUT + (EPI == EPI_GLU ? r >> 1 : r), p.O - 1);
+            rows[r] = (EPI == EPI_GLU && (r & 1) ? p.w2 : p.w) + (size_t)o * p.K;
         }
+    };
+    uint4 wv[U][R];
+    auto load = [&](int u, int b) {
+        const int i = s0 + (b * U + u) * 32 + lane;
+        if (i < s1) {
+#pragma unroll
+            for (int r = 0; r < R; r++) wv[u][r] = ldcs16(rows[r] + (size_t)i * N);
+        }
+    };
+    set_rows(min(g0, n_groups - 1));
+    if (vec) {
+#pragma unroll
+        for (int u = 0; u < U; u++) load(u, 0);
     }
     pdl_wait();
-    if (NORM == NORM_RMS) {
-        float ss = 0.0f;
-        for (int c = threadIdx.x; c < p.K; c += blockDim.x) { const float v = p.x[c]; ss += v * v; }
-        ss = block_sum(ss, red);
-        const float inv = 1.0f / sqrtf(ss / (float)p.K + p.eps);
-        for (int c = threadIdx.x; c < p.K; c += blockDim.x) { AT r; from_f(r, p.x[c] * inv * p.nw[c]); gv_xs[c] = to_f(r); }
-    } else if (NORM == NORM_LAYER) {
-        float mean, inv;
-        layernorm_stats(p.x, p.K, red, mean, inv, p.eps);
-        for (int c = threadIdx.x; c < p.K; c += blockDim.x) { AT r; from_f(r, (p.x[c] - mean) * inv * p.nw[c]); gv_xs[c] = to_f(r); }
-    } else if (NORM == NORM_TANH) {
-        const float alpha = *p.tn.alpha;
-        for (int c = threadIdx.x; c < p.K; c += blockDim.x) { AT r; from_f(r, tanhnorm_apply(p.tn, alpha, c, p.x[c])); gv_xs[c] = to_f(r); }
-    } else {
-        for (int c = threadIdx.x; c < p.K; c += blockDim.x) gv_xs[c] = to_f(p.a[c]);
+    const AT* xp = p.a;
+    if (NORM != NORM_NONE || p.staged) {
+        AT* xs = reinterpret_cast<AT*>(gv_sm);
+        if (NORM == NORM_RMS) {
+            float ss = 0.0f;
+#pragma unroll 8
+            for (int c = threadIdx.x; c < p.K; c += GV_THREADS) { const float v = p.x[c]; ss += v * v; }
+            ss = block_sum(ss, red);
+            const float inv = 1.0f / sqrtf(ss / (float)p.K + p.eps);
+#pragma unroll 8
+            for (int c = threadIdx.x; c < p.K; c += GV_THREADS) from_f(xs[c], p.x[c] * inv * p.nw[c]);
+        } else if (NORM == NORM_LAYER) {
+            float mean, inv;
+            layernorm_stats(p.x, p.K, red, mean, inv, p.eps);
+#pragma unroll 8
+            for (int c = threadIdx.x; c < p.K; c += GV_THREADS) from_f(xs[c], (p.x[c] - mean) * inv * p.nw[c]);
+        } else if (NORM == NORM_TANH) {
+            const float alpha = *p.tn.alpha;
+#pragma unroll 8
+            for (int c = threadIdx.x; c < p.K; c += GV_THREADS) from_f(xs[c], tanhnorm_apply(p.tn, alpha, c, p.x[c]));
+        } else {
+            for (int c = threadIdx.x; c < p.K; c += GV_THREADS) xs[c] = p.a[c];
+        }
+        xp = xs;
+        __syncthreads();
     }
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const bool vec = p.K % Vec16<WT>::N == 0;   // every weight row then starts on a 16-byte boundary
-    if (p.ksplit) {
-        // few output rows (a down or output projection): a warp per row pair would leave most of the GPU idle, so the
-        // warps of a CTA share a row pair, each walking one slice of K; partial sums meet in shared memory
-        constexpr int N = Vec16<WT>::N;
-        const int pieces = p.K / N;                                // ksplit is only chosen when K % N == 0
-        const int per = (pieces + nw - 1) / nw;
-        const int k0 = min(pieces, warp * per) * N, k1 = min(pieces, (warp + 1) * per) * N;
-        float* part = red + 36;                                    // [2][nw]
-        for (int o = 2 * blockIdx.x; o < p.O; o += 2 * gridDim.x) {
-            const int o1 = o + 1 < p.O ? o + 1 : o;
-            const WT* const rows[2] = {p.w + (size_t)o * p.K + k0, p.w + (size_t)o1 * p.K + k0};
-            float r[2];
-            dot_rows<WT, 2>(rows, gv_xs + k0, k1 - k0, lane, true, r);
-            if (lane == 0) { part[warp] = r[0]; part[nw + warp] = r[1]; }
-            __syncthreads();
-            if (warp == 0 && lane < 2) {
-                float a = 0.0f;
-                for (int w = 0; w < nw; w++) a += part[lane * nw + w];
-                if (lane == 0) epi_apply<EPI, AT>(p.e, 0, o, a, 0.0f);
-                else if (o1 != o) epi_apply<EPI, AT>(p.e, 0, o1, a, 0.0f);
+    int turn = 0;
+    for (int base = blockIdx.x * gpc; base < n_groups; base += stride, turn ^= 1) {
+        const int g = base + warp / ks;
+        float acc[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) acc[r] = 0.0f;
+        if (vec) {
+            for (int b = 0; b < n_batch; b++) {
+                const bool more = b + 1 < n_batch;
+                uint4 xq[U];
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const int i = s0 + (b * U + u) * 32 + lane;
+                    if (i < s1) xq[u] = *reinterpret_cast<const uint4*>(xp + (size_t)i * N);
+                }
+                if (!more && base + stride < n_groups) set_rows(min(g + stride, n_groups - 1));
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const int i = s0 + (b * U + u) * 32 + lane;
+                    if (i < s1) {
+                        float xv[N];
+                        widen16(xq[u], xv, (const AT*)nullptr);
+#pragma unroll
+                        for (int r = 0; r < R; r++) {
+                            float v[N];
+                            widen16(wv[u][r], v, (const WT*)nullptr);
+#pragma unroll
+                            for (int j = 0; j < N; j++) acc[r] = fmaf(v[j], xv[j], acc[r]);
+                        }
+                    }
+                    if (more) load(u, b + 1);
+                    else if (base + stride < n_groups) load(u, 0);   // the next task's first pieces
+                }
             }
-            __syncthreads();
+        } else {
+            set_rows(min(g, n_groups - 1));
+            for (int k = s0 + lane; k < s1; k += 32)
+#pragma unroll
+                for (int r = 0; r < R; r++) acc[r] = fmaf(to_f(rows[r][k]), to_f(xp[k]), acc[r]);
         }
-    } else if (EPI == EPI_GLU) {
-        for (int o = blockIdx.x * nw + warp; o < p.O; o += gridDim.x * nw) {
-            const WT* const rows[2] = {p.w + (size_t)o * p.K, p.w2 + (size_t)o * p.K};
-            float r[2];
-            dot_rows<WT, 2>(rows, gv_xs, p.K, lane, vec, r);
-            if (lane == 0) epi_apply<EPI, AT>(p.e, 0, o, r[0], r[1]);
+#pragma unroll
+        for (int r = 0; r < R; r++) acc[r] = warp_sum(acc[r]);
+        if (ks > 1) {
+            if (lane == 0)
+#pragma unroll
+                for (int r = 0; r < R; r++) part[turn][warp][r] = acc[r];
+            __syncthreads();   // (the other copy of part is free: everyone passed the barrier after its last use)
+            if (slice == 0)
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    acc[r] = part[turn][warp][r];
+                    for (int w = 1; w < ks; w++) acc[r] += part[turn][warp + w][r];
+                }
         }
-    } else {
-        for (int o = 2 * (blockIdx.x * nw + warp); o < p.O; o += 2 * gridDim.x * nw) {
-            const int o1 = o + 1 < p.O ? o + 1 : o;
-            const WT* const rows[2] = {p.w + (size_t)o * p.K, p.w + (size_t)o1 * p.K};
-            float r[2];
-            dot_rows<WT, 2>(rows, gv_xs, p.K, lane, vec, r);
-            if (lane == 0) {
-                epi_apply<EPI, AT>(p.e, 0, o, r[0], 0.0f);
-                if (o1 != o) epi_apply<EPI, AT>(p.e, 0, o1, r[1], 0.0f);
-            }
+        if (slice == 0 && g < n_groups && lane < OUT && g * OUT + lane < p.O) {
+            if (EPI == EPI_GLU) epi_apply<EPI, AT>(p.e, 0, g * OUT + lane, lane ? acc[2] : acc[0], lane ? acc[3] : acc[1]);
+            else epi_apply<EPI, AT>(p.e, 0, g * OUT + lane, lane == 0 ? acc[0] : lane == 1 ? acc[1] : lane == 2 ? acc[2] : acc[3], 0.0f);
         }
     }
     if (EPI == EPI_STORE && p.ln.counter) {

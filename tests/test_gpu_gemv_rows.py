@@ -1,0 +1,24 @@
+"""The one-row product (gemv_rows_kernel) at the edges of its split: rows that are one 16-byte piece, rows whose pieces do not fill a
+round of 32 lanes or a slice of K, one row more or less than a task, K split over two to eight warps, rows that do not start
+on 16-byte boundaries.  Decode steps of one-layer Genetar models against the float64 implementation, held to the tolerances of
+test_gpu_genetar.py (2e-4 and 4e-2 of the logits' root mean square)."""
+import numpy as np
+import pytest
+
+import genetar_oracle as G
+
+pytestmark = pytest.mark.gpu
+TOL = {"float32": 2e-4, "bfloat16": 4e-2}
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("width,ff,vocab", [(8, 8, 5), (72, 1, 3), (264, 136, 61), (1032, 520, 65), (520, 2056, 64), (512, 4104, 33), (27, 23, 10)])
+def test_decode_steps(gpu_lib, tmp_path, dtype, width, ff, vocab):
+    cfg = G.make_config([G.attention_layer("attention_2", heads=4, kv_heads=2, dim=16, vdim=16, ff=ff, v_mix=False)], width=width, vocab=vocab)
+    W = G.random_weights(cfg, seed=width + ff)
+    toks = np.random.default_rng(ff).integers(0, vocab, 6).tolist()
+    want, _ = G.forward(cfg, W, toks)
+    m = gpu_lib.Transformer.open(G.write_model(str(tmp_path / "m"), cfg, W), dtype=dtype, max_tokens=16)
+    got = np.stack([m.forward(t, i).copy() for i, t in enumerate(toks)])
+    assert G.rel_rms(got, want) < TOL[dtype]
+    m.close()
