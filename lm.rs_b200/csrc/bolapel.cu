@@ -355,7 +355,7 @@ template <typename AT, typename WT> class BolapelModel : public DenseModel<AT, W
         {
             EmbedRowsParams<WT> p{};
             p.embed = embed; p.bigram = nullptr; p.tokens = d_tokens; p.x = x; p.width = width; p.ps = ps;
-            embed_rows_kernel<WT><<<T, 128, 0, st>>>(p);
+            embed_rows_kernel<WT><<<embed_grid(T, width), EMBED_THREADS, 0, st>>>(p);
             if (check_launch("embed_rows_kernel")) return 1;
         }
         if (residual_rows(st, T, nullptr, mixer_of(0), ps)) return 1;

@@ -99,12 +99,16 @@ template <typename WT> struct EmbedRowsParams {
     float scale = 1.0f;
     WT* h = nullptr;                     // when set: x again in the operand type (a sublayer that reads the embedding unnormed)
 };
-template <typename WT> __global__ void __launch_bounds__(128) embed_rows_kernel(const EmbedRowsParams<WT> p) {
+// grid (T, column blocks).  A thread's columns are loaded before the first of them is stored: one column after the other cost a step of
+// one token 10 us of memory latency (width 2048, cold row).
+constexpr int EMBED_THREADS = 128, EMBED_COLS = 4;
+inline dim3 embed_grid(int T, int width) { return dim3(T, (width + EMBED_THREADS * EMBED_COLS - 1) / (EMBED_THREADS * EMBED_COLS)); }
+template <typename WT> __global__ void __launch_bounds__(EMBED_THREADS) embed_rows_kernel(const EmbedRowsParams<WT> p) {
     pdl_launch();
     pdl_wait();
     const uint32_t t = blockIdx.x, pos = pos_of(p.ps) + t;
     uint32_t tok;
-    if (p.ps.sp) { tok = p.ps.sp->token; if (threadIdx.x == 0) p.tokens[pos] = tok; }
+    if (p.ps.sp) { tok = p.ps.sp->token; if (threadIdx.x == 0 && blockIdx.y == 0) p.tokens[pos] = tok; }
     else tok = p.tokens[pos];
     const WT* e = p.embed + (size_t)tok * p.width;
     const WT* b = nullptr;
@@ -117,10 +121,19 @@ template <typename WT> __global__ void __launch_bounds__(128) embed_rows_kernel(
         b = p.bigram + (size_t)row * p.width;
     }
     float* x = p.x + (size_t)t * p.width;
-    for (int c = threadIdx.x; c < p.width; c += blockDim.x) {
-        const float v = (to_f(e[c]) + (b ? to_f(b[c]) : 0.0f)) * p.scale;
-        x[c] = v;
-        if (p.h) from_f(p.h[(size_t)t * p.width + c], v);
+    const int c0 = blockIdx.y * EMBED_THREADS * EMBED_COLS + threadIdx.x;
+    float v[EMBED_COLS];
+#pragma unroll
+    for (int i = 0; i < EMBED_COLS; i++) {
+        const int c = c0 + i * EMBED_THREADS;
+        v[i] = c < p.width ? (to_f(e[c]) + (b ? to_f(b[c]) : 0.0f)) * p.scale : 0.0f;
+    }
+#pragma unroll
+    for (int i = 0; i < EMBED_COLS; i++) {
+        const int c = c0 + i * EMBED_THREADS;
+        if (c >= p.width) continue;
+        x[c] = v[i];
+        if (p.h) from_f(p.h[(size_t)t * p.width + c], v[i]);
     }
 }
 

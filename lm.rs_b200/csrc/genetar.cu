@@ -235,7 +235,7 @@ template <typename AT, typename WT> class GenetarModel : public DenseModel<AT, W
             EmbedRowsParams<WT> p{};
             p.embed = embed; p.bigram = bigram; p.tokens = d_tokens; p.x = x; p.width = width; p.ps = ps;
             p.buckets = buckets; p.mul_prev = mul_prev; p.mul_cur = mul_cur;
-            embed_rows_kernel<WT><<<T, 128, 0, st>>>(p);
+            embed_rows_kernel<WT><<<embed_grid(T, width), EMBED_THREADS, 0, st>>>(p);
             if (check_launch("embed_rows_kernel")) return 1;
         }
         for (size_t li = 0; li < layers.size(); li++) {

@@ -212,7 +212,7 @@ template <typename AT, typename WT> class LutesunModel : public LatentModel<AT, 
         MoeRouterParams<AT> rp{};
         rp.h = h; rp.ld = width; rp.router = L.router; rp.correction = L.correction; rp.E = n_out; rp.extra = sh ? 1 : 0; rp.top = f.top; rp.width = width;
         rp.groups = f.groups; rp.keep = f.keep; rp.softmax = 1; rp.scale = f.scale; rp.z = rz; rp.idx = eidx; rp.wts = wts;
-        if (launch_k("moe_logits_kernel", st, pdl_now, moe_logits_kernel<AT>, dim3(T, (n_out + rp.extra + 3) / 4), dim3(128), 0, rp)) return 1;
+        if (launch_k("moe_logits_kernel", st, pdl_now, T == 1 ? moe_logits_kernel<AT, true> : moe_logits_kernel<AT, false>, moe_logits_grid(T, n_out + rp.extra), moe_logits_block(T), 0, rp)) return 1;
         if (launch_k("moe_topk_kernel", st, pdl_now, moe_topk_kernel<AT>, dim3(T), dim3(32), ((size_t)2 * n_out + f.groups) * 4, rp)) return 1;
         MoeCombineResNormParams<AT> np{};
         MoeCombineParams& cp = np.c;
@@ -257,7 +257,7 @@ template <typename AT, typename WT> class LutesunModel : public LatentModel<AT, 
         {
             EmbedRowsParams<WT> p{};
             p.embed = embed; p.tokens = d_tokens; p.x = x; p.width = width; p.ps = ps; p.scale = embed_scale; p.h = h;
-            embed_rows_kernel<WT><<<T, 128, 0, st>>>(p);
+            embed_rows_kernel<WT><<<embed_grid(T, width), EMBED_THREADS, 0, st>>>(p);
             if (check_launch("embed_rows_kernel")) return 1;
         }
         for (size_t li = 0; li < layers.size(); li++) {

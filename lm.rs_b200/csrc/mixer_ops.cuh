@@ -163,9 +163,22 @@ static __global__ void __launch_bounds__(256) latent_expand_kernel(const LatentE
 //   v_plain      the values are cached as they are instead of being divided by their root mean square per head
 constexpr int CONV_MAX_TAPS = 16;
 DN_DEVINL float conv_input(const float* in, int ld, const float* tail, int C, int taps, int tq, int c, uint32_t pos0) {
-    if (tq >= 0) return in[(size_t)tq * ld + c];
-    if ((long long)pos0 + tq < 0) return 0.0f;
-    return tail[(size_t)(taps - 1 + tq) * C + c];
+    // (one load whichever side it comes from: a branch per tap would keep the taps' loads from going out together)
+    const float* src = tq >= 0 ? in + (size_t)tq * ld + c : tail + (size_t)(taps - 1 + tq) * C + c;
+    return tq < 0 && (long long)pos0 + tq < 0 ? 0.0f : *src;
+}
+// sum over the taps of channel c, the last one on row t (wconv [C][taps])
+DN_DEVINL float conv_sum(const float* in, int ld, const float* tail, const float* wconv, int C, int taps, int t, int c, uint32_t pos0) {
+    float a = 0.0f;
+    if (taps == 4) {   // the usual width: the four weights in one load, the four inputs in flight together
+        const float4 w = *reinterpret_cast<const float4*>(wconv + (size_t)c * 4);
+        const float v0 = conv_input(in, ld, tail, C, 4, t - 3, c, pos0), v1 = conv_input(in, ld, tail, C, 4, t - 2, c, pos0);
+        const float v2 = conv_input(in, ld, tail, C, 4, t - 1, c, pos0), v3 = conv_input(in, ld, tail, C, 4, t, c, pos0);
+        return fmaf(w.w, v3, fmaf(w.z, v2, fmaf(w.y, v1, fmaf(w.x, v0, a))));
+    }
+#pragma unroll 4
+    for (int j = 0; j < taps; j++) a = fmaf(wconv[(size_t)c * taps + j], conv_input(in, ld, tail, C, taps, t - (taps - 1 - j), c, pos0), a);
+    return a;
 }
 struct QkvJointNormParams {
     const float* qkv; int ld;   // [q (H*dk) | k (G*dk) | v (G*dv)], biases already added
@@ -190,10 +203,7 @@ template <int THREADS> __global__ void __launch_bounds__(THREADS) qkv_jointnorm_
     const float* row = p.qkv + (size_t)t * p.ld;
     const int nq = p.H * p.dk, nk = p.G * p.dk, C = nq + nk + p.G * p.dv;
     auto conv = [&](int c) {   // channel c of this token after the convolution
-        float a = 0.0f;
-#pragma unroll 4
-        for (int j = 0; j < p.taps; j++) a = fmaf(p.wconv[(size_t)c * p.taps + j], conv_input(p.qkv, p.ld, p.tail, C, p.taps, t - (p.taps - 1 - j), c, pos0), a);
-        return a;
+        return conv_sum(p.qkv, p.ld, p.tail, p.wconv, C, p.taps, t, c, pos0);
     };
     auto move_tail = [&](int c) {   // the last taps-1 inputs of channel c become its tail (this thread alone touches the channel)
         float nv[CONV_MAX_TAPS];
@@ -289,21 +299,36 @@ template <typename AT> __global__ void __launch_bounds__(128) delta_pre_kernel(c
     const float* row = p.in + (size_t)t * p.ld;
     float* out = p.qkv_out + (size_t)t * C;
     auto conv_silu = [&](int c) {
-        float a = 0.0f;
-        for (int j = 0; j < p.taps; j++) a = fmaf(p.wconv[(size_t)c * p.taps + j], conv_input(p.in, p.ld, p.tail, C, p.taps, t - (p.taps - 1 - j), c, pos0), a);
-        return silu(a);
+        return silu(conv_sum(p.in, p.ld, p.tail, p.wconv, C, p.taps, t, c, pos0));
     };
     for (int task = wid; task < nqk + v_tasks + 1; task += wtotal) {
         if (task < nqk) {   // one q or k head: convolution, SiLU, unit length (q also / sqrt(dk))
+            // heads of up to 128 channels stay in registers, and all their loads come before the first store (a store could alias the next
+            // load for all the compiler knows: channel after channel waited for memory, 41 us for 512 tokens of
+            // 6144 channels with the taps one by one, 24 now)
             const int c0 = task * p.dk;
+            const float unit = task < p.G ? 1.0f / sqrtf((float)p.dk) : 1.0f;
             float ss = 0.0f;
+            if (p.dk <= 128) {
+                float v[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) { const int d = lane + 32 * i; v[i] = d < p.dk ? conv_silu(c0 + d) : 0.0f; ss += v[i] * v[i]; }
+                const float inv = unit / sqrtf(warp_sum(ss) + 1e-6f);
+#pragma unroll
+                for (int i = 0; i < 4; i++) if (lane + 32 * i < p.dk) out[c0 + lane + 32 * i] = v[i] * inv;
+                continue;
+            }
             for (int d = lane; d < p.dk; d += 32) { const float v = conv_silu(c0 + d); out[c0 + d] = v; ss += v * v; }
             ss = warp_sum(ss);
-            const float inv = (task < p.G ? 1.0f / sqrtf((float)p.dk) : 1.0f) / sqrtf(ss + 1e-6f);
+            const float inv = unit / sqrtf(ss + 1e-6f);
             for (int d = lane; d < p.dk; d += 32) out[c0 + d] *= inv;   // a lane rescales what it wrote itself
         } else if (task < nqk + v_tasks) {
             const int c0 = nqk * p.dk, i0 = (task - nqk) * 128, i1 = min(nv, i0 + 128);
-            for (int i = i0 + lane; i < i1; i += 32) out[c0 + i] = conv_silu(c0 + i);
+            float v[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) { const int d = i0 + lane + 32 * i; v[i] = d < i1 ? conv_silu(c0 + d) : 0.0f; }
+#pragma unroll
+            for (int i = 0; i < 4; i++) if (i0 + lane + 32 * i < i1) out[c0 + i0 + lane + 32 * i] = v[i];
         } else {
             for (int h = lane; h < p.H; h += 32) p.beta[(size_t)t * p.H + h] = 1.0f / (1.0f + expf(-row[C + h]));
             if (p.head_decay)

@@ -394,7 +394,7 @@ template <typename AT, typename WT> class RupenexModel : public DenseModel<AT, W
         MoeRouterParams<AT> rp{};
         rp.h = h; rp.ld = width; rp.router = L.router; rp.correction = L.correction; rp.E = n_out; rp.top = c.top; rp.width = width; rp.softmax = 1;
         rp.scale = 1.0f; rp.z = rz; rp.idx = eidx; rp.wts = wts;
-        if (launch_k("moe_logits_kernel", st, pdl_now, moe_logits_kernel<AT>, dim3(T, (n_out + 3) / 4), dim3(128), 0, rp)) return 1;
+        if (launch_k("moe_logits_kernel", st, pdl_now, T == 1 ? moe_logits_kernel<AT, true> : moe_logits_kernel<AT, false>, moe_logits_grid(T, n_out), moe_logits_block(T), 0, rp)) return 1;
         if (launch_k("moe_topk_kernel", st, pdl_now, moe_topk_kernel<AT>, dim3(T), dim3(32), (size_t)2 * n_out * 4, rp)) return 1;
         MoeCombineParams cp{};
         cp.y = ye; cp.wts = wts; cp.top = c.top; cp.width = width; cp.idx = eidx; cp.n_real = c.E; cp.xin = x; cp.ld_in = width; cp.x = x; cp.ldx = width;
@@ -439,7 +439,7 @@ template <typename AT, typename WT> class RupenexModel : public DenseModel<AT, W
         {
             EmbedRowsParams<WT> p{};
             p.embed = embed; p.bigram = nullptr; p.tokens = d_tokens; p.x = x; p.width = width; p.ps = ps;
-            embed_rows_kernel<WT><<<T, 128, 0, st>>>(p);
+            embed_rows_kernel<WT><<<embed_grid(T, width), EMBED_THREADS, 0, st>>>(p);
             if (check_launch("embed_rows_kernel")) return 1;
             if (norm_into_residual(st, T, x, embed_norm, nullptr)) return 1;
         }

@@ -341,7 +341,8 @@ template <typename AT, typename WT> class TudatarModel : public LatentModel<AT, 
         QkvJointNormParams np{};
         np.qkv = proj; np.ld = L.in_rows; np.H = c.H; np.G = c.G; np.dk = c.dk; np.dv = c.dv; np.wq = L.qnorm; np.wk = L.knorm; np.eps = info.eps;
         np.q_out = qa; np.kcache = L.kcache; np.vcache = L.vcache; np.ps = ps;
-        if (launch_k("qkv_jointnorm_post_kernel", st, pdl_now, qkv_jointnorm_post_kernel<256>, dim3(T, 3), dim3(256), 0, np)) return 1;
+        if (T == 1 ? launch_k("qkv_jointnorm_post_kernel", st, pdl_now, qkv_jointnorm_post_kernel<1024>, dim3(1, 3), dim3(1024), 0, np)
+                   : launch_k("qkv_jointnorm_post_kernel", st, pdl_now, qkv_jointnorm_post_kernel<256>, dim3(T, 3), dim3(256), 0, np)) return 1;
         AttnRowsParams<AT> p{};
         p.q = qa; p.kcache = L.kcache; p.vcache = L.vcache; p.out = att;
         p.T = T; p.H = c.H; p.G = c.G; p.dk = c.dk; p.dv = c.dv; p.scale = c.scale; p.ps = ps;
@@ -416,7 +417,7 @@ template <typename AT, typename WT> class TudatarModel : public LatentModel<AT, 
         MoeRouterParams<AT> rp{};
         rp.h = T > 1 ? h : nullptr; rp.x = x; rp.tn = L.n2.view(); rp.ld = width; rp.router = L.router; rp.correction = L.correction;
         rp.E = f.E; rp.top = f.top; rp.width = width; rp.scale = f.scale; rp.z = rz; rp.idx = eidx; rp.wts = wts;
-        if (launch_k("moe_logits_kernel", st, pdl_now, moe_logits_kernel<AT>, dim3(T, (f.E + 3) / 4), dim3(128), 0, rp)) return 1;
+        if (launch_k("moe_logits_kernel", st, pdl_now, T == 1 ? moe_logits_kernel<AT, true> : moe_logits_kernel<AT, false>, moe_logits_grid(T, f.E), moe_logits_block(T), 0, rp)) return 1;
         if (launch_k("moe_topk_kernel", st, pdl_now, moe_topk_kernel<AT>, dim3(T), dim3(32), (size_t)2 * f.E * 4, rp)) return 1;
         MoeCombineParams cp{};
         cp.y = y; cp.wts = wts; cp.x = x; cp.ldx = width; cp.n = L.n2b.view(); cp.top = f.top; cp.width = width;
@@ -450,7 +451,7 @@ template <typename AT, typename WT> class TudatarModel : public LatentModel<AT, 
         {
             EmbedRowsParams<WT> p{};
             p.embed = embed; p.bigram = nullptr; p.tokens = d_tokens; p.x = x; p.width = width; p.ps = ps;
-            embed_rows_kernel<WT><<<T, 128, 0, st>>>(p);
+            embed_rows_kernel<WT><<<embed_grid(T, width), EMBED_THREADS, 0, st>>>(p);
             if (check_launch("embed_rows_kernel")) return 1;
         }
         for (size_t li = 0; li < layers.size(); li++) {
