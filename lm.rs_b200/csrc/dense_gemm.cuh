@@ -40,6 +40,7 @@ struct TcGemmParams {
     // grouped form (one matrix per expert over rows sorted by expert): blockIdx.z = group z owns rows grp[z] .. grp[z+1] of A and
     // of the output and rows z*O .. z*O+O of the weight tensor map; null: one matrix for all T rows
     const int* grp;
+    int stages;   // two-SM kernel: stages of its ring
 };
 
 DN_DEVINL bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
@@ -93,6 +94,48 @@ DN_DEVINL void tg_tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
           "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
         : "r"(taddr)
         : "memory");
+}
+
+// 32 x 32 results (stg[row][column], rows of 33 floats) through the epilogue; lane = column o, rows t0 .. t0 + 31 below row_end
+template <int EPI> DN_DEVINL void tg_store_block(const EpiParams<__nv_bfloat16>& e, const float* stg, int t0, int o, int row_end, int O, int lane) {
+    if (o >= O) return;
+    if constexpr (EPI == EPI_STORE) {
+        float* __restrict__ dst = e.out + (size_t)t0 * e.ldo + o;
+        const float bias = e.bias ? e.bias[o] : 0.0f;
+#pragma unroll 8
+        for (int r = 0; r < 32; r++)
+            if (t0 + r < row_end) {
+                const float a = e.bias ? stg[r * 33 + lane] * e.scale + bias : stg[r * 33 + lane] * e.scale;
+                dst[(size_t)r * e.ldo] = e.softcap > 0.0f ? e.softcap * tanhf(a / e.softcap) : a;
+            }
+    } else if constexpr (EPI == EPI_RESID) {
+        float* __restrict__ dst = e.out + (size_t)t0 * e.ldo + o;
+        const float lsv = e.ls[o], lbv = e.lb ? e.lb[o] : 0.0f;
+        const float alpha = e.tanh_alpha ? *e.tanh_alpha : 0.0f;
+#pragma unroll 1
+        for (int r0 = 0; r0 < 32; r0 += 8) {
+            float x[8];
+#pragma unroll
+            for (int r = 0; r < 8; r++) x[r] = (t0 + r0 + r < row_end) ? dst[(size_t)(r0 + r) * e.ldo] : 0.0f;
+#pragma unroll
+            for (int r = 0; r < 8; r++)
+                if (t0 + r0 + r < row_end) {
+                    float a = stg[(r0 + r) * 33 + lane];
+                    if (e.tanh_alpha) a = tanhf(alpha * a);
+                    dst[(size_t)(r0 + r) * e.ldo] = e.lb ? x[r] + (lsv * a + lbv) : x[r] + lsv * a;
+                }
+        }
+    } else {
+        __nv_bfloat16* __restrict__ dst = e.act + (size_t)t0 * e.lda + o;
+        const float bias = EPI == EPI_ACT && e.bias ? e.bias[o] : 0.0f;
+#pragma unroll 8
+        for (int r = 0; r < 32; r++)
+            if (t0 + r < row_end) {
+                float a = stg[r * 33 + lane];
+                if constexpr (EPI == EPI_ACT) a = act_apply(e, a + bias);
+                dst[(size_t)r * e.lda] = __float2bfloat16_rn(a);
+            }
+    }
 }
 
 // EPI_GLU: the B tile is 64 rows of the gate matrix followed by the same 64 rows of the up matrix, so accumulator
@@ -205,47 +248,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
                     stg[lane * 33 + j] = val;
                 }
                 __syncwarp();
-                const int o = n0 + c0 + lane;
-                const int t0 = m0 + quad * 32;
-                if (o < p.O) {
-                    if constexpr (EPI == EPI_STORE) {
-                        float* __restrict__ dst = p.e.out + (size_t)t0 * p.e.ldo + o;
-                        const float bias = p.e.bias ? p.e.bias[o] : 0.0f;
-#pragma unroll 8
-                        for (int r = 0; r < 32; r++)
-                            if (t0 + r < row_end) {
-                                const float a = p.e.bias ? stg[r * 33 + lane] * p.e.scale + bias : stg[r * 33 + lane] * p.e.scale;
-                                dst[(size_t)r * p.e.ldo] = p.e.softcap > 0.0f ? p.e.softcap * tanhf(a / p.e.softcap) : a;
-                            }
-                    } else if constexpr (EPI == EPI_RESID) {
-                        float* __restrict__ dst = p.e.out + (size_t)t0 * p.e.ldo + o;
-                        const float lsv = p.e.ls[o], lbv = p.e.lb ? p.e.lb[o] : 0.0f;
-                        const float alpha = p.e.tanh_alpha ? *p.e.tanh_alpha : 0.0f;
-#pragma unroll 1
-                        for (int r0 = 0; r0 < 32; r0 += 8) {
-                            float x[8];
-#pragma unroll
-                            for (int r = 0; r < 8; r++) x[r] = (t0 + r0 + r < row_end) ? dst[(size_t)(r0 + r) * p.e.ldo] : 0.0f;
-#pragma unroll
-                            for (int r = 0; r < 8; r++)
-                                if (t0 + r0 + r < row_end) {
-                                    float a = stg[(r0 + r) * 33 + lane];
-                                    if (p.e.tanh_alpha) a = tanhf(alpha * a);
-                                    dst[(size_t)(r0 + r) * p.e.ldo] = p.e.lb ? x[r] + (lsv * a + lbv) : x[r] + lsv * a;
-                                }
-                        }
-                    } else {
-                        __nv_bfloat16* __restrict__ dst = p.e.act + (size_t)t0 * p.e.lda + o;
-                        const float bias = EPI == EPI_ACT && p.e.bias ? p.e.bias[o] : 0.0f;
-#pragma unroll 8
-                        for (int r = 0; r < 32; r++)
-                            if (t0 + r < row_end) {
-                                float a = stg[r * 33 + lane];
-                                if constexpr (EPI == EPI_ACT) a = act_apply(p.e, a + bias);
-                                dst[(size_t)r * p.e.lda] = __float2bfloat16_rn(a);
-                            }
-                    }
-                }
+                tg_store_block<EPI>(p.e, stg, m0 + quad * 32, n0 + c0 + lane, row_end, p.O, lane);
                 __syncwarp();
             }
         }
@@ -255,6 +258,201 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(BN) : "memory");
+    }
+    if (threadIdx.x == 0 && *abort_flag && p.err) *p.err = 1;
+}
+
+// ---- two SMs on one tile (tcgen05 cta_group::2): prompts of more than 128 rows ----------------------------------------------------
+// What bounded the one-CTA kernel at 512 rows is not the tensor pipe but the operand traffic between L2 and the SMs: a 128 x 128 tile
+// reads 256 operand rows for 16 K outputs, and gate + up at width 2048 (34 GFLOP, 21 us at the measured peak) moves 537 MB in 53 us; the down
+// projection, whose 64-wide tiles read 192 rows for 8 K outputs, 403 MB in 56 us.  Here a pair of CTAs shares a tile of 256 rows x BN columns: each
+// CTA stages its own 128 rows of A and half of the BN rows of W, one thread of the even CTA issues M = 256 MMAs that read both
+// CTAs' shared memory, and each CTA's TMEM receives its own 128 rows x BN columns.  Twice the outputs per operand row.
+//   BN 256   stages of 32 KB.  With more CTAs than SMs two share an SM (3 stages and 256 TMEM columns each): one tile's epilogue runs under
+//            the other's MMAs.  With one CTA per SM it gets all of the ring: 6 stages
+//   BN 128   where 256-wide tiles would leave SMs without work: 3 stages of 24 KB, three CTAs per SM (4 stages and two CTAs: 90 us
+//            instead of 67 for the residual products of 2048 rows at width 3072)
+//   SPLIT 2  where even those would: two pairs (a cluster of four) take halves of K; each then finishes half of the columns, adding the
+//            other's sums, which arrive through distributed shared memory, in a fixed order.  4 stages, or 8 with one CTA per SM
+// EPI_GLU: the even CTA's half of W are gate rows, the odd one's the same up rows: accumulator columns c and c + BN / 2.
+// Barriers: the copies of both CTAs complete on the even CTA's `full`; the MMA's commit frees the stage in both.  Every mbarrier wait
+// is bounded as in the kernel above.
+DN_DEVINL uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %cluster_ctarank;" : "=r"(r)); return r; }
+DN_DEVINL uint32_t cluster_addr(const void* p, uint32_t rank) {   // the same shared-memory address in another CTA of the cluster
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
+    return r;
+}
+DN_DEVINL void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+DN_DEVINL void tg_tma_load_2d_pair(void* dst, const CUtensorMap* map, int x, int y, uint32_t bar) {   // bar: a cluster address
+    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+                     smem_u32(dst)),
+                 "l"(map), "r"(x), "r"(y), "r"(bar)
+                 : "memory");
+}
+DN_DEVINL void tg_mma_pair(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+DN_DEVINL void tg_commit_pair(uint64_t* bar, uint16_t mask) {   // arrives on this barrier in every CTA of the mask
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "h"(mask) : "memory");
+}
+template <int BN> __host__ __device__ constexpr uint32_t tg_idesc_pair() {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
+}
+__host__ __device__ constexpr int tg_pair_stages(int bn, int split, bool alone) { return bn == 256 || split == 1 ? (alone ? 6 : 3) : (alone ? 8 : 4); }
+constexpr size_t tg_pair_smem(int bn, int stages) { return 1024 + (size_t)stages * (TG_A_BYTES + bn / 2 * TG_KB) + 256; }
+template <int EPI, int BN, int SPLIT>
+__global__ void __launch_bounds__(TG_THREADS, 2)
+gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ CUtensorMap tm_b2,
+                      const TcGemmParams p) {
+    constexpr bool GLU = EPI == EPI_GLU;
+    constexpr int OUT_COLS = GLU ? BN / 2 : BN, HALF_B = BN / 2;
+    constexpr uint32_t STAGE = TG_A_BYTES + HALF_B * TG_KB;
+    static_assert((size_t)tg_pair_stages(BN, SPLIT, false) * STAGE >= 4 * 32 * 33 * 4 + (SPLIT > 1 ? 128 * (BN / 2) * 4 : 0), "the idle ring holds the epilogue's buffers");
+    extern __shared__ uint8_t tg_raw[];
+    uint8_t* tiles = tg_raw + (((smem_u32(tg_raw) + 1023u) & ~1023u) - smem_u32(tg_raw));
+    uint64_t* full = reinterpret_cast<uint64_t*>(tiles + (size_t)p.stages * STAGE);
+    uint64_t* empty = full + p.stages;
+    uint64_t* tfull = empty + p.stages;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tfull + 1);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_rank(), side = rank & 1, split = rank >> 1;
+    const int m0 = blockIdx.y * 256 + (int)side * 128, n0 = (int)(blockIdx.x / (2 * SPLIT)) * OUT_COLS;
+    const int KS = (p.K * 2 + TG_KB - 1) / TG_KB;
+    const int g0 = KS * (int)split / SPLIT, g1 = KS * ((int)split + 1) / SPLIT;   // this pair's stages of K
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < p.stages; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        mbar_init(tfull, 1);
+        *abort_flag = 0;
+        fence_barrier_init();
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "n"(BN) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    cluster_sync();   // the other CTAs' barriers exist before anything is signalled there
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem_base = *tmem_slot;
+
+    if (warp == 0) {
+        if (lane == 0) {   // ---- TMA producer: this CTA's rows of A and of W ----
+            int issued = 0;
+            for (int g = g0, s = 0, round = 0; g < g1; g++) {
+                if (!mbar_wait_bounded(&empty[s], (round & 1) ^ 1, abort_flag)) break;
+                uint8_t* a_t = tiles + (size_t)s * STAGE;
+                if (side == 0) mbar_expect_tx(&full[s], 2 * STAGE);   // both CTAs' bytes
+                const uint32_t bar = cluster_addr(&full[s], rank & ~1u);
+                tg_tma_load_2d_pair(a_t, &tm_a, g * TG_KB, m0, bar);
+                if (GLU) tg_tma_load_2d_pair(a_t + TG_A_BYTES, side ? &tm_b2 : &tm_b, g * TG_KB, n0, bar);
+                else tg_tma_load_2d_pair(a_t + TG_A_BYTES, &tm_b, g * TG_KB, n0 + (int)side * HALF_B, bar);
+                issued++;
+                if (++s == p.stages) { s = 0; round++; }
+            }
+            if (*abort_flag && side == 0) {   // gave up somewhere: let the copies already requested land before shared memory goes away
+                for (int i = issued > p.stages ? issued - p.stages : 0; i < issued; i++)
+                    for (uint32_t w = 0; w < TG_SPIN_LIMIT && !mbar_try_wait(&full[i % p.stages], (i / p.stages) & 1); w++) {}
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0 && side == 0) {   // ---- MMA issuer of the pair ----
+            constexpr uint32_t idesc = tg_idesc_pair<BN>();
+            const uint16_t mask = (uint16_t)(3u << (rank & ~1u));
+            bool ok = true;
+            for (int i = 0, s = 0, round = 0; i < g1 - g0; i++) {
+                ok = mbar_wait_bounded(&full[s], round & 1, abort_flag);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint8_t* a_t = tiles + (size_t)s * STAGE;
+                const uint64_t da = tg_desc_sw128(a_t), db = tg_desc_sw128(a_t + TG_A_BYTES);
+#pragma unroll
+                for (int k = 0; k < TG_KB / 32; k++) tg_mma_pair(tmem_base, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (i > 0 || k > 0) ? 1u : 0u);
+                tg_commit_pair(&empty[s], mask);
+                if (++s == p.stages) { s = 0; round++; }
+            }
+            if (ok) tg_commit_pair(tfull, mask);
+        }
+    }
+    __syncwarp();
+    const int quad = warp & 3;
+    const uint32_t tmem_lane = tmem_base + ((uint32_t)(quad * 32) << 16);
+    constexpr int CHUNKS = OUT_COLS / 32, MINE = CHUNKS / SPLIT;   // 32-column chunks of the output, and those this pair finishes
+    float4* recv = reinterpret_cast<float4*>(tiles + 4 * 32 * 33 * 4);   // SPLIT: the other pair's sums, [chunk][gate | up][8][row]
+    bool ok = true;
+    if (warp >= 2) {
+        ok = mbar_wait_bounded(tfull, 0, abort_flag);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    }
+    if constexpr (SPLIT > 1) {
+        cluster_sync();   // every pair's MMAs are done (or given up): the rings are free
+        if (warp >= 2 && ok) {
+            const int other = 1 - (int)split;
+            const uint32_t dst = cluster_addr(recv, (uint32_t)other * 2 + side) + (uint32_t)(quad * 32 + lane) * 16;
+            for (int m = 0; m < MINE * (GLU ? 2 : 1); m++) {
+                const int c0 = (GLU ? (m & 1) * HALF_B : 0) + (other * MINE + (GLU ? m >> 1 : m)) * 32;
+                uint32_t v[32];
+                tg_tmem_ld32(tmem_lane + (uint32_t)c0, v);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + (uint32_t)((m * 8 + j) * 128) * 16), "r"(v[4 * j]), "r"(v[4 * j + 1]),
+                                 "r"(v[4 * j + 2]), "r"(v[4 * j + 3])
+                                 : "memory");
+            }
+        }
+        cluster_sync();   // the sums have arrived
+    }
+    if (warp >= 2 && ok && m0 < p.T) {   // ---- epilogue: as in the kernel above, 32 x 32 blocks through the idle ring ----
+        float* stg = reinterpret_cast<float*>(tiles) + (size_t)(warp - 2) * 32 * 33;
+#pragma unroll 1
+        for (int m = 0; m < MINE; m++) {
+            const int c0 = ((int)split * MINE + m) * 32;
+            uint32_t v[32], u[GLU ? 32 : 1];
+            tg_tmem_ld32(tmem_lane + (uint32_t)c0, v);
+            if constexpr (GLU) tg_tmem_ld32(tmem_lane + (uint32_t)(HALF_B + c0), u);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            if constexpr (SPLIT > 1) {   // first half of K + second half of K, whichever is here
+                auto add = [&](uint32_t (&w)[32], int slot) {
+#pragma unroll
+                    for (int j = 0; j < 8; j++) {
+                        const float4 o = recv[(slot * 8 + j) * 128 + quad * 32 + lane];
+                        const float f[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+                        for (int i = 0; i < 4; i++) w[4 * j + i] = __float_as_uint(__uint_as_float(w[4 * j + i]) + f[i]);
+                    }
+                };
+                add(v, GLU ? 2 * m : m);
+                if constexpr (GLU) add(u, 2 * m + 1);
+            }
+#pragma unroll
+            for (int j = 0; j < 32; j++) {
+                float val = __uint_as_float(v[j]);
+                if constexpr (GLU) val = glu_apply(p.e, val, __uint_as_float(u[j]));
+                stg[lane * 33 + j] = val;
+            }
+            __syncwarp();
+            tg_store_block<EPI>(p.e, stg, m0 + quad * 32, n0 + c0 + lane, p.T, p.O, lane);
+            __syncwarp();
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    cluster_sync();   // nobody's shared memory, barriers or TMEM go away while another CTA of the cluster may still touch them
+    if (warp == 1) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(BN) : "memory");
     }
     if (threadIdx.x == 0 && *abort_flag && p.err) *p.err = 1;
 }
@@ -270,7 +468,7 @@ struct DenseGemmCtx {
     int* h_err = nullptr;   // mapped, pinned
     int* d_err = nullptr;
     std::map<std::pair<const void*, int>, CUtensorMap> wmaps;   // (weight matrix, box rows) -> tensor map
-    bool attr_set[4][2] = {};
+    bool attr_set[4][2] = {}, pair_attr_set[4][3] = {};
     ~DenseGemmCtx() { if (h_err) cudaFreeHost(h_err); }
 };
 // a [rows][row_bytes used of pitch_bytes] byte matrix, box 128 bytes x box_rows rows, 128B swizzle, zeros outside
@@ -280,7 +478,7 @@ inline bool tg_make_map(DenseGemmCtx& c, CUtensorMap* map, const void* base, siz
     cuuint32_t box[2] = {(cuuint32_t)TG_KB, (cuuint32_t)box_rows};
     cuuint32_t estr[2] = {1, 1};
     return c.enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 template <typename AT, typename WT> inline bool dense_gemm_usable(int T, int K, int O, int lda) {
     if (!std::is_same<AT, __nv_bfloat16>::value || !std::is_same<WT, __nv_bfloat16>::value) return false;
@@ -312,10 +510,21 @@ inline int dense_gemm_launch(DenseGemmCtx& c, cudaStream_t st, int T, const AT* 
         if ((reinterpret_cast<uintptr_t>(a) & 15) || (reinterpret_cast<uintptr_t>(w) & 15) || (w2 && (reinterpret_cast<uintptr_t>(w2) & 15))) return -1;
         if (*c.h_err) { err = "a tensor-core matrix product gave up waiting on one of its barriers (device status flag set)"; return 1; }
         constexpr bool GLU = EPI == EPI_GLU;
+        // Two-SM tiles for ungrouped products of more than 128 rows.  The form whose CTAs, spread over the SMs, do the fewest columns
+        // one after the other; 128-wide tiles move half as many outputs per operand byte of W, which costs about a sixth
+        int form = -1;   // 0: 256 columns, 1: 128 columns, 2: 128 columns and K split over two pairs
+        if (n_groups == 0 && T > 128) {
+            const int ty = (T + 255) / 256;
+            const auto ctas = [&](int bn) { const int oc = GLU ? bn / 2 : bn; return 2 * ty * ((O + oc - 1) / oc); };
+            const auto rounds = [&](int n) { return (n + c.sms - 1) / c.sms; };
+            form = rounds(ctas(256)) * 256 * 6 <= rounds(ctas(128)) * 128 * 7 ? 0 : 1;
+            if (form == 1 && ctas(128) <= c.sms) form = K >= 1024 ? 2 : -1;   // few tiles and a short K: the one-CTA kernel's smaller tiles
+            if (ty > 65535) form = -1;
+        }
         // 64-wide tiles when 128-wide ones would not give every SM a CTA
         const size_t w_rows = n_groups > 0 ? (size_t)n_groups * O : (size_t)O;
-        const bool narrow = !GLU && O > 64 && ((O + 127) / 128) * ((T + TG_M - 1) / TG_M) < c.sms;
-        const int box_rows = (GLU || narrow) ? 64 : 128;
+        const bool narrow = form < 0 && !GLU && O > 64 && ((O + 127) / 128) * ((T + TG_M - 1) / TG_M) < c.sms;
+        const int box_rows = form >= 0 ? (form == 0 ? 128 : 64) : (GLU || narrow) ? 64 : 128;
         auto wmap = [&](const void* base, CUtensorMap* out) {
             auto key = std::make_pair(base, box_rows * 1000003 + (int)(w_rows % 1000003));
             auto it = c.wmaps.find(key);
@@ -332,6 +541,28 @@ inline int dense_gemm_launch(DenseGemmCtx& c, cudaStream_t st, int T, const AT* 
         if (!wmap(w, &tb)) return -1;
         tb2 = tb;
         if (GLU && !wmap(w2, &tb2)) return -1;
+        if (form >= 0) {
+            TcGemmParams p{};
+            p.T = T; p.K = K; p.O = O; p.e = e; p.err = c.d_err;
+            auto kernel = form == 0 ? gemm_bf16_pair_kernel<EPI, 256, 1> : form == 1 ? gemm_bf16_pair_kernel<EPI, 128, 1> : gemm_bf16_pair_kernel<EPI, 128, 2>;
+            const int bn = form == 0 ? 256 : 128;
+            if (!c.pair_attr_set[EPI][form]) {
+                if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tg_pair_smem(bn, tg_pair_stages(bn, form == 2 ? 2 : 1, true))) != cudaSuccess) { err = "cudaFuncSetAttribute(gemm_bf16_pair_kernel) failed"; return 1; }
+                c.pair_attr_set[EPI][form] = true;
+            }
+            const int cluster = form == 2 ? 4 : 2, oc = bn / (GLU ? 2 : 1);
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3((O + oc - 1) / oc * cluster, (T + 255) / 256); cfg.blockDim = dim3(TG_THREADS); cfg.stream = st;
+            p.stages = tg_pair_stages(bn, form == 2 ? 2 : 1, (int)(cfg.gridDim.x * cfg.gridDim.y) <= c.sms);
+            cfg.dynamicSmemBytes = tg_pair_smem(bn, p.stages);
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+            cfg.attrs = attr; cfg.numAttrs = 1;
+            const cudaError_t ce = cudaLaunchKernelEx(&cfg, kernel, ta, tb, tb2, p);
+            if (ce != cudaSuccess) { err = std::string("gemm_bf16_pair_kernel: ") + cudaGetErrorString(ce); return 1; }
+            return 0;
+        }
         if (!c.attr_set[EPI][narrow]) {
             cudaError_t ae = narrow ? cudaFuncSetAttribute(gemm_bf16_tc_kernel<EPI, GLU ? 128 : 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TG_SMEM)
                                     : cudaFuncSetAttribute(gemm_bf16_tc_kernel<EPI, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TG_SMEM);
