@@ -369,15 +369,18 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
     }
     template <bool SIG> int launch_attn_tiles(cudaStream_t st, AttnRowsParams<AT> p, int gx) {
         p.async = p.dk % 4 == 0 && p.dv % 4 == 0 && p.k_ld % 4 == 0 && p.v_ld % 4 == 0;
+        p.sms = sms;
         const size_t smem = attn_tile_smem(p.dk, p.dv, p.v_in_k);
         const dim3 grid(gx, (p.T + p.TQ - 1) / p.TQ);
-        auto go = [&](auto kernel) { return optin(kernel, smem) || launch_k("attn_tile_kernel", st, pdl_now, kernel, grid, dim3(TA_THREADS), smem, p); };
+        auto go = [&](auto kernel, int threads) { return optin(kernel, smem) || launch_k("attn_tile_kernel", st, pdl_now, kernel, grid, dim3(threads), smem, p); };
         if constexpr (!SIG) {
-            if (p.v_in_k) return p.dv <= 64 ? go(attn_tile_kernel<AT, 1, 0, SIG, true>) : go(attn_tile_kernel<AT, 2, 0, SIG, true>);
+            if (p.v_in_k) return p.dv <= 64 ? go(attn_tile_kernel<AT, 1, 0, 1, SIG, true>, 128) : go(attn_tile_kernel<AT, 2, 0, 1, SIG, true>, 128);
         }
+        // values of one 64-column block: two groups of warps per CTA, so that an SM holds 16 warps instead of 8 or 12 (wider values need
+        // too many registers for that)
         const int pitch = attn_tile_pitch(p.dk);
-        if (p.dv <= 64) return pitch == 64 ? go(attn_tile_kernel<AT, 1, 64, SIG, false>) : pitch == 128 ? go(attn_tile_kernel<AT, 1, 128, SIG, false>) : go(attn_tile_kernel<AT, 1, 0, SIG, false>);
-        return pitch == 128 ? go(attn_tile_kernel<AT, 2, 128, SIG, false>) : pitch == 96 ? go(attn_tile_kernel<AT, 2, 96, SIG, false>) : go(attn_tile_kernel<AT, 2, 0, SIG, false>);
+        if (p.dv <= 64) return pitch == 64 ? go(attn_tile_kernel<AT, 1, 64, 2, SIG, false>, 256) : pitch == 128 ? go(attn_tile_kernel<AT, 1, 128, 2, SIG, false>, 256) : go(attn_tile_kernel<AT, 1, 0, 2, SIG, false>, 256);
+        return pitch == 128 ? go(attn_tile_kernel<AT, 2, 128, 1, SIG, false>, 128) : pitch == 96 ? go(attn_tile_kernel<AT, 2, 96, 1, SIG, false>, 128) : go(attn_tile_kernel<AT, 2, 0, 1, SIG, false>, 128);
     }
     // attention over T query rows: the caller fills the tensors, head geometry, pitches, scale, soft-cap, window, kept first keys,
     // sink, gates and penalty;
