@@ -72,8 +72,8 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
     std::map<int, GraphEntry> graphs;   // decode step per position bucket
     std::set<int> warmed;
     const StepParams* graph_step = nullptr;
-    // programmatic dependent launch of the decode chain is an option, off by default: measured slower here (1.32 vs 1.14 ms
-    // per step at 16 layers of width 2048): the early-launched CTAs of the next kernels sit on the SMs while they wait
+    // programmatic dependent launch of the decode chain is an option.  An architecture turns it on where it measures faster (Genetar);
+    // chains of many small kernels lose a little (Tudatar, 16 steps of 3 layers: 2.96 -> 3.03 ms)
     int use_graph = 1, use_pdl = 0;
 
     // what an architecture implements
