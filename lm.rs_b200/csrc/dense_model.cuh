@@ -510,21 +510,23 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
         for (size_t c0 = 0; c0 < n; c0 += chunk_rows) {
             const int T = (int)std::min(chunk_rows, n - c0);
             PosSrc ps{nullptr, pos + (uint32_t)c0};
-            if (run_layers(st, T, ps, pos + (uint32_t)c0)) return 1;
             // wanted rows of this chunk, in the order of `want`
             std::vector<uint32_t> rows, outk;
             for (size_t k = 0; k < n_want; k++)
                 if (want[k] >= c0 && want[k] < c0 + (size_t)T) { rows.push_back(want[k] - (uint32_t)c0); outk.push_back((uint32_t)k); }
-            if (rows.empty()) continue;
             const int m = (int)rows.size();
             bool contiguous = true;
             for (int i = 1; i < m; i++) contiguous = contiguous && outk[i] == outk[0] + (uint32_t)i;
+            if (m > 0 && T > 1) {   // their list goes ahead of the layers: nothing waits for the host between the last layer and the head
+                GCK(cudaMemcpyAsync(d_rows, rows.data(), (size_t)m * 4, cudaMemcpyHostToDevice, st));
+                GCK(cudaStreamSynchronize(st));   // `rows` is a local
+            }
+            if (run_layers(st, T, ps, pos + (uint32_t)c0)) return 1;
+            if (m == 0) continue;
             if (T == 1) {
                 for (int i = 0; i < m; i++) if (head_rows(st, 1, nullptr, d_out + (size_t)outk[i] * vocab)) return 1;
                 continue;
             }
-            GCK(cudaMemcpyAsync(d_rows, rows.data(), (size_t)m * 4, cudaMemcpyHostToDevice, st));
-            GCK(cudaStreamSynchronize(st));   // `rows` is a local
             if (contiguous) {
                 if (head_rows(st, m, d_rows, d_out + (size_t)outk[0] * vocab)) return 1;
             } else {

@@ -97,6 +97,7 @@ struct lmrs_b200 {
     int pfa_quads = 4;         // fused batched-rows attention: row quads (warps) per CTA, 4 or 8 (LMRS_B200_PFA_QUADS)
     int use_pf_attn = 1;       // batched-rows attention: 1 = fused throughput kernel (prefill_attn.cuh), 2 = its two-kernel form, 0 = the per-row decode kernel
     size_t rows_cap = 0;
+    uint32_t* d_emb_tok = nullptr; float* d_emb_out = nullptr; size_t emb_cap = 0;   // get_embeddings: rows it has room for
     StepParams* d_step = nullptr;
     StepParams* h_step_ring = nullptr;  // pinned
     int step_slot = 0;
@@ -1447,7 +1448,7 @@ extern "C" void lmrs_b200_destroy(lmrs_b200_t* m) {
     cudaFree(m->pf_g); cudaFree(m->pf_u); cudaFree(m->pf_h); cudaFree(m->pf_down); cudaFree(m->pf_scores); cudaFree(m->d_kcache); cudaFree(m->d_vcache); cudaFree(m->d_rope_cos); cudaFree(m->d_rope_sin);
     cudaFree(m->d_x[0]); cudaFree(m->d_x[1]); cudaFree(m->d_q); cudaFree(m->d_knew); cudaFree(m->d_att);
     cudaFree(m->d_wo_out); cudaFree(m->d_h); cudaFree(m->d_down_out); if (!m->d_xchg) cudaFree(m->d_logits); cudaFree(m->d_scores);
-    cudaFree(m->d_step); cudaFree(m->d_rows); cudaFree(m->d_ll); cudaFree(m->d_fin_scratch);
+    cudaFree(m->d_step); cudaFree(m->d_rows); cudaFree(m->d_emb_tok); cudaFree(m->d_emb_out); cudaFree(m->d_ll); cudaFree(m->d_fin_scratch);
     cudaFree(m->d_amax); cudaFree(m->d_aidx); cudaFree(m->d_ticket); cudaFree(m->d_next); cudaFree(m->d_gen);
     if (m->h_gen) cudaFreeHost(m->h_gen);
     if (m->ev_pf0) cudaEventDestroy(m->ev_pf0);
@@ -1729,9 +1730,15 @@ extern "C" int lmrs_b200_get_embeddings(const lmrs_b200_t* cm, const uint32_t* t
     for (size_t i = 0; i < n; i++)
         if (tokens[i] >= m->args.vocab_size) return fail("token out of range");
     CK(cudaSetDevice(m->device));
-    uint32_t* d_tok; float* d_out;
-    CK(cudaMalloc(&d_tok, n * 4));
-    CK(cudaMalloc(&d_out, n * (size_t)m->args.dim * 4));
+    if (m->emb_cap < n) {   // kept between calls (allocating and freeing both cost more than the lookup)
+        cudaFree(m->d_emb_tok); cudaFree(m->d_emb_out);
+        m->d_emb_tok = nullptr; m->d_emb_out = nullptr; m->emb_cap = 0;
+        CK(cudaMalloc(&m->d_emb_tok, n * 4));
+        CK(cudaMalloc(&m->d_emb_out, n * (size_t)m->args.dim * 4));
+        m->emb_cap = n;
+    }
+    uint32_t* d_tok = m->d_emb_tok;
+    float* d_out = m->d_emb_out;
     CK(cudaMemcpyAsync(d_tok, tokens, n * 4, cudaMemcpyHostToDevice, m->stream));
     EmbedParams p{};
     p.dim = m->args.dim; p.q_type = m->args.q_type; p.q = m->emb.q; p.s = m->emb.s; p.apply_scale = 0;   // :659-669: no Gemma scaling
@@ -1742,7 +1749,6 @@ extern "C" int lmrs_b200_get_embeddings(const lmrs_b200_t* cm, const uint32_t* t
     CK(e);
     CK(cudaMemcpyAsync(out, d_out, n * (size_t)m->args.dim * 4, cudaMemcpyDeviceToHost, m->stream));
     CK(cudaStreamSynchronize(m->stream));
-    cudaFree(d_tok); cudaFree(d_out);
     return 0;
 }
 
