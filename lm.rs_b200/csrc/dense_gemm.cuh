@@ -10,6 +10,7 @@
 // tensor maps carry the true extents, TMA fills rows >= T, weight rows >= O and the K tail with zeros, and the epilogue
 // masks its stores.  What the shape must satisfy: K and lda multiples of 8 elements (16-byte row pitch) and 16-byte
 // aligned bases.  Three stages of 32 KB leave room for two CTAs per SM: one tile's epilogue runs under the other's MMAs.
+// Prompts of more than 128 rows run on a two-SM form of the same kernel, further down.
 // Every wait is bounded: a wait that runs out raises a flag in mapped host memory, the roles stop, in-flight copies are
 // waited for (bounded again), TMEM is freed and the kernel returns; the next launch reports the flag.
 #pragma once

@@ -13,7 +13,7 @@
 //   gemv_rows_kernel         one token row:  weights streamed once (HBM-bound), optional fused RMS-norm prologue,
 //                            epilogues: store*scale+bias | x += ls * f(acc) + lb | act(gate) * up | store in the operand
 //                            type; a batch dimension (per-head matrices, or experts picked by a device-side index list)
-//   gemm_tiled_kernel        many rows, any shape, CUDA cores (the f32 path and ragged shapes); same epilogues; batched
+//   gemm_tiled_kernel        many rows, any shape, CUDA cores (what neither dense_gemm.cuh nor dense_gemm_f32.cuh takes); same epilogues; batched
 //                            over column blocks (one matrix per head) or grouped over row ranges (one matrix per expert)
 //   qkv_post_kernel          per head: unit RMS norm of q/k or partial rotary, value mixing with an earlier layer's
 //                            values, sigmoid head gate, K/V rows written to the cache
@@ -23,7 +23,7 @@
 //                            per head instead of the softmax, per-head or per-element sigmoid output gates, grouped query
 //                            heads, query tile x KV head per CTA, K and V rows
 //                            with their own pitch (V may be a prefix of the K row: attention over a shared latent),
-//                            optional split over the keys (decode) + attn_combine_kernel
+//                            optional split over the keys (decode) + attn_combine_kernel; prompts run on attn_tiles.cuh
 // What the design wants in 32-bit (norms, scores, softmax, residual, angles) is 32-bit here in both operand types.
 #pragma once
 #include <cuda_bf16.h>
