@@ -243,13 +243,20 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
         return 0;
     }
     bool pdl_now = false;   // set while a decode step is being enqueued
+    // Lets a kernel ask for `smem` bytes of dynamic shared memory.  Without it a launch may use 48 KB, the kernel's own static arrays
+    // included (a one-row product 12288 floats wide asks for exactly 48 KB beside a few hundred static bytes).
+    std::map<const void*, size_t> smem_limit;   // dynamic bytes each kernel may ask for so far
     template <typename K> int optin(K kernel, size_t smem) {
-        if (smem <= 48 * 1024) return 0;
-        static std::map<const void*, size_t> done;
-        auto it = done.find((const void*)kernel);
-        if (it != done.end() && it->second >= smem) return 0;
+        if (smem == 0) return 0;
+        auto it = smem_limit.find((const void*)kernel);
+        if (it == smem_limit.end()) {
+            cudaFuncAttributes fa;
+            GCK(cudaFuncGetAttributes(&fa, kernel));
+            it = smem_limit.emplace((const void*)kernel, 48 * 1024 - std::min<size_t>(48 * 1024, fa.sharedSizeBytes)).first;
+        }
+        if (smem <= it->second) return 0;
         GCK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        done[(const void*)kernel] = smem;
+        it->second = smem;
         return 0;
     }
 

@@ -14,6 +14,10 @@ TOL = {"float32": 2e-4, "bfloat16": 4e-2}
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("width,ff,vocab", [(8, 8, 5), (72, 1, 3), (264, 136, 61), (1032, 520, 65), (520, 2056, 64), (512, 4104, 33), (27, 23, 10)])
 def test_decode_steps(gpu_lib, tmp_path, dtype, width, ff, vocab):
+    check_one_layer(gpu_lib, tmp_path, dtype, width, ff, vocab)
+
+
+def check_one_layer(gpu_lib, tmp_path, dtype, width, ff, vocab):
     cfg = G.make_config([G.attention_layer("attention_2", heads=4, kv_heads=2, dim=16, vdim=16, ff=ff, v_mix=False)], width=width, vocab=vocab)
     W = G.random_weights(cfg, seed=width + ff)
     toks = np.random.default_rng(ff).integers(0, vocab, 6).tolist()
@@ -22,3 +26,9 @@ def test_decode_steps(gpu_lib, tmp_path, dtype, width, ff, vocab):
     got = np.stack([m.forward(t, i).copy() for i, t in enumerate(toks)])
     assert G.rel_rms(got, want) < TOL[dtype]
     m.close()
+
+
+@pytest.mark.parametrize("dtype,width", [("float32", 12288), ("bfloat16", 24448)])
+def test_input_rows_of_about_48_kb(gpu_lib, tmp_path, dtype, width):
+    """normalised rows whose shared memory reaches 48 KB only together with the kernel's own arrays"""
+    check_one_layer(gpu_lib, tmp_path, dtype, width, 8, 5)
