@@ -247,7 +247,7 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
     // included (a one-row product 12288 floats wide asks for exactly 48 KB beside a few hundred static bytes).
     std::map<const void*, size_t> smem_limit;   // dynamic bytes each kernel may ask for so far
     template <typename K> int optin(K kernel, size_t smem) {
-        if (smem == 0) return 0;
+        if (smem <= 32 * 1024) return 0;   // (no kernel here has 16 KB of static arrays)
         auto it = smem_limit.find((const void*)kernel);
         if (it == smem_limit.end()) {
             cudaFuncAttributes fa;
@@ -342,13 +342,16 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
         const int K = std::max(p.K, p.extra.w ? p.extra.K : 0), O = std::max(p.O, p.extra.w ? p.extra.O : 0);
         auto aligned = [](const void* a, long long stride) { return (reinterpret_cast<uintptr_t>(a) & 15) == 0 && stride * (long long)sizeof(AT) % 16 == 0; };
         p.staged = NORM != NORM_NONE || !aligned(p.a, nb > 1 || p.bidx ? p.a_bs : 0) || !aligned(p.extra.a, 0);
-        const size_t smem = p.staged ? ((size_t)K * sizeof(AT) + 15) & ~(size_t)15 : 0;
-        if (optin(gemv_rows_kernel<AT, WT, EPI, NORM>, smem)) return 1;
+        const size_t row = p.staged ? ((size_t)K * sizeof(AT) + 15) & ~(size_t)15 : 0;
         // few rows: warps split K until every SM has about two CTAs' warps at work, down to two pieces per lane (2048 x 8192 bf16 without the
         // split: 512 tasks for 2368 warps)
         const int out = EPI == EPI_GLU ? GV_ROWS / 2 : GV_ROWS, groups = (O + out - 1) / out, pieces = K / Vec16<WT>::N;
         p.ks = 1;
         while (p.ks < 8 && (long long)groups * nb * p.ks < 16LL * sms && pieces >= 128 * p.ks) p.ks *= 2;
+        p.row_at = GV_SUMS_BYTES;
+        if (row + GV_SUMS_BYTES > 227 * 1024) { p.ks = 1; p.row_at = GV_NORM_BYTES; }   // the widest rows leave no room for the slices' sums
+        const size_t smem = row + p.row_at;
+        if (optin(gemv_rows_kernel<AT, WT, EPI, NORM>, smem)) return 1;
         const int gpc = 8 / p.ks, tasks = (groups + gpc - 1) / gpc, cap_x = std::max(1, 2 * sms / nb);
         const int rounds = (tasks + cap_x - 1) / cap_x;
         return launch_k("gemv_rows_kernel", st, pdl_now, gemv_rows_kernel<AT, WT, EPI, NORM>, dim3((tasks + rounds - 1) / rounds, nb), dim3(GV_THREADS), smem, p);

@@ -619,6 +619,7 @@ template <typename AT, typename WT> struct GemvRowsParams {
     const WT* w; const WT* w2;   // [O][K]; w2: the "up" matrix of EPI_GLU
     int K, O;
     int ks;                   // slices of K that the warps of a CTA share (1, 2, 4 or 8)
+    int row_at;               // byte offset of the staged row in shared memory
     int staged;               // the input row goes through shared memory (always with a norm; otherwise when it is not 16-byte aligned)
     EpiParams<AT> e;
     const int* bidx; long long a_bs, w_bs, o_bs;
@@ -640,13 +641,17 @@ DN_DEVINL void widen16(const uint4& q, float (&v)[8], const __nv_bfloat16*) {
 }
 template <typename WT> DN_DEVINL void load16(const WT* p, float (&v)[Vec16<WT>::N]) { widen16(ldcs16(p), v, p); }
 constexpr int GV_ROWS = 4, GV_PIECES = 4, GV_THREADS = 256;   // weight rows of a task, 16-byte pieces of each a lane has in flight
+// Shared memory before the staged input row: a norm's 33 sums, then, with K split, two copies of the warps' GV_ROWS sums in their place.
+// (Static arrays would come off what is left for the row: with 512 bytes of them a normalised f32 row of 57988 to 58052 columns found
+// no room.  And one size for every split: kernels that follow one another with 144 and 256 bytes cost a step of Tudatar 4 %.)
+constexpr int GV_NORM_BYTES = 36 * 4, GV_SUMS_BYTES = 2 * GV_THREADS / 32 * GV_ROWS * 4;
 template <typename AT, typename WT, int EPI, int NORM>
 static __global__ void __launch_bounds__(GV_THREADS, 2) gemv_rows_kernel(const GemvRowsParams<AT, WT> pp) {
     static_assert(std::is_same<AT, WT>::value, "the input row has the weights' type");
-    extern __shared__ __align__(16) unsigned char gv_sm[];   // the staged input row
+    extern __shared__ __align__(16) unsigned char gv_sm[];   // [sums | the staged input row]
     constexpr int N = Vec16<WT>::N, R = GV_ROWS, U = GV_PIECES, OUT = EPI == EPI_GLU ? R / 2 : R, NW = GV_THREADS / 32;
-    __shared__ float red[36];
-    __shared__ float part[2][NW][R];
+    float* red = reinterpret_cast<float*>(gv_sm);                              // a norm's sums
+    float (*part)[NW][R] = reinterpret_cast<float (*)[NW][R]>(gv_sm);          // then, K split: two copies of the warps' sums
     GemvRowsParams<AT, WT> p = pp;
     pdl_launch();
     if (p.extra.w && blockIdx.y == gridDim.y - 1) {
@@ -694,7 +699,7 @@ static __global__ void __launch_bounds__(GV_THREADS, 2) gemv_rows_kernel(const G
     pdl_wait();
     const AT* xp = p.a;
     if (NORM != NORM_NONE || p.staged) {
-        AT* xs = reinterpret_cast<AT*>(gv_sm);
+        AT* xs = reinterpret_cast<AT*>(gv_sm + p.row_at);
         if (NORM == NORM_RMS) {
             float ss = 0.0f;
 #pragma unroll 8
@@ -778,15 +783,11 @@ static __global__ void __launch_bounds__(GV_THREADS, 2) gemv_rows_kernel(const G
         }
     }
     if (EPI == EPI_STORE && p.ln.counter) {
-        __shared__ unsigned int last;
+        unsigned int ticket = 0;
         __threadfence();   // this thread's stores of the row before the ticket
         __syncthreads();
-        if (threadIdx.x == 0) {
-            const unsigned int ticket = atomicAdd(p.ln.counter, 1u);
-            last = ticket == gridDim.x * gridDim.y - 1 ? 1u : 0u;
-        }
-        __syncthreads();
-        if (last) {
+        if (threadIdx.x == 0) ticket = atomicAdd(p.ln.counter, 1u);
+        if (__syncthreads_or(threadIdx.x == 0 && ticket == gridDim.x * gridDim.y - 1)) {
             __threadfence();
             const float* row = p.e.out;
             layernorm_row<AT>([&](int c) { return __ldcg(row + c); }, p.O, p.ln.w, p.ln.eps, red, p.ln.x, p.ln.ls, nullptr, p.ln.h);

@@ -32,3 +32,9 @@ def check_one_layer(gpu_lib, tmp_path, dtype, width, ff, vocab):
 def test_input_rows_of_about_48_kb(gpu_lib, tmp_path, dtype, width):
     """normalised rows whose shared memory reaches 48 KB only together with the kernel's own arrays"""
     check_one_layer(gpu_lib, tmp_path, dtype, width, 8, 5)
+
+
+def test_widest_f32_input_rows(gpu_lib, tmp_path):
+    """58048 columns leave room for the sums of a K split in an SM's 227 KB, 58052 do not"""
+    for width in (58048, 58052):
+        check_one_layer(gpu_lib, tmp_path, "float32", width, 8, 5)
