@@ -210,16 +210,20 @@ def test_long_greedy_generation_through_the_generate_loop(gpu_lib, tmp_path, dty
     # forward_argmax is the same pick
     m.forward_tokens(prompt[:-1], 0, [])
     assert m.forward_argmax(prompt[-1], len(prompt) - 1) == ids[0]
-    # decode steps replayed from CUDA graphs and launched one by one are the same arithmetic
-    m.set_option("graphs", 0)
-    m.forward_tokens(prompt[:-1], 0, [])
-    assert m.generate_greedy(prompt[-1], len(prompt) - 1, n_new).tolist() == ids
-    # ... and so are steps whose kernels are chained with programmatic dependent launch, replayed or not
-    for graphs in (1, 0):
-        m.set_option("graphs", graphs)
-        m.set_option("pdl", 1)
-        m.forward_tokens(prompt[:-1], 0, [])
-        assert m.generate_greedy(prompt[-1], len(prompt) - 1, n_new).tolist() == ids
+    # decode steps replayed from CUDA graphs or launched one by one, chained with programmatic dependent launch (the default) or
+    # each after the end of the last, are the same arithmetic: the same picks, and the same bits of the logits
+    # (a step is launched, then captured, then replayed: the last tokens of one key-tile bucket are replays)
+    logits = None
+    for pdl in (0, 1):
+        for graphs in (0, 1):
+            m.set_option("graphs", graphs)
+            m.set_option("pdl", pdl)
+            m.forward_tokens(prompt[:-1], 0, [])
+            assert m.generate_greedy(prompt[-1], len(prompt) - 1, n_new).tolist() == ids, (pdl, graphs)
+            m.forward_tokens(prompt[:-1], 0, [])
+            got = np.stack([m.forward(t, len(prompt) - 1 + i).copy() for i, t in enumerate([prompt[-1]] + ids[:70])])
+            logits = got if logits is None else logits
+            assert np.array_equal(got, logits), (pdl, graphs)
     with pytest.raises(gpu_lib.LmrsError):
         m.forward(1, 21 + n_new)   # beyond the cache
     m.close()
