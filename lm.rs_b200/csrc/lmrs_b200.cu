@@ -97,7 +97,7 @@ struct lmrs_b200 {
     int pfa_quads = 4;         // fused batched-rows attention: row quads (warps) per CTA, 4 or 8 (LMRS_B200_PFA_QUADS)
     int use_pf_attn = 1;       // batched-rows attention: 1 = fused throughput kernel (prefill_attn.cuh), 2 = its two-kernel form, 0 = the per-row decode kernel
     size_t rows_cap = 0;
-    uint32_t* d_emb_tok = nullptr; float* d_emb_out = nullptr; size_t emb_cap = 0;   // get_embeddings: rows it has room for
+    uint32_t* d_emb_tok = nullptr; float* d_emb_out = nullptr; size_t emb_cap = 0;   // get_embeddings: rows it has room for, at most seq_len
     StepParams* d_step = nullptr;
     StepParams* h_step_ring = nullptr;  // pinned
     int step_slot = 0;
@@ -1730,24 +1730,28 @@ extern "C" int lmrs_b200_get_embeddings(const lmrs_b200_t* cm, const uint32_t* t
     for (size_t i = 0; i < n; i++)
         if (tokens[i] >= m->args.vocab_size) return fail("token out of range");
     CK(cudaSetDevice(m->device));
-    if (m->emb_cap < n) {   // kept between calls (allocating and freeing both cost more than the lookup)
+    // The buffers are kept between calls (allocating and freeing both cost more than the lookup), at most seq_len rows of them -- the longest
+    // prompt; longer requests go through them in portions.
+    const size_t dim = m->args.dim, cap = std::min<size_t>(n, m->args.seq_len);
+    if (m->emb_cap < cap) {
         cudaFree(m->d_emb_tok); cudaFree(m->d_emb_out);
         m->d_emb_tok = nullptr; m->d_emb_out = nullptr; m->emb_cap = 0;
-        CK(cudaMalloc(&m->d_emb_tok, n * 4));
-        CK(cudaMalloc(&m->d_emb_out, n * (size_t)m->args.dim * 4));
-        m->emb_cap = n;
+        CK(cudaMalloc(&m->d_emb_tok, cap * 4));
+        CK(cudaMalloc(&m->d_emb_out, cap * dim * 4));
+        m->emb_cap = cap;
     }
-    uint32_t* d_tok = m->d_emb_tok;
-    float* d_out = m->d_emb_out;
-    CK(cudaMemcpyAsync(d_tok, tokens, n * 4, cudaMemcpyHostToDevice, m->stream));
     EmbedParams p{};
     p.dim = m->args.dim; p.q_type = m->args.q_type; p.q = m->emb.q; p.s = m->emb.s; p.apply_scale = 0;   // :659-669: no Gemma scaling
-    p.tokens = d_tok; p.step = m->d_step; p.out = d_out;
-    bool pdl = m->use_pdl; m->use_pdl = false;
-    cudaError_t e = launch(m, embed_kernel, dim3((unsigned)n), dim3(256), 0, p);
-    m->use_pdl = pdl;
-    CK(e);
-    CK(cudaMemcpyAsync(out, d_out, n * (size_t)m->args.dim * 4, cudaMemcpyDeviceToHost, m->stream));
+    p.tokens = m->d_emb_tok; p.step = m->d_step; p.out = m->d_emb_out;
+    for (size_t i = 0; i < n; i += m->emb_cap) {
+        const size_t rows = std::min(m->emb_cap, n - i);
+        CK(cudaMemcpyAsync(m->d_emb_tok, tokens + i, rows * 4, cudaMemcpyHostToDevice, m->stream));
+        bool pdl = m->use_pdl; m->use_pdl = false;
+        cudaError_t e = launch(m, embed_kernel, dim3((unsigned)rows), dim3(256), 0, p);
+        m->use_pdl = pdl;
+        CK(e);
+        CK(cudaMemcpyAsync(out + i * dim, m->d_emb_out, rows * dim * 4, cudaMemcpyDeviceToHost, m->stream));
+    }
     CK(cudaStreamSynchronize(m->stream));
     return 0;
 }

@@ -73,6 +73,21 @@ def test_get_embeddings_bit_exact(gpu_lib, ref, synth, name, q_type):
         gpu.get_embeddings([gpu.args.vocab_size])
 
 
+def test_get_embeddings_of_more_rows_than_the_context(gpu_lib, synth):
+    """a bulk lookup gives every row, and what the handle keeps of it on the device is at most seq_len rows"""
+    import torch
+    gpu, _ = gpu_lib.Transformer.new(synth("tiny-llama", 1))
+    vocab, dim, seq_len = gpu.args.vocab_size, gpu.args.dim, gpu.args.seq_len
+    table = gpu.get_embeddings(np.arange(vocab)).reshape(vocab, dim)
+    n = max(5 * seq_len + 3, (256 << 20) // (4 * dim))   # 256 MB of rows
+    toks = prompt_tokens(vocab, n)
+    before = torch.cuda.mem_get_info()[0]
+    rows = gpu.get_embeddings(toks).reshape(n, dim)
+    assert before - torch.cuda.mem_get_info()[0] <= seq_len * (dim + 1) * 4 + (16 << 20)   # (whole allocation granules)
+    assert np.array_equal(rows, table[toks])
+    gpu.close()
+
+
 @pytest.mark.parametrize("name,q_type", [("tiny-llama", 1), ("tiny-gemma", 1), ("tiny-phi", 1), ("tiny-llama", 2)])
 def test_fill_kv_cache_then_decode(gpu_lib, ref, synth, name, q_type):
     """The multimodal path of the bins: get_embeddings ++ features -> fill_kv_cache -> forward (chat.rs:110-119)."""
