@@ -1,0 +1,22 @@
+// dense_dispatch.h -- which kernel a call of the folder models takes, where that depends on sizes and was measured: plain functions of
+// the sizes and of the device, so that they can be read (and tested) without a GPU.
+#pragma once
+#include <algorithm>
+
+namespace lmrs {
+namespace dense {
+
+// Attention of a prompt or portion, T tokens x HC grouped query heads per CTA column (G * chunks columns): the register-tiled kernel of
+// attn_tiles.cuh (64 rows per CTA), or attn_rows_kernel (16 rows)?  A CTA walks all of its rows' keys by itself, so what counts first is how
+// many SMs have one.  As long as the small tiles are all resident at once, two per SM, they win or draw: 128 tokens of 16 ungrouped heads
+// of 128 behind 2000 keys take 1393 us a call (2 layers) with the large tiles, which occupy 32 SMs, and 1107 us with the small ones; 64 tokens of 24
+// heads on 8 KV heads of 128 1310 and 1084.  From the first CTA that has to wait for another one on the large tiles win: 192 tokens of those 24 heads
+// (312 small tiles) 507 us a layer behind 2000 keys against 733 (without earlier keys 157 against 153), 256 tokens of 32 heads of 64 (512) 308
+// against 519.  64-wide heads between 148 and 296 small tiles draw within 2 %.
+inline bool attn_large_tiles(int sms, int T, int columns, int HC) {
+    const int tokens = std::max(1, 16 / HC);
+    return (long long)columns * ((T + tokens - 1) / tokens) > 2LL * sms;
+}
+
+}  // namespace dense
+}  // namespace lmrs

@@ -19,6 +19,7 @@
 
 #include "arch.h"
 #include "attn_tiles.cuh"
+#include "dense_dispatch.h"
 #include "dense_gemm.cuh"
 #include "dense_gemm_f32.cuh"
 #include "dense_ops.cuh"
@@ -75,6 +76,7 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
     // programmatic dependent launch of the decode chain is an option.  An architecture turns it on where it measures faster (Genetar);
     // chains of many small kernels lose a little (Tudatar, 16 steps of 3 layers: 2.96 -> 3.03 ms)
     int use_graph = 1, use_pdl = 0;
+    int attn_tiles = -1;   // option: 1 / 0 the register-tiled attention wherever it can run / nowhere, -1 by attn_large_tiles
 
     // what an architecture implements
     virtual size_t n_layers() const = 0;
@@ -410,9 +412,9 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
         // a one-row step over few KV heads: fewer query heads per CTA, so that more SMs share the keys
         while (T == 1 && p.HC > 4 && p.G * ((kv_mul + p.HC - 1) / p.HC) * tiles < sms) p.HC /= 2;
         const int chunks = (kv_mul + p.HC - 1) / p.HC;
-        // Prompts and long portions: the register-tiled kernel, from one whole tile of rows on (the values in one or two 64-column
-        // blocks).  Fewer rows spread better over the 16-row tiles of attn_rows_kernel.
-        if (T > 1 && (long long)T * p.HC >= TA_ROWS && p.dv <= 128 && attn_tile_smem(p.dk, p.dv, p.v_in_k) <= 227 * 1024) {
+        // Prompts and long portions: the register-tiled kernel (the values in one or two 64-column blocks), where there are tiles enough
+        const bool large = attn_tiles < 0 ? (long long)T * p.HC >= TA_ROWS && attn_large_tiles(sms, T, p.G * chunks, p.HC) : attn_tiles > 0;
+        if (T > 1 && large && p.dv <= 128 && attn_tile_smem(p.dk, p.dv, p.v_in_k) <= 227 * 1024) {
             p.TQ = std::max(1, TA_ROWS / p.HC);
             if ((T + p.TQ - 1) / p.TQ <= 65535) return launch_attn_tiles<SIG>(st, p, p.G * chunks);
         }
@@ -567,6 +569,7 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
         if (!strcmp(name, "chunk_rows")) chunk_rows = (size_t)std::max(1, value);
         else if (!strcmp(name, "tensor_cores")) use_tc = value;
         else if (!strcmp(name, "graphs")) { use_graph = value; if (!value) drop_graphs(); }
+        else if (!strcmp(name, "attn_tiles")) attn_tiles = value;
         else if (!strcmp(name, "pdl")) { use_pdl = value; drop_graphs(); }
         else set_model_option(name, value);
     }

@@ -1,7 +1,10 @@
 """The register-tiled prompt attention (csrc/attn_tiles.cuh) where its tiles end: head sizes of every shared-memory pitch and
 value width, query rows and keys around whole tiles of 64, grouped heads that do not divide a tile, prompts cut in portions.
 One-layer Genetar models in float32 against the float64 implementation, held to that mode's 2e-4 of the logits' root mean square
-(test_gpu_genetar.py); the windowed, chunked, penalised, sink and latent forms run in the test files of their models."""
+(test_gpu_genetar.py).  The windowed, chunked, penalised, sink and latent forms: the mixed models of the other test files, held to
+theirs.  These calls are too small to take the kernel by themselves: option "attn_tiles" 1."""
+import importlib
+
 import numpy as np
 import pytest
 
@@ -29,9 +32,35 @@ def test_tile_edges(gpu_lib, tmp_path, heads, kv_heads, dim, vdim, n):
     toks = np.random.default_rng(n).integers(0, cfg["vocab"], n).tolist()
     want, _ = G.forward(cfg, W, toks)
     m = gpu_lib.Transformer.open(G.write_model(str(tmp_path / "m"), cfg, W), dtype="float32", max_tokens=160)
+    m.set_option("attn_tiles", 1)
     whole = m.forward_tokens(toks, 0, list(range(n)))
     assert G.rel_rms(whole, want) < 2e-4
     cut = max(1, n // 2 - 3)   # a portion that starts inside a tile
     parts = np.concatenate([m.forward_tokens(toks[:cut], 0, list(range(cut))), m.forward_tokens(toks[cut:], cut, list(range(n - cut)))])
     assert G.rel_rms(parts, want) < 2e-4
+    m.close()
+
+
+@pytest.mark.parametrize("arch", ["tudatar", "rupenex", "badepel", "bolapel", "lutesun"])
+@pytest.mark.parametrize("shared_latent", [False, True])
+def test_forms_of_the_other_models(gpu_lib, tmp_path, arch, shared_latent):
+    """windows with and without kept keys, blocks with sigmoid weights, penalties, sinks, gates, both latent forms: a prompt over
+    three key tiles whole, and in portions that start inside a tile, in 64-row tiles as in 16-row ones"""
+    if shared_latent and arch != "lutesun":
+        pytest.skip("one form")
+    T = importlib.import_module(f"test_gpu_{arch}")
+    n = 150
+    cfg = T.mixed_cfg()
+    toks = T.tokens_for(cfg, n)
+    W = T.weights_for(cfg, toks, seed=1) if hasattr(T, "weights_for") else T.O.random_weights(cfg, seed=1)
+    want, _ = T.O.forward(cfg, W, toks)
+    m = T.open_model(gpu_lib, tmp_path, cfg, W, "float32")
+    if shared_latent:
+        m.set_option("latent_expand_rows", 1000)
+    for tiles in (1, 0):
+        m.set_option("attn_tiles", tiles)
+        assert T.O.rel_rms(m.forward_tokens(toks, 0, list(range(n))), want) < T.TOL["float32"], tiles
+        cuts = [0, 67, 74, 140, n]   # one portion of seven rows: latent heads in their shared form
+        parts = [m.forward_tokens(toks[a:b], a, list(range(b - a))) for a, b in zip(cuts, cuts[1:])]
+        assert T.O.rel_rms(np.concatenate(parts), want) < T.TOL["float32"], tiles
     m.close()
