@@ -60,10 +60,10 @@ static __global__ void __launch_bounds__(128 * KH, 2) attn_tile_kernel(const Att
     const int kv_mul = p.H / p.G, chunks = (kv_mul + p.HC - 1) / p.HC;
     // late query tiles see the most keys: they are scheduled first.  When every CTA is resident at once, two on some SMs, the second ones go
     // out in the opposite order, so that the SMs with the longest tiles get the shortest as well (512 tokens x 32 heads: 9 key tiles on
-    // the busiest SM instead of 12, 66 us -> 59)
+    // the busiest SM instead of 12, 66 us -> 59; attn_order_turns_at)
     int id = blockIdx.y * gridDim.x + blockIdx.x;
     const int n_cta = gridDim.x * gridDim.y;
-    if (n_cta <= 2 * p.sms && id >= p.sms) id = p.sms + (n_cta - 1 - id);
+    if (n_cta <= 2 * p.turn && id >= p.turn) id = p.turn + (n_cta - 1 - id);
     const int bx = id % gridDim.x, by = id / gridDim.x;
     const int g = bx / chunks, h0 = (bx % chunks) * p.HC;
     const int t0 = (int)(gridDim.y - 1 - by) * p.TQ;

@@ -18,5 +18,11 @@ inline bool attn_large_tiles(int sms, int T, int columns, int HC) {
     return (long long)columns * ((T + tokens - 1) / tokens) > 2LL * sms;
 }
 
+// The large tiles with the most keys go out first.  Where the grid is at most two CTAs per SM the second half goes out in the opposite order, so
+// that an SM with a long tile gets a short one beside it -- if two CTAs of `smem` bytes fit an SM (228 KB, 1 KB of it reserved per CTA).  Where
+// only one fits (heads wider than 128 with values wider than 64) the second half is a second wave and starts with its longest tiles too.
+// Returns the CTA from which on the order turns, 0: none.
+inline int attn_order_turns_at(int sms, long long smem) { return 2 * (smem + 1024) <= 228 * 1024 ? sms : 0; }
+
 }  // namespace dense
 }  // namespace lmrs

@@ -381,8 +381,8 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
     }
     template <bool SIG> int launch_attn_tiles(cudaStream_t st, AttnRowsParams<AT> p, int gx) {
         p.async = p.dk % 4 == 0 && p.dv % 4 == 0 && p.k_ld % 4 == 0 && p.v_ld % 4 == 0;
-        p.sms = sms;
         const size_t smem = attn_tile_smem(p.dk, p.dv, p.v_in_k);
+        p.turn = attn_order_turns_at(sms, (long long)smem);
         const dim3 grid(gx, (p.T + p.TQ - 1) / p.TQ);
         auto go = [&](auto kernel, int threads) { return optin(kernel, smem) || launch_k("attn_tile_kernel", st, pdl_now, kernel, grid, dim3(threads), smem, p); };
         if constexpr (!SIG) {

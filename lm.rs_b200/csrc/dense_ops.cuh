@@ -998,7 +998,7 @@ template <typename AT> struct AttnRowsParams {
     int nbuf;                 // 2: the tiles are double-buffered (async only), 1: loaded in place
     float scale, softcap;
     int out_ld;               // operand-type elements between consecutive tokens of `out` (H*dv unless the heads are written into a wider row)
-    int sms;                  // SMs of the device (attn_tile_kernel)
+    int turn;                 // attn_tile_kernel: CTA from which on the query tiles go out in the opposite order (0: none)
     int has_out_scale;        // 1: the output row times out_scale (a mixer that is summed with another one at a fixed weight)
     float out_scale;
     PosSrc ps;

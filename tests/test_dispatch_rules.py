@@ -59,3 +59,8 @@ def test_attention_tiles(rules):
     for row, large in zip(ATTENTION, rules(calls)):
         times = row[5:]
         assert times[large] <= 1.03 * min(times), row
+
+
+def test_order_of_the_large_tiles(rules):
+    """turns only where two CTAs share an SM: 114,688 bytes (128-wide heads) twice, 147,456 (192-wide keys, 128-wide values) once"""
+    assert rules([f'printf("%d ", attn_order_turns_at(148, {b}));' for b in (114688, 115712, 115713, 147456)]) == [148, 148, 0, 0]
