@@ -24,5 +24,10 @@ inline bool attn_large_tiles(int sms, int T, int columns, int HC) {
 // Returns the CTA from which on the order turns, 0: none.
 inline int attn_order_turns_at(int sms, long long smem) { return 2 * (smem + 1024) <= 228 * 1024 ? sms : 0; }
 
+// Two-SM products (dense_gemm.cuh): does a CTA get an SM's whole ring?  Only when all clusters then run at once; `at_once` is what the device
+// says of one CTA per SM, which for clusters of four is less than its SMs hold (33 on 148).  36 of them (512 x 2304, K 2048) take 24.7 us
+// with the whole ring, 15.7 with half of it and two CTAs on some SMs; 32 of them (512 x 2048) 13.1 and 13.3.
+inline bool gemm_whole_sm(long long clusters, int at_once) { return clusters <= at_once; }
+
 }  // namespace dense
 }  // namespace lmrs

@@ -23,6 +23,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "dense_dispatch.h"
 #include "dense_ops.cuh"
 
 namespace lmrs {
@@ -270,7 +271,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
 // CTA stages its own 128 rows of A and half of the BN rows of W, one thread of the even CTA issues M = 256 MMAs that read both
 // CTAs' shared memory, and each CTA's TMEM receives its own 128 rows x BN columns.  Twice the outputs per operand row.
 //   BN 256   stages of 32 KB.  With more CTAs than SMs two share an SM (3 stages and 256 TMEM columns each): one tile's epilogue runs under
-//            the other's MMAs.  With one CTA per SM it gets all of the ring: 6 stages
+//            the other's MMAs.  With one CTA per SM it gets all of the ring: 6 stages (gemm_whole_sm)
 //   BN 128   where 256-wide tiles would leave SMs without work: 3 stages of 24 KB, three CTAs per SM (4 stages and two CTAs: 90 us
 //            instead of 67 for the residual products of 2048 rows at width 3072)
 //   SPLIT 2  where even those would: two pairs (a cluster of four) take halves of K; each then finishes half of the columns, adding the
@@ -470,6 +471,7 @@ struct DenseGemmCtx {
     int* d_err = nullptr;
     std::map<std::pair<const void*, int>, CUtensorMap> wmaps;   // (weight matrix, box rows) -> tensor map
     bool attr_set[4][2] = {}, pair_attr_set[4][3] = {};
+    int at_once[2] = {};   // clusters of two and of four CTAs that run at the same time with one CTA per SM (0: not asked yet)
     ~DenseGemmCtx() { if (h_err) cudaFreeHost(h_err); }
 };
 // a [rows][row_bytes used of pitch_bytes] byte matrix, box 128 bytes x box_rows rows, 128B swizzle, zeros outside
@@ -480,6 +482,18 @@ inline bool tg_make_map(DenseGemmCtx& c, CUtensorMap* map, const void* base, siz
     cuuint32_t estr[2] = {1, 1};
     return c.enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+// (a cluster lies within one group of SMs, and the groups' sizes need not divide: 33 clusters of four on 148 SMs)
+template <typename K> inline int tg_clusters_at_once(K kernel, int cluster, size_t smem, int sms) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(cluster * sms); cfg.blockDim = dim3(TG_THREADS); cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) { (void)cudaGetLastError(); n = 0; }
+    return n > 0 ? n : sms / cluster;
 }
 template <typename AT, typename WT> inline bool dense_gemm_usable(int T, int K, int O, int lda) {
     if (!std::is_same<AT, __nv_bfloat16>::value || !std::is_same<WT, __nv_bfloat16>::value) return false;
@@ -552,9 +566,11 @@ inline int dense_gemm_launch(DenseGemmCtx& c, cudaStream_t st, int T, const AT* 
                 c.pair_attr_set[EPI][form] = true;
             }
             const int cluster = form == 2 ? 4 : 2, oc = bn / (GLU ? 2 : 1);
+            int& at_once = c.at_once[form == 2];
+            if (!at_once) at_once = tg_clusters_at_once(kernel, cluster, tg_pair_smem(bn, tg_pair_stages(bn, form == 2 ? 2 : 1, true)), c.sms);
             cudaLaunchConfig_t cfg{};
             cfg.gridDim = dim3((O + oc - 1) / oc * cluster, (T + 255) / 256); cfg.blockDim = dim3(TG_THREADS); cfg.stream = st;
-            p.stages = tg_pair_stages(bn, form == 2 ? 2 : 1, (int)(cfg.gridDim.x * cfg.gridDim.y) <= c.sms);
+            p.stages = tg_pair_stages(bn, form == 2 ? 2 : 1, gemm_whole_sm((long long)cfg.gridDim.x / cluster * cfg.gridDim.y, at_once));
             cfg.dynamicSmemBytes = tg_pair_smem(bn, p.stages);
             cudaLaunchAttribute attr[1];
             attr[0].id = cudaLaunchAttributeClusterDimension;

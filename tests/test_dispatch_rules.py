@@ -64,3 +64,8 @@ def test_attention_tiles(rules):
 def test_order_of_the_large_tiles(rules):
     """turns only where two CTAs share an SM: 114,688 bytes (128-wide heads) twice, 147,456 (192-wide keys, 128-wide values) once"""
     assert rules([f'printf("%d ", attn_order_turns_at(148, {b}));' for b in (114688, 115712, 115713, 147456)]) == [148, 148, 0, 0]
+
+
+def test_ring_of_the_two_sm_products(rules):
+    """clusters of four: 33 at once with one CTA per SM; more of them share SMs instead of forming a second wave"""
+    assert rules([f'printf("%d ", gemm_whole_sm({n}, 33));' for n in (32, 33, 34, 37, 74)]) == [1, 1, 0, 0, 0]
