@@ -12,7 +12,7 @@ namespace dense {
 // of 128 behind 2000 keys take 1393 us a call (2 layers) with the large tiles, which occupy 32 SMs, and 1107 us with the small ones; 64 tokens of 24
 // heads on 8 KV heads of 128 1310 and 1084.  From the first CTA that has to wait for another one on the large tiles win: 192 tokens of those 24 heads
 // (312 small tiles) 507 us a layer behind 2000 keys against 733 (without earlier keys 157 against 153), 256 tokens of 32 heads of 64 (512) 308
-// against 519.  64-wide heads between 148 and 296 small tiles draw within 2 %.
+// against 519.  64-wide heads between 148 and 296 small tiles draw within 2 % (6 % for the small ones at 768 tokens of 4 heads).
 inline bool attn_large_tiles(int sms, int T, int columns, int HC) {
     const int tokens = std::max(1, 16 / HC);
     return (long long)columns * ((T + tokens - 1) / tokens) > 2LL * sms;
@@ -28,6 +28,45 @@ inline int attn_order_turns_at(int sms, long long smem) { return 2 * (smem + 102
 // says of one CTA per SM, which for clusters of four is less than its SMs hold (33 on 148).  36 of them (512 x 2304, K 2048) take 24.7 us
 // with the whole ring, 15.7 with half of it and two CTAs on some SMs; 32 of them (512 x 2048) 13.1 and 13.3.
 inline bool gemm_whole_sm(long long clusters, int at_once) { return clusters <= at_once; }
+
+// The bf16 product of more than 128 rows, one matrix: the one-CTA kernel (128 rows x 128 or 64 columns) or one of the two-SM forms (256 rows x 256,
+// x 128, or x 128 with K split over two pairs).  None wins everywhere: the large tiles move fewer operand bytes per output, but fewer of them
+// fill the SMs less evenly, their single epilogue is longer, and a half-empty 256-row tile costs what a full one does.  So the time of each is
+// estimated from how its tiles fall on the SMs,
+//     rounds x epilogue + max(rounds x K x latency, tiles on the busiest SM x K x rate),     rounds = tiles on the busiest SM / CTAs that share it,
+// with constants fitted to 4064 products on the 4 kernels, timed on a B200 (129 - 2048 rows, 256 - 12288 columns, K 256 - 12288, weights from
+// HBM).  Against the best kernel for each of them the estimate's choice loses 0.2 % on average (5 % or more for 1.2 % of them, 31 % for one of 2048
+// rows, 6144 columns and K 8192); choosing by columns per SM alone, with the one-CTA kernel only for few tiles and K < 1024, lost 10 %, and a third of
+// the products were slower than on the one-CTA kernel.
+// us on one CTA | 256 | 128 | split: 257 x 12288 gate/up, K 4096: 99 | 127 | 104 | 156;
+// 384 x 5120 added to the residual, K 256: 7.6 | 16.2 | 11.9 | 18.6;
+// 512 x 2048 added to the residual, K 8192: 45 | 51 | 44 | 27;
+// 512 x 9216 gate/up, K 2048: 51 | 42 | 52 | 80;
+// 2048 x 3072 added to the residual, K 8192: 133 | 112 | 85 | 115.
+enum { GEMM_BY_SIZE = -2, GEMM_ONE_CTA = -1, GEMM_256 = 0, GEMM_128 = 1, GEMM_SPLIT = 2 };
+inline bool gemm_narrow(bool glu, int T, int O, int sms) {   // one-CTA kernel: 64-wide tiles when 128-wide ones would not give every SM a CTA
+    return !glu && O > 64 && (long long)((O + 127) / 128) * ((T + 127) / 128) < sms;
+}
+inline int gemm_form(bool glu, int T, int K, int O, int sms, int pairs, int quads) {   // pairs, quads: clusters of two and four at once
+    struct Cost { float latency, rate, epi, epi_glu; };   // us per 1000 of K; us per 1000 of K and tile; us
+    static const Cost cost[5] = {{6.2f, 3.0f, 7.8f, 11.6f}, {5.4f, 5.3f, 15.8f, 22.1f}, {4.9f, 3.1f, 8.6f, 12.3f}, {2.2f, 1.8f, 8.4f, 10.4f},
+                                 {4.6f, 2.9f, 5.7f, 5.7f}};   // one CTA, 256, 128, split; one CTA with 64-wide tiles
+    const auto up = [](long long a, long long b) { return (a + b - 1) / b; };
+    const auto estimate = [&](const Cost& c, long long tiles, int at_once, int shared) {
+        const double load = (double)up(tiles, at_once), rounds = (double)up((long long)load, shared), k = K * 1e-3;
+        return rounds * (glu ? c.epi_glu : c.epi) + std::max(rounds * k * c.latency, load * k * c.rate);
+    };
+    const bool narrow = gemm_narrow(glu, T, O, sms);
+    int best = GEMM_ONE_CTA;
+    double least = estimate(cost[narrow ? 4 : 0], up(O, glu || narrow ? 64 : 128) * up(T, 128), sms, 2);
+    for (int f = GEMM_256; f <= GEMM_SPLIT; f++) {
+        if (f == GEMM_SPLIT && K <= 64) continue;   // each half needs a stage of K
+        const int columns = (f == GEMM_256 ? 256 : 128) / (glu ? 2 : 1);
+        const double t = estimate(cost[f + 1], up(O, columns) * up(T, 256), f == GEMM_SPLIT ? quads : pairs, f == GEMM_128 ? 3 : 2);
+        if (t < least) { least = t; best = f; }
+    }
+    return best;
+}
 
 }  // namespace dense
 }  // namespace lmrs

@@ -10,7 +10,7 @@
 // tensor maps carry the true extents, TMA fills rows >= T, weight rows >= O and the K tail with zeros, and the epilogue
 // masks its stores.  What the shape must satisfy: K and lda multiples of 8 elements (16-byte row pitch) and 16-byte
 // aligned bases.  Three stages of 32 KB leave room for two CTAs per SM: one tile's epilogue runs under the other's MMAs.
-// Prompts of more than 128 rows run on a two-SM form of the same kernel, further down.
+// Prompts of more than 128 rows may run on a two-SM form of the same kernel, further down (gemm_form).
 // Every wait is bounded: a wait that runs out raises a flag in mapped host memory, the roles stop, in-flight copies are
 // waited for (bounded again), TMEM is freed and the kernel returns; the next launch reports the flag.
 #pragma once
@@ -272,10 +272,11 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
 // CTAs' shared memory, and each CTA's TMEM receives its own 128 rows x BN columns.  Twice the outputs per operand row.
 //   BN 256   stages of 32 KB.  With more CTAs than SMs two share an SM (3 stages and 256 TMEM columns each): one tile's epilogue runs under
 //            the other's MMAs.  With one CTA per SM it gets all of the ring: 6 stages (gemm_whole_sm)
-//   BN 128   where 256-wide tiles would leave SMs without work: 3 stages of 24 KB, three CTAs per SM (4 stages and two CTAs: 90 us
-//            instead of 67 for the residual products of 2048 rows at width 3072)
-//   SPLIT 2  where even those would: two pairs (a cluster of four) take halves of K; each then finishes half of the columns, adding the
+//   BN 128   twice as many tiles, shorter epilogues: 3 stages of 24 KB, three CTAs per SM (4 stages and two CTAs: 90 us instead of 67 for the
+//            residual products of 2048 rows at width 3072)
+//   SPLIT 2  for few tiles and a long K: two pairs (a cluster of four) take halves of K; each then finishes half of the columns, adding the
 //            other's sums, which arrive through distributed shared memory, in a fixed order.  4 stages, or 8 with one CTA per SM
+// Which form, or the kernel above: gemm_form.
 // EPI_GLU: the even CTA's half of W are gate rows, the odd one's the same up rows: accumulator columns c and c + BN / 2.
 // Barriers: the copies of both CTAs complete on the even CTA's `full`; the MMA's commit frees the stage in both.  Every mbarrier wait
 // is bounded as in the kernel above.
@@ -472,6 +473,7 @@ struct DenseGemmCtx {
     std::map<std::pair<const void*, int>, CUtensorMap> wmaps;   // (weight matrix, box rows) -> tensor map
     bool attr_set[4][2] = {}, pair_attr_set[4][3] = {};
     int at_once[2] = {};   // clusters of two and of four CTAs that run at the same time with one CTA per SM (0: not asked yet)
+    int form = GEMM_BY_SIZE;   // option: this form for every product of more than 128 rows that it can serve
     ~DenseGemmCtx() { if (h_err) cudaFreeHost(h_err); }
 };
 // a [rows][row_bytes used of pitch_bytes] byte matrix, box 128 bytes x box_rows rows, 128B swizzle, zeros outside
@@ -483,17 +485,23 @@ inline bool tg_make_map(DenseGemmCtx& c, CUtensorMap* map, const void* base, siz
     return c.enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
-// (a cluster lies within one group of SMs, and the groups' sizes need not divide: 33 clusters of four on 148 SMs)
-template <typename K> inline int tg_clusters_at_once(K kernel, int cluster, size_t smem, int sms) {
+// clusters of the two-SM form that run at the same time with one CTA per SM (a cluster lies within one group of SMs, and the groups' sizes
+// need not divide: 33 clusters of four on 148 SMs)
+template <int EPI, int BN, int SPLIT> inline int tg_clusters_at_once(int sms) {
+    const size_t smem = tg_pair_smem(BN, tg_pair_stages(BN, SPLIT, true));
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(cluster * sms); cfg.blockDim = dim3(TG_THREADS); cfg.dynamicSmemBytes = smem;
+    cfg.gridDim = dim3(2 * SPLIT * sms); cfg.blockDim = dim3(TG_THREADS); cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[0].val.clusterDim.x = 2 * SPLIT; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) { (void)cudaGetLastError(); n = 0; }
-    return n > 0 ? n : sms / cluster;
+    if (cudaFuncSetAttribute(gemm_bf16_pair_kernel<EPI, BN, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, gemm_bf16_pair_kernel<EPI, BN, SPLIT>, &cfg) != cudaSuccess) {
+        (void)cudaGetLastError();
+        n = 0;
+    }
+    return n > 0 ? n : sms / (2 * SPLIT);
 }
 template <typename AT, typename WT> inline bool dense_gemm_usable(int T, int K, int O, int lda) {
     if (!std::is_same<AT, __nv_bfloat16>::value || !std::is_same<WT, __nv_bfloat16>::value) return false;
@@ -525,20 +533,16 @@ inline int dense_gemm_launch(DenseGemmCtx& c, cudaStream_t st, int T, const AT* 
         if ((reinterpret_cast<uintptr_t>(a) & 15) || (reinterpret_cast<uintptr_t>(w) & 15) || (w2 && (reinterpret_cast<uintptr_t>(w2) & 15))) return -1;
         if (*c.h_err) { err = "a tensor-core matrix product gave up waiting on one of its barriers (device status flag set)"; return 1; }
         constexpr bool GLU = EPI == EPI_GLU;
-        // Two-SM tiles for ungrouped products of more than 128 rows.  The form whose CTAs, spread over the SMs, do the fewest columns
-        // one after the other; 128-wide tiles move half as many outputs per operand byte of W, which costs about a sixth
-        int form = -1;   // 0: 256 columns, 1: 128 columns, 2: 128 columns and K split over two pairs
-        if (n_groups == 0 && T > 128) {
-            const int ty = (T + 255) / 256;
-            const auto ctas = [&](int bn) { const int oc = GLU ? bn / 2 : bn; return 2 * ty * ((O + oc - 1) / oc); };
-            const auto rounds = [&](int n) { return (n + c.sms - 1) / c.sms; };
-            form = rounds(ctas(256)) * 256 * 6 <= rounds(ctas(128)) * 128 * 7 ? 0 : 1;
-            if (form == 1 && ctas(128) <= c.sms) form = K >= 1024 ? 2 : -1;   // few tiles and a short K: the one-CTA kernel's smaller tiles
-            if (ty > 65535) form = -1;
+        int form = GEMM_ONE_CTA;   // two-SM tiles: ungrouped products of more than 128 rows
+        if (n_groups == 0 && T > 128 && (T + 255) / 256 <= 65535) {
+            if (!c.at_once[0]) {
+                c.at_once[0] = tg_clusters_at_once<EPI, 128, 1>(c.sms);
+                c.at_once[1] = tg_clusters_at_once<EPI, 128, 2>(c.sms);
+            }
+            form = c.form == GEMM_BY_SIZE || (c.form == GEMM_SPLIT && K <= 64) ? gemm_form(GLU, T, K, O, c.sms, c.at_once[0], c.at_once[1]) : c.form;
         }
-        // 64-wide tiles when 128-wide ones would not give every SM a CTA
         const size_t w_rows = n_groups > 0 ? (size_t)n_groups * O : (size_t)O;
-        const bool narrow = form < 0 && !GLU && O > 64 && ((O + 127) / 128) * ((T + TG_M - 1) / TG_M) < c.sms;
+        const bool narrow = form < 0 && gemm_narrow(GLU, T, O, c.sms);
         const int box_rows = form >= 0 ? (form == 0 ? 128 : 64) : (GLU || narrow) ? 64 : 128;
         auto wmap = [&](const void* base, CUtensorMap* out) {
             auto key = std::make_pair(base, box_rows * 1000003 + (int)(w_rows % 1000003));
@@ -566,11 +570,9 @@ inline int dense_gemm_launch(DenseGemmCtx& c, cudaStream_t st, int T, const AT* 
                 c.pair_attr_set[EPI][form] = true;
             }
             const int cluster = form == 2 ? 4 : 2, oc = bn / (GLU ? 2 : 1);
-            int& at_once = c.at_once[form == 2];
-            if (!at_once) at_once = tg_clusters_at_once(kernel, cluster, tg_pair_smem(bn, tg_pair_stages(bn, form == 2 ? 2 : 1, true)), c.sms);
             cudaLaunchConfig_t cfg{};
             cfg.gridDim = dim3((O + oc - 1) / oc * cluster, (T + 255) / 256); cfg.blockDim = dim3(TG_THREADS); cfg.stream = st;
-            p.stages = tg_pair_stages(bn, form == 2 ? 2 : 1, gemm_whole_sm((long long)cfg.gridDim.x / cluster * cfg.gridDim.y, at_once));
+            p.stages = tg_pair_stages(bn, form == 2 ? 2 : 1, gemm_whole_sm((long long)cfg.gridDim.x / cluster * cfg.gridDim.y, c.at_once[form == GEMM_SPLIT]));
             cfg.dynamicSmemBytes = tg_pair_smem(bn, p.stages);
             cudaLaunchAttribute attr[1];
             attr[0].id = cudaLaunchAttributeClusterDimension;

@@ -570,6 +570,7 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
         else if (!strcmp(name, "tensor_cores")) use_tc = value;
         else if (!strcmp(name, "graphs")) { use_graph = value; if (!value) drop_graphs(); }
         else if (!strcmp(name, "attn_tiles")) attn_tiles = value;
+        else if (!strcmp(name, "gemm_form")) gemm_ctx.form = std::max(-2, std::min(2, value));
         else if (!strcmp(name, "pdl")) { use_pdl = value; drop_graphs(); }
         else set_model_option(name, value);
     }
