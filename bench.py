@@ -1,6 +1,6 @@
 #!/usr/bin/env python
-"""bench.py -- headline benchmark of the lm.rs hot path on B200 (decode tok/s + prefill tok/s,
-Llama-3.2-1B Q8_0, vs the CPU path, with the HBM roofline fraction).
+"""bench.py -- headline benchmark of the lm.rs hot path on B200 (decode tok/s + prefill tok/s, Llama-3.2-1B Q8_0, vs the CPU
+path, with the HBM roofline fraction).
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl b200|reference] [--model NAME] [--pos P]
     python -m torch.distributed.run --nproc-per-node N ... bench.py --gpus N ...      (N > 1, one rank per GPU)
@@ -35,7 +35,7 @@ import threading
 import time
 
 # the process group of this benchmark only carries barriers and the max-reduce of the timings: no NVLink-SHARP multicast
-# buffers to set up and tear down (the decode data path does not use NCCL at all, DESIGN.md section 6)
+# buffers to set up and tear down (the decode data path does not use NCCL at all)
 os.environ.setdefault("NCCL_NVLS_ENABLE", "0")
 ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path[:0] = [os.path.join(ROOT, "lm.rs_b200"), os.path.join(ROOT, "oracle")]
@@ -564,7 +564,7 @@ def main():
     m.set_stream(stream.cuda_stream)
     toks = np.random.default_rng(2).integers(0, a.vocab_size, args.warmup + args.steps)
     pos = args.pos
-    for i in range(args.warmup):       # warm-up and timed steps cover the SAME positions P..P+K-1 (BASELINE: "64 tokens at pos 512")
+    for i in range(args.warmup):       # warm-up and timed steps cover the SAME positions P..P+K-1 (64 tokens at position 512)
         m.forward_device(int(toks[i]), pos + (i % args.steps))
     barrier()
     l0 = m.kernel_launches()

@@ -3,9 +3,9 @@
  * quantized transformer forward path.
  *
  * The reference (samuel-vitorino/lm.rs) has no FFI/plugin interface; its drop-in boundary is the pub
- * API of `lmrs::transformer` that the chat/backend bins call (SURVEY.md section 8b).  Every entry point
+ * API of `lmrs::transformer` that the chat/backend bins call.  Every entry point
  * below names the reference item it replaces (paths relative to the reference repo).  A Rust shim with
- * the identical pub surface forwards to these symbols (lm.rs_b200/rust/, INTEGRATION.md).
+ * the identical pub surface forwards to these symbols (lm.rs_b200/rust/).
  *
  * Conventions: plain pointers and sizes, no C++/torch types.  Every function returns 0 on success and a
  * non-zero status on failure; lmrs_b200_last_error() then returns a thread-local message.  (The
@@ -46,7 +46,7 @@ typedef struct lmrs_b200 lmrs_b200_t;
  * device = CUDA ordinal (-1: current device). */
 int lmrs_b200_create(const uint8_t* file, size_t len, int device, lmrs_b200_t** out, size_t* end_offset);
 
-/* Row-sharded variant for N GPUs, one process per GPU (BASELINE north_star; SURVEY.md section 8e): rank r
+/* Row-sharded variant for N GPUs, one process per GPU: rank r
  * of world owns head-aligned output-row shards of wq/wk/wv/w1/w3 and input-column shards of wo/w2, and
  * all-reduces the residual contribution twice per layer.  nccl_unique_id: the 128 bytes produced by
  * lmrs_b200_nccl_unique_id() on rank 0 and broadcast by the caller (torch.distributed/MPI/...). */
@@ -57,7 +57,7 @@ int lmrs_b200_nccl_unique_id(void* out128);
 /* impl Drop for Transformer                                      src/transformer.rs:688-711 */
 void lmrs_b200_destroy(lmrs_b200_t* m);
 
-/* Transformer::new on `n_gpus` GPUs of THIS process (devices 0 .. n_gpus-1), the form SURVEY.md section 8b proposes: one
+/* Transformer::new on `n_gpus` GPUs of THIS process (devices 0 .. n_gpus-1): one
  * handle per GPU behind the returned one, weights row-sharded like create_sharded, the GPUs mapped into one another with
  * cudaDeviceEnablePeerAccess and exchanging their partial results from inside the kernels (no NCCL, no second process, no
  * host synchronisation between the GPUs).  Every entry point below accepts the returned handle and drives all GPUs from

@@ -91,7 +91,7 @@ LMRS_DEVINL void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory");
 LMRS_DEVINL void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---- "LL" activation exchange between co-resident kernels of one decode step --------------------------------
-// A gpu-scope release/acquire pair costs ~1 us on B200 (each fence ~0.5 us, tools/micro/barrier_probe.cu) and a
+// A gpu-scope release/acquire pair costs ~1 us on B200 (each fence ~0.5 us) and a
 // kernel boundary 2-3 us (griddepcontrol.wait + first loads).  The decode chain therefore hands activations over
 // WITHOUT fences: every element travels as one 64-bit word (f32 bits | step sequence number << 32) written with a
 // single relaxed 8-byte store (single-copy atomic), and a consumer polls the words themselves until they carry the

@@ -30,7 +30,7 @@ LMRS_HD float matmul_f32_element(const float* xr, const float* wr, int n) {
 }
 
 // `matmul_rest` (:252-280): eight lane accumulators over the chunks, final_sum = 0 + reduce_add, then the tail -- which
-// reads x[r] of the FIRST row whatever row is being computed (:273-275; kept)
+// reads x[r] of the FIRST row whatever row is being computed (:273-275; kept: the numbers are the reference's)
 LMRS_HD float matmul_rest_element(const float* xr, const float* x_row0, const float* wr, int n) {
     float lanes[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
     const int n_simd = n / 8;

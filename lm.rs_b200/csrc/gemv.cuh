@@ -23,8 +23,8 @@
 // accumulator in ascending group order starting from 0.0 (a 16-step shuffle scan per half-warp), so
 // matmul_q8/matmul_q4 results are BIT-IDENTICAL to the CPU path; -fmad=false keeps mul/add unfused.
 //
-// The kernel is specialised on (prologue, epilogue, exchange mode): a launch only carries the code it runs (round 1
-// shipped ONE kernel with three prologues x five epilogues whose top stall was instruction fetch).  Exchange mode LL:
+// The kernel is specialised on (prologue, epilogue, exchange mode): a launch only carries the code it runs (ONE
+// kernel with three prologues x five epilogues had instruction fetch as its top stall).  Exchange mode LL:
 // the activations between the kernels of a decode step travel as (value, sequence) words polled by the consumer
 // (common.cuh), the kernels are launched early (programmatic dependent launch) and never call griddepcontrol.wait, so
 // consecutive kernels are co-resident (<= 128 registers, two CTAs per SM) and a hand-over costs a poll, not a kernel

@@ -1325,7 +1325,7 @@ static int create_common(const uint8_t* file, size_t len, int device, int rank, 
     m->rank = rank; m->world = world;
     m->use_graph = env_int("LMRS_B200_GRAPH", 1) != 0;
     m->use_pdl = env_int("LMRS_B200_PDL", 1) != 0;
-    // ring geometry: 16 warps x 2 stages measured best for the decode chain (profiles/r2_decode_experiments.md): the exact-
+    // ring geometry: 16 warps x 2 stages measured best for the decode chain: the exact-
     // order prologues and the per-stage scans are latency chains that want warps, deeper rings measured slower
     m->gemv_cfg = env_int("LMRS_B200_GEMV_CFG", 3);
     if (m->gemv_cfg < 0 || m->gemv_cfg >= N_GEMV_CFG) m->gemv_cfg = 0;
@@ -1333,8 +1333,7 @@ static int create_common(const uint8_t* file, size_t len, int device, int rank, 
     // Hand-over between the kernels of a step.  Default: kernel boundaries (programmatic dependent launch +
     // griddepcontrol.wait), one matrix-vector CTA per SM.  LMRS_B200_LL=1: fence-free LL exchange between co-resident
     // kernels (common.cuh) -- bit-identical and covered by the tests, but measured SLOWER on B200 (an L2 round trip costs
-    // 0.3-0.6 us, a hand-over needs two or three of them, and co-resident waiting kernels slow the running one; see
-    // profiles/r2_decode_experiments.md), so it is opt-in.
+    // 0.3-0.6 us, a hand-over needs two or three of them, and co-resident waiting kernels slow the running one), so it is opt-in.
     m->use_ll = env_int("LMRS_B200_LL", 0) != 0 && world == 1;
     m->use_pf_attn = env_int("LMRS_B200_PF_ATTN", 1);
     m->pfa_quads = env_int("LMRS_B200_PFA_QUADS", 4) == 8 ? 8 : 4;

@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(512) prefill_av_kernel(const PrefillAttnParams
 // accumulators are stored pair-interleaved) and the K / V operand of a step is a scalar the packed instruction broadcasts.
 // The first build of this kernel (one row per 8-lane group, q and K re-read from shared memory for every 4 multiply-adds) was
 // bound by the shared-memory pipe, not by arithmetic (ncu: short-scoreboard stalls 5x the issue slots, a 128-bit LDS costs a
-// warp four pipe cycles whatever it broadcasts; profiles/r2_ncu_prefill_attn_raw.csv), so the work is register-tiled:
+// warp four pipe cycles whatever it broadcasts), so the work is register-tiled:
 //   scores   NQD warps = row quads x 32 lanes; thread (quad, lane j) owns the 4 x 4 tile of rows {two pairs} x positions
 //            4j..4j+3 of every 128-position K tile (K transposed to [d][position]): per d ONE 16-byte load of the two q pairs
 //            and ONE of four K values feed 8 packed multiply/add pairs = 16 ascending-d chains;

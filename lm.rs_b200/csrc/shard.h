@@ -1,5 +1,5 @@
 // shard.h -- multi-GPU exchange for the row-sharded forward (one process per GPU).  The reference has no
-// distributed code at all; the sharding scheme is the one BASELINE.json's north_star defines:
+// distributed code at all; the sharding scheme is head-aligned output rows and input columns:
 // two sums of the dim-sized residual contribution per block + one logits gather per token.  Default data path: the peer
 // exchange fused into the kernels (common.cuh: every GPU pushes its partial into all peers' buffers over NVLink); NCCL
 // only bootstraps it (all-gather of the IPC handles) and remains as the fallback data path (LMRS_B200_PEER=0).

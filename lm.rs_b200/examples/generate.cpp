@@ -8,7 +8,7 @@
 //                GENERATE_SERIAL=1   the reference's own call pattern: one forward() per prompt token, logits to the host,
 //                                    host argmax (chat.rs:196-214, sampler.rs:109-113)
 // Maps the model file like the reference does (memmap2, chat.rs:60-65) and hands it to lmrs_b200_create.  Default call
-// pattern = what the GPU path makes worthwhile in a caller (SURVEY.md section 8f-3): the prompt's embeddings go through ONE
+// pattern = what the GPU path makes worthwhile in a caller: the prompt's embeddings go through ONE
 // batched fill_kv_cache (the multimodal bins already do this, chat.rs:110-119; row-wise identical results for LLAMA / PHI),
 // the last prompt token and every generated one through generate_greedy (pick and feedback on the device).
 // There is no CPU fallback: without an sm_100 device the create call fails and this exits 1.

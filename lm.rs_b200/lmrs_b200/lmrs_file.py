@@ -70,7 +70,7 @@ def parse_header(buf) -> LmrsArgs:
     return LmrsArgs(*f)
 
 
-# name -> header values of the checkpoints the reference README lists (SURVEY.md section 8 preamble)
+# name -> header values of the checkpoints the reference README lists
 MODEL_SHAPES = {
     "llama-3.2-1b": dict(dim=2048, hidden_dim=8192, n_layers=16, n_heads=32, head_size=64, n_kv_heads=8,
                          vocab_size=128256, seq_len=131072, rms_norm_eps=1e-5, rope_theta=500000.0, model_type=LLAMA),
@@ -150,7 +150,7 @@ def file_size(a: LmrsArgs) -> int:
 
 
 def decode_bytes_per_token(a: LmrsArgs, pos: int | None = None) -> int:
-    """ALGORITHMIC HBM bytes one decode step must move (SURVEY.md section 8d): every layer matrix and the
+    """ALGORITHMIC HBM bytes one decode step must move: every layer matrix and the
     classifier (q bytes + scales) once, the norm vectors, plus -- if pos is given -- the K/V rows read
     ((pos+1) * kv_dim * 4 * 2 per layer) and written (kv_dim*4*2 per layer)."""
     total = 0

@@ -65,7 +65,7 @@ class Transformer:
 
     @classmethod
     def new_sharded(cls, data, device: int, rank: int, world: int, nccl_unique_id: bytes):
-        """One process per GPU, output rows sharded across `world` ranks (SURVEY.md section 8e)."""
+        """One process per GPU, output rows sharded across `world` ranks."""
         buf = np.frombuffer(data, dtype=np.uint8) if not isinstance(data, np.ndarray) else np.ascontiguousarray(data, np.uint8)
         h, end = C.c_void_p(), C.c_size_t()
         idbuf = C.create_string_buffer(bytes(nccl_unique_id), 128) if world > 1 else None

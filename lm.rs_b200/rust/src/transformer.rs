@@ -17,7 +17,7 @@ use crate::quantization::{QuantType, QuantizedTensor};
 
 // ---- tensor views over the mapped file: `src/vision.rs:2` and `src/processor.rs:2` import these two helpers from this
 // module (reference src/transformer.rs:16-48), so the multimodal build needs them here too.  They stay host-side: the
-// vision tower still runs on the reference's CPU operators (or on the operator-level C ABI, INTEGRATION.md).
+// vision tower still runs on the reference's CPU operators (or on the operator-level C ABI).
 
 /// The next `n * size_each` f32 values of the file; advances `offset` past them.
 pub fn init_param<'a>(data: &'a [u8], offset: &mut usize, n: u32, size_each: u32) -> &'a [f32] {

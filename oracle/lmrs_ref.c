@@ -10,7 +10,7 @@
  * compiled here, so this restatement is validated only by hand-derived KATs
  * (tests/test_oracle_kat.py) and the reference's Python exporter (tests/golden/).
  *
- * Third-party arithmetic that is NOT in /root/reference: crate `wide` ^0.7.28
+ * Third-party arithmetic that is NOT in the reference's tree: crate `wide` ^0.7.28
  * (Cargo.toml:14; no Cargo.lock) supplies f32x8/i32x8.  Integer lanes are order-independent.
  * For f32x8::reduce_add this file uses the crate's AVX sequence as published
  * (add hi/lo 128-bit halves, then movehl, then lane 1):
@@ -171,7 +171,7 @@ void lmrs_ref_matmul_q8(float* xout, const int8_t* xq, const float* xs, const in
     matmul_q8_kshards(xout, xq, xs, wq, ws, rows, n, o, gs, 1);
 }
 /* `shards` > 1 is NOT a reference feature: it restates the summation order of lmrs_b200's row-sharded N-GPU mode
- *  so that N-GPU runs can be checked bit for bit: the K groups are split into `shards` equal
+ * so that N-GPU runs can be checked bit for bit: the K groups are split into `shards` equal
  * contiguous ranges, each range is accumulated from 0.0 in ascending order (one GPU's partial), and the partials are
  * added in ascending rank order starting from rank 0's. */
 static void matmul_q8_kshards(float* xout, const int8_t* xq, const float* xs, const int8_t* wq, const float* ws,

@@ -7,7 +7,7 @@
  * load this library.  The product (liblmrs_b200.so) never links or calls it.
  *
  * PARITY STATUS: "parity unpinned".  The reference ships no tests, golden vectors
- * or fixtures for this path (SURVEY.md section 4 / 8c) and its Rust crate cannot be built
+ * or fixtures for this path and its Rust crate cannot be built
  * in this image (no rustc/cargo; deps `wide`, `rayon` un-vendored).  The oracle is
  * pinned only by known-answer vectors hand-derived from the cited source lines
  * (tests/test_oracle_kat.py) and by the reference's *Python* exporter for the

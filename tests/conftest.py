@@ -11,7 +11,7 @@ for p in (os.path.join(ROOT, "lm.rs_b200"), os.path.join(ROOT, "oracle"), ROOT):
 
 
 def pytest_configure(config):
-    config.addinivalue_line("markers", "gpu: needs a real B200 (run with -m gpu on the GPU box)")
+    config.addinivalue_line("markers", "gpu: needs a real B200 (run with -m gpu)")
 
 
 @pytest.fixture(scope="session")

@@ -1,6 +1,6 @@
 """Generates the committed golden fixtures by RUNNING THE REFERENCE'S OWN PYTHON EXPORTER (export.py, utils/io.py,
-utils/quantization.py at /root/reference) on tiny seeded safetensors models.  Only runs in the authoring
-container (the GPU box has no /root/reference); the outputs are committed:
+utils/quantization.py) on tiny seeded safetensors models.  Only runs in the authoring
+container, where the reference lies beside; the outputs are committed:
 
     tests/golden/<name>.lmrs          the exporter's output, byte for byte
     tests/golden/<name>.src.npz       the f32 source tensors fed to the exporter (HF names)

@@ -1,5 +1,5 @@
 """LMRS v4 format: our layout/quantizer restatement vs files produced by the REFERENCE'S OWN exporter
-(tests/golden/*.lmrs, generated by tests/golden/make_golden.py from /root/reference/export.py)."""
+(tests/golden/*.lmrs, generated by tests/golden/make_golden.py with the reference's export.py)."""
 import os
 
 import numpy as np

@@ -1,7 +1,7 @@
 """Model-level parity on the GPU: Transformer.{new, forward, get_embeddings, fill_kv_cache} through the C ABI
 against the CPU oracle on identical synthetic LMRS files and prompts.
 
-Bar: BASELINE.json north_star asks for logits within 1e-3 max-abs of the CPU path.  Because the path re-quantizes
+Bar: logits within 1e-3 max-abs of the CPU path.  Because the path re-quantizes
 activations (discontinuous rounding), that is only reliably achievable by reproducing every f32 operation bit for
 bit (see lm.rs_b200/csrc/exact_math.cuh), so LLAMA/PHI logits, KV rows and residual streams are compared for
 EXACT equality; GEMMA goes through an f64 tanh (CUDA libdevice vs glibc) and keeps the 1e-3 tolerance."""
@@ -49,7 +49,7 @@ def test_forward_logits_match_oracle(gpu_lib, ref, synth, name, q_type):
 
 @pytest.mark.parametrize("name", ["ref_llama_q8", "ref_gemma_q4", "ref_phi_q8"])
 def test_files_written_by_the_reference_exporter(gpu_lib, ref, name):
-    """tests/golden/*.lmrs come from /root/reference/export.py itself (tests/golden/make_golden.py)."""
+    """tests/golden/*.lmrs come from the reference's export.py itself (tests/golden/make_golden.py)."""
     buf = np.fromfile(os.path.join(os.path.dirname(__file__), "golden", name + ".lmrs"), dtype=np.uint8)
     cpu = ref.RefTransformer(buf)
     gpu, end = gpu_lib.Transformer.new(buf)
@@ -144,7 +144,7 @@ def test_two_handles_are_independent(gpu_lib, ref, synth):
 
 
 def test_llama_1b_q8_full_shape(gpu_lib, ref, lf):
-    """BASELINE config 2 shape (Llama-3.2-1B Q8_0, synthetic weights): logits within 1e-3 at a few positions, incl.
+    """Llama-3.2-1B Q8_0 shape, synthetic weights: logits within 1e-3 at a few positions, incl.
     after a 96-embedding fill_kv_cache."""
     buf = lf.write_synthetic(lf.model_args("llama-3.2-1b", 1), seed=0, mode="fast")
     cpu = ref.RefTransformer(buf)
@@ -162,7 +162,7 @@ def test_llama_1b_q8_full_shape(gpu_lib, ref, lf):
 
 @pytest.mark.parametrize("name,q_type,layers", [("llama-3.2-3b", 2, 3), ("phi-3.5-mini", 1, 2), ("gemma-2-9b", 1, 2), ("llama-3.2-3b", 1, 2)])
 def test_full_shapes_of_the_other_baseline_configs(gpu_lib, ref, lf, name, q_type, layers):
-    """BASELINE configs 3-5 at their real dim / hidden / heads / head_size / vocabulary (Llama-3.2-3B Q4_0 and Q8_0,
+    """The other benchmarked models at their real dim / hidden / heads / head_size / vocabulary (Llama-3.2-3B Q4_0 and Q8_0,
     Phi-3.5-mini Q8_0 with its separate lm_head, Gemma-2-9B Q8_0 with dim 3584 = 28 groups and att_dim > dim), truncated to
     a few blocks so the CPU oracle finishes in seconds: a 40-embedding fill_kv_cache (tcgen05 GEMM path for Q8_0, per-token
     chain for Q4_0), then decode steps.  LLAMA / PHI bit for bit, GEMMA (f64 tanh in two libms) within 1e-3."""

@@ -84,7 +84,7 @@ def _worker(rank, world, port, out_dir, name, expect_error=None, peer=True, pf_r
 
 
 # tiny models only: on deeper random-weight models any f32 re-association flips activation-quantization codes and the
-# deviation is amplified far beyond 1e-3 (DESIGN.md section 2), which is exactly what the partial sums of N > 1 do
+# deviation is amplified far beyond 1e-3, which is exactly what the partial sums of N > 1 do
 def test_two_gpu_sharded_forward_matches_oracle(tmp_path):
     """NCCL fallback data path (collectives between the kernels)."""
     import torch

@@ -1,7 +1,7 @@
 """Known-answer tests that pin the CPU oracle (oracle/lmrs_ref.c) to the reference SOURCE semantics.
 
 The reference ships no tests or golden vectors for this path and its Rust crate cannot be built here
-("parity unpinned", SURVEY.md section 8c), so these vectors are hand-derived from the cited lines."""
+("parity unpinned"), so these vectors are hand-derived from the cited lines."""
 import numpy as np
 import pytest
 

@@ -1,4 +1,4 @@
-"""N > 1 path on CPU: the row-sharding scheme of lmrs_b200_create_sharded (SURVEY.md section 8e / DESIGN.md section 6) restated with the
+"""N > 1 path on CPU: the row-sharding scheme of lmrs_b200_create_sharded restated with the
 oracle's operators, run as 2 (and 4) `gloo` ranks: head-aligned row shards of Wq/Wk/Wv/W1/W3, 128-aligned input-column shards
 of Wo/W2, one sum-all-reduce of the dim-vector after Wo and after W2, vocab-row shards of the classifier + all-gather.
 Checks (a) the exchange plumbing bench.py uses (unique-id style byte broadcast, all_reduce, all_gather) and (b) that the
@@ -66,7 +66,7 @@ def _worker(rank, world, port, out_dir, name="tiny-llama", ordered=False):
         return [p_.numpy() for p_ in parts]
 
     def ordered_exchange(v):
-        """the peer exchange of lmrs_b200 (DESIGN.md section 6): every rank receives every partial and adds them in ascending
+        """the peer exchange of lmrs_b200: every rank receives every partial and adds them in ascending
         rank order starting from rank 0's -- deterministic, unlike the association inside an all-reduce"""
         parts = gather(v)
         total = parts[0].copy()
@@ -144,7 +144,7 @@ def _worker(rank, world, port, out_dir, name="tiny-llama", ordered=False):
 def test_row_sharding_matches_unsharded_logits(tmp_path, world, name):
     """2 ranks on the 2-layer model; 4 ranks on its 8-head / 4-KV-head variant (one KV head, 128 attention columns and 128
     hidden rows per rank).  Deeper models are not usable here: any f32 re-association flips activation-quantization codes
-    and a 4-layer model already deviates by 1.5e-2 with 4 ranks (DESIGN.md section 2)."""
+    and a 4-layer model already deviates by 1.5e-2 with 4 ranks."""
     torch = pytest.importorskip("torch")
     import torch.multiprocessing as mp
     port = _free_port()
