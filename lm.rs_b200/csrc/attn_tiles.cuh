@@ -1,6 +1,6 @@
 // attn_tiles.cuh -- attention of many query rows (prompts and long portions) in f32 on CUDA cores, as two register-tiled
-// products per key tile.  Same parameters and arithmetic rules as attn_rows_kernel (dense_ops.cuh), which serves steps of one
-// or a few rows.
+// products per key tile.  Same parameters and arithmetic rules as attn_rows_kernel (dense_ops.cuh), which serves one-row steps and the
+// portions that would leave SMs idle here (attn_large_tiles).
 #pragma once
 #include "dense_ops.cuh"
 
@@ -44,7 +44,8 @@ DN_DEVINL float lg2(float v) { float r; asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(
 // rows (p.v_in_k): no V tile, and the next K tile is copied after the values instead of under them.  QS: the pitch of the q and k
 // rows in shared memory (0: any, from dk; a pitch known here leaves the inner loop without address arithmetic).
 // KH 2: two groups of four warps take half of every tile's keys each, with sums of their own that meet at the end: 16 warps per SM
-// instead of 12 (71 -> 66 us; only one value block leaves the registers for it).
+// instead of 12 (512 tokens, 32 heads of 64: 71 -> 66 us before the order of the tiles was changed; only one value block leaves the
+// registers for it).
 template <typename AT, int NV, int QS, int KH, bool SIG, bool VK>
 static __global__ void __launch_bounds__(128 * KH, 2) attn_tile_kernel(const AttnRowsParams<AT> p) {
     extern __shared__ __align__(16) float ta_sm[];
@@ -283,7 +284,7 @@ static __global__ void __launch_bounds__(128 * KH, 2) attn_tile_kernel(const Att
         }
     }
     if constexpr (KH == 2) {   // the second group's (maximum, sum, output), one row of values per thread, through the idle tiles
-        constexpr int VALS = 4 * (8 * NV + 2);   // 40 or 72 x 128 floats: the q and k tiles hold at least 2 x 64 x 32, the values' tile the rest
+        constexpr int VALS = 4 * (8 * NV + 2);   // 40 x 128 floats: the q and k tiles hold at least 2 x 64 x 32 floats, the values' tile the rest
         static_assert(NV == 1 && !VK, "room for the exchange");
         const int tid = threadIdx.x & 127;
         __syncthreads();

@@ -966,8 +966,8 @@ static __global__ void __launch_bounds__(128) qkv_post_kernel(const QkvPostParam
 // row slot r = (token r / HC, head r % HC).  Keys are walked in tiles of 64 staged in shared memory: lane j scores keys j
 // and j + 32 of the tile for each of its rows (K rows padded so that the 16-byte reads of 32 lanes do not collide), an
 // online softmax keeps (max, sum) per row, the probabilities go through shared memory and lane c accumulates output
-// columns c, c + 32, ... .  Tiles start at multiples of 64 keys whatever the portion, so a row's arithmetic does not
-// depend on how the prompt was cut.  With nsplit > 1 (decode) CTA `split` walks tiles split, split + nsplit, ... and writes
+// columns c, c + 32, ... .  Tiles start at multiples of 64 keys whatever the portion, so within this kernel a row's arithmetic does
+// not depend on how the prompt was cut; portions that attn_large_tiles sends to attn_tile_kernel sum in another order.  With nsplit > 1 (decode) CTA `split` walks tiles split, split + nsplit, ... and writes
 // (max, sum, unnormalised row) to scratch for attn_combine_kernel.
 constexpr int ATT_KT = 64, ATT_WARPS = 4;
 // exp and tanh of the attention inner loop on the special-function unit: ex2.approx is good to about 2e-7 relative, and
