@@ -353,10 +353,12 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
         p.row_at = GV_SUMS_BYTES;
         if (row + GV_SUMS_BYTES > 227 * 1024) { p.ks = 1; p.row_at = GV_NORM_BYTES; }   // the widest rows leave no room for the slices' sums
         const size_t smem = row + p.row_at;
-        if (optin(gemv_rows_kernel<AT, WT, EPI, NORM>, smem)) return 1;
         const int gpc = 8 / p.ks, tasks = (groups + gpc - 1) / gpc, cap_x = std::max(1, 2 * sms / nb);
         const int rounds = (tasks + cap_x - 1) / cap_x;
-        return launch_k("gemv_rows_kernel", st, pdl_now, gemv_rows_kernel<AT, WT, EPI, NORM>, dim3((tasks + rounds - 1) / rounds, nb), dim3(GV_THREADS), smem, p);
+        const dim3 grid((tasks + rounds - 1) / rounds, nb);
+        auto go = [&](auto kernel) { return optin(kernel, smem) || launch_k("gemv_rows_kernel", st, pdl_now, kernel, grid, dim3(GV_THREADS), smem, p); };
+        const int u = gemv_pieces((pieces + p.ks - 1) / p.ks);
+        return u == 1 ? go(gemv_rows_kernel<AT, WT, EPI, NORM, 1>) : u == 2 ? go(gemv_rows_kernel<AT, WT, EPI, NORM, 2>) : go(gemv_rows_kernel<AT, WT, EPI, NORM, 4>);
     }
 
     template <int RW, int NI, bool SIG> int launch_attn_t(cudaStream_t st, AttnRowsParams<AT> p, int grid_x, int grid_y) {

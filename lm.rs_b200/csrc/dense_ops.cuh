@@ -581,7 +581,7 @@ template <int EPI, typename AT> DN_DEVINL void epi_apply(const EpiParams<AT>& e,
 
 // ---- one row times a matrix: W [O][K] streamed once ----------------------------------------------------------------------
 // Bound by HBM for large matrices and by latency for all of them: a decode step is a chain of such products of 8 to 70 MB, 1 to 10 us
-// each at full bandwidth.  So every lane has 16 loads of 16 bytes in flight (256 threads, two CTAs per SM: 19 MB over the chip), the
+// each at full bandwidth.  So every lane has 16 loads of 16 bytes in flight where rows are long enough (256 threads, two CTAs per SM: 19 MB over the chip), the
 // first of them issued before the input is waited for or normalised, and every register is loaded again as soon as it has been
 // used, across task borders.  A task is GV_ROWS weight rows (EPI_GLU: two gate rows and the same two up rows) times one of `ks` slices of
 // K, one per warp; the warps of a CTA that share rows add their slices in a fixed order.  The grid is persistent.  (Two rows per warp, 4
@@ -640,16 +640,21 @@ DN_DEVINL void widen16(const uint4& q, float (&v)[8], const __nv_bfloat16*) {
     for (int i = 0; i < 4; i++) { v[2 * i] = __uint_as_float(w[i] << 16); v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
 }
 template <typename WT> DN_DEVINL void load16(const WT* p, float (&v)[Vec16<WT>::N]) { widen16(ldcs16(p), v, p); }
-constexpr int GV_ROWS = 4, GV_PIECES = 4, GV_THREADS = 256;   // weight rows of a task, 16-byte pieces of each a lane has in flight
+constexpr int GV_ROWS = 4, GV_THREADS = 256;   // weight rows of a task
 // Shared memory before the staged input row: a norm's 33 sums, then, with K split, two copies of the warps' GV_ROWS sums in their place.
 // (Static arrays would come off what is left for the row: with 512 bytes of them a normalised f32 row of 57988 to 58052 columns found
 // no room.  And one size for every split: kernels that follow one another with 144 and 256 bytes cost a step of Tudatar 4 %.)
 constexpr int GV_NORM_BYTES = 36 * 4, GV_SUMS_BYTES = 2 * GV_THREADS / 32 * GV_ROWS * 4;
-template <typename AT, typename WT, int EPI, int NORM>
+// U: 16-byte pieces of each row a lane has in flight: 4, or as many as a short slice has at most (32 U pieces: gemv_pieces).  The form with four
+// walks the other pieces of a short row all the same: steps of small models were slower with it than with two rows per warp and 4 loads in flight
+// (us per greedily generated token, two rows | four pieces always | now: Bolapel, 4 layers, width 256: 98 - 103 | 108 | 104; Lutesun,
+// 2 layers, width 256: 86 | 91 | 80 - 86; Rupenex, 2 layers, width 128: 78 - 81 | 84 | 78; Tudatar, 4 layers, width 512: 162 | 160 | 150).
+inline int gemv_pieces(int per) { return per <= 32 ? 1 : per <= 64 ? 2 : 4; }
+template <typename AT, typename WT, int EPI, int NORM, int U>
 static __global__ void __launch_bounds__(GV_THREADS, 2) gemv_rows_kernel(const GemvRowsParams<AT, WT> pp) {
     static_assert(std::is_same<AT, WT>::value, "the input row has the weights' type");
     extern __shared__ __align__(16) unsigned char gv_sm[];   // [sums | the staged input row]
-    constexpr int N = Vec16<WT>::N, R = GV_ROWS, U = GV_PIECES, OUT = EPI == EPI_GLU ? R / 2 : R, NW = GV_THREADS / 32;
+    constexpr int N = Vec16<WT>::N, R = GV_ROWS, OUT = EPI == EPI_GLU ? R / 2 : R, NW = GV_THREADS / 32;
     float* red = reinterpret_cast<float*>(gv_sm);                              // a norm's sums
     float (*part)[NW][R] = reinterpret_cast<float (*)[NW][R]>(gv_sm);          // then, K split: two copies of the warps' sums
     GemvRowsParams<AT, WT> p = pp;

@@ -132,8 +132,8 @@ template <typename AT, typename WT> class GenetarModel : public DenseModel<AT, W
     int load(const std::string& dir, const Json& cfg, const ArchOptions& opt) {
         sms = opt.sms;
         gemm_ctx.sms = opt.sms;
-        B::use_pdl = 1;   // its decode chain is mostly one-row products that have their first weights in flight while they wait: 364 -> 342 us
-                          // per step (6 layers at width 2048), 84 -> 79 (3 layers at width 256)
+        B::use_pdl = 1;   // its decode chain is mostly one-row products that have their first weights in flight while they wait: 370 -> 346 us
+                          // per step (6 layers at width 2048, waited for on the host), 96 -> 85 (3 layers at width 256)
         width = (int)cfg.at("width").number(0);
         vocab = (int)cfg.at("vocab").number(0);
         if (width <= 0 || vocab <= 0) { error = "config.json: width and vocab are required"; return 1; }

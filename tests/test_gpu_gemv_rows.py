@@ -1,6 +1,6 @@
 """The one-row product (gemv_rows_kernel) at the edges of its split: rows that are one 16-byte piece, rows whose pieces do not fill a
 round of 32 lanes or a slice of K, one row more or less than a task, K split over two to eight warps, rows that do not start
-on 16-byte boundaries.  Decode steps of one-layer Genetar models against the float64 implementation, held to the tolerances of
+on 16-byte boundaries, rows of one and two rounds (one and two pieces in flight).  Decode steps of one-layer Genetar models against the float64 implementation, held to the tolerances of
 test_gpu_genetar.py (2e-4 and 4e-2 of the logits' root mean square)."""
 import numpy as np
 import pytest
@@ -12,7 +12,8 @@ TOL = {"float32": 2e-4, "bfloat16": 4e-2}
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
-@pytest.mark.parametrize("width,ff,vocab", [(8, 8, 5), (72, 1, 3), (264, 136, 61), (1032, 520, 65), (520, 2056, 64), (512, 4104, 33), (27, 23, 10)])
+@pytest.mark.parametrize("width,ff,vocab", [(8, 8, 5), (72, 1, 3), (264, 136, 61), (1032, 520, 65), (520, 2056, 64), (512, 4104, 33), (27, 23, 10),
+                                            (256, 512, 61), (128, 264, 33)])
 def test_decode_steps(gpu_lib, tmp_path, dtype, width, ff, vocab):
     check_one_layer(gpu_lib, tmp_path, dtype, width, ff, vocab)
 
