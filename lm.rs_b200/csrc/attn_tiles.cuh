@@ -126,7 +126,7 @@ static __global__ void __launch_bounds__(128 * KH, 2) attn_tile_kernel(const Att
         for (int e = threadIdx.x; e < TA_KEYS * (VS - v4); e += TA_THREADS) Vs[(e / (VS - v4)) * VS + v4 + e % (VS - v4)] = 0.0f;
     }
 
-    constexpr float LOG2E = 1.4426950408889634f;
+    constexpr float LOG2E = 1.4426950408889634f, MASKED = -1e30f * LOG2E;   // what a hidden key scores (scores are in powers of two here)
     float m[4], l[4];   // running maximum (of scores * log2(e)) and this lane's share of the sum
     f32pair o[4][4 * NV];
     int last[4];        // last visible key of row i (-1: no such row)
@@ -135,7 +135,7 @@ static __global__ void __launch_bounds__(128 * KH, 2) attn_tile_kernel(const Att
         const int r = rg + 4 * i, t = t0 + r / p.HC, hl = h0 + r % p.HC;
         const bool ok = r / p.HC < p.TQ && t < p.T && hl < kv_mul;
         last[i] = ok ? (int)pos0 + t : -1;
-        m[i] = !SIG && p.sink && ok && half == 0 ? p.sink[g * kv_mul + hl] * LOG2E : -1e30f;
+        m[i] = !SIG && p.sink && ok && half == 0 ? p.sink[g * kv_mul + hl] * LOG2E : MASKED;
         l[i] = (SIG || (p.sink && ok)) && cg == 0 && half == 0 ? 1.0f : 0.0f;
 #pragma unroll
         for (int c = 0; c < 4 * NV; c++) o[i][c] = 0ull;
@@ -222,7 +222,7 @@ static __global__ void __launch_bounds__(128 * KH, 2) attn_tile_kernel(const Att
                 for (int j = 0; j < J; j++) {
                     const int key = j0 + k0 + cg + 8 * j, dist = last[i] - key;
                     const bool vis = dist >= 0 && key >= first && (p.window <= 0 || dist < p.window || key < p.keep_first);
-                    if (!vis) { hidden |= 1u << j; a[j] = SIG ? 0.0f : -1e30f; }
+                    if (!vis) { hidden |= 1u << j; a[j] = SIG ? 0.0f : MASKED; }
                 }
             }
             if (!SIG) {

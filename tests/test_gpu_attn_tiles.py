@@ -41,6 +41,22 @@ def test_tile_edges(gpu_lib, tmp_path, heads, kv_heads, dim, vdim, n):
     m.close()
 
 
+def test_scores_as_low_as_the_other_kernel_takes_them(gpu_lib, tmp_path):
+    """a row whose only visible keys score between -1e30 and -1e30 / log2(e): still an average of their values"""
+    cfg = G.make_config([G.attention_layer("attention", heads=4, kv_heads=4, dim=16, vdim=16, ff=0, v_mix=False, scale=-5e28, softcap=None)], bigram=None)
+    W = G.random_weights(cfg, seed=3)
+    W["l0.mix.k"] = W["l0.mix.q"]   # q . k of a token with itself is 16: its score is -8e29
+    toks = np.random.default_rng(3).integers(0, cfg["vocab"], 40).tolist()
+    m = gpu_lib.Transformer.open(G.write_model(str(tmp_path / "m"), cfg, W), dtype="float32", max_tokens=64)
+    m.set_option("attn_tiles", 0)
+    want = m.forward_tokens(toks, 0, list(range(40)))
+    m.set_option("attn_tiles", 1)
+    got = m.forward_tokens(toks, 0, list(range(40)))
+    assert np.isfinite(want[0]).all() and np.isfinite(got).all()
+    assert G.rel_rms(got[0], want[0]) < 2e-4   # (later rows: a hard choice among 16-dimensional products, ties included)
+    m.close()
+
+
 @pytest.mark.parametrize("arch", ["tudatar", "rupenex", "badepel", "bolapel", "lutesun"])
 @pytest.mark.parametrize("shared_latent", [False, True])
 def test_forms_of_the_other_models(gpu_lib, tmp_path, arch, shared_latent):
