@@ -450,6 +450,10 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_con
             __syncwarp();
         }
     }
+    // After a give-up: a stage that only one CTA of the pair had asked for completes on no barrier that anyone waits for, and MMAs issued
+    // before it may still run.  Both get a millisecond to end before memory goes away.
+    if (threadIdx.x == 0 && *abort_flag)
+        for (int i = 0; i < 1000; i++) __nanosleep(1000);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     cluster_sync();   // nobody's shared memory, barriers or TMEM go away while another CTA of the cluster may still touch them
