@@ -23,7 +23,7 @@
 //                            per head instead of the softmax, per-head or per-element sigmoid output gates, grouped query
 //                            heads, query tile x KV head per CTA, K and V rows
 //                            with their own pitch (V may be a prefix of the K row: attention over a shared latent),
-//                            optional split over the keys (decode) + attn_combine_kernel; prompts run on attn_tiles.cuh
+//                            optional split over the keys (decode) + attn_combine_kernel; long portions run on attn_tiles.cuh
 // What the design wants in 32-bit (norms, scores, softmax, residual, angles) is 32-bit here in both operand types.
 #pragma once
 #include <cuda_bf16.h>

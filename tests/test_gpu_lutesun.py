@@ -203,7 +203,7 @@ def test_the_latent_space_and_the_per_head_form_agree(gpu_lib, tmp_path, dtype):
 
 
 def test_long_prompts_take_the_wide_query_tiles(gpu_lib, tmp_path):
-    """portions with enough rows for eight rows per warp (the grid covers the GPU twice) equal the same prompt in small portions"""
+    """portions with enough rows for 64-row tiles (more than two 16-row tiles per SM) equal the same prompt in small portions"""
     cfg = O.make_config([D(heads=12, dim=8, rot_dim=4, vdim=8, kv_rank=12, size=100, mlp=None), G(heads=12, dim=8, rot_dim=4, vdim=40, kv_rank=16, q_rank=16, size=0, mlp=None)],
                         width=32, vocab=60)
     n = 900
