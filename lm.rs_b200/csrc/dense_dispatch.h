@@ -18,6 +18,16 @@ inline bool attn_large_tiles(int sms, int T, int columns, int HC) {
     return (long long)columns * ((T + tokens - 1) / tokens) > 2LL * sms;
 }
 
+// Attention of T > 1 rows on the tensor cores (attn_tensor.cuh), or on CUDA cores (the two kernels below)?  What counts is how many keys a tile
+// of rows walks: a launch that splits keys and values and the first tile's latency cost about 20 us a layer more, then a tile of 128 keys takes
+// 5 us (128-wide heads) where attn_rows_kernel takes 20 or more.  us per call of 2 layers, the better CUDA-core kernel | tensor cores: 128 tokens behind 300, Llama-3.2-1B shapes
+// 420 | 436, -3B shapes 524 | 509; 256 tokens, Phi-3.5-mini shapes 446 | 461; 512 tokens, 4 heads of 64 235 | 224; 2 tokens behind 1000, 1B shapes 504 | 503, behind 2000
+// 656 | 561; 512 tokens behind 2000, 3B shapes 1649 | 692.  With a window or blocks a row sees no more keys than that, and its tile those of 128 rows.
+inline bool attn_tensor(int T, long long pos, int window, int chunk) {
+    const long long reach = window > 0 ? window : chunk > 0 ? chunk : pos + T;
+    return std::min(pos + T, reach + 128) >= 512;
+}
+
 // The large tiles with the most keys go out first.  Where the grid is at most two CTAs per SM the second half goes out in the opposite order, so
 // that an SM with a long tile gets a short one beside it -- if two CTAs of `smem` bytes fit an SM (228 KB, 1 KB of it reserved per CTA).  Where
 // only one fits (heads wider than 128 with values wider than 64) the second half is a second wave and starts with its longest tiles too.

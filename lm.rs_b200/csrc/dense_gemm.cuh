@@ -480,6 +480,21 @@ struct DenseGemmCtx {
     int form = GEMM_BY_SIZE;   // option: this form for every product of more than 128 rows that it can serve
     ~DenseGemmCtx() { if (h_err) cudaFreeHost(h_err); }
 };
+// the tensor-map encoder and the mapped status word, once; c.enc stays null without them
+inline void tg_init(DenseGemmCtx& c) {
+    if (c.tried) return;
+    c.tried = true;
+    void* fp = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fp, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
+        c.enc = (TgEncodeTiledFn)fp;
+    if (c.enc && cudaHostAlloc(&c.h_err, sizeof(int), cudaHostAllocMapped) == cudaSuccess) {
+        *c.h_err = 0;
+        if (cudaHostGetDevicePointer(&c.d_err, c.h_err, 0) != cudaSuccess) c.enc = nullptr;
+    } else {
+        c.enc = nullptr;
+    }
+}
 // a [rows][row_bytes used of pitch_bytes] byte matrix, box 128 bytes x box_rows rows, 128B swizzle, zeros outside; every kernel here asks L2 for
 // 256 bytes at a time (1 - 4 % faster than 128)
 inline bool tg_make_map(DenseGemmCtx& c, CUtensorMap* map, const void* base, size_t row_bytes, size_t pitch_bytes, size_t rows, int box_rows) {
@@ -521,19 +536,7 @@ inline int dense_gemm_launch(DenseGemmCtx& c, cudaStream_t st, int T, const AT* 
     if constexpr (!std::is_same<AT, __nv_bfloat16>::value || !std::is_same<WT, __nv_bfloat16>::value) {
         return -1;
     } else {
-        if (!c.tried) {
-            c.tried = true;
-            void* fp = nullptr;
-            cudaDriverEntryPointQueryResult q;
-            if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fp, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
-                c.enc = (TgEncodeTiledFn)fp;
-            if (c.enc && cudaHostAlloc(&c.h_err, sizeof(int), cudaHostAllocMapped) == cudaSuccess) {
-                *c.h_err = 0;
-                if (cudaHostGetDevicePointer(&c.d_err, c.h_err, 0) != cudaSuccess) c.enc = nullptr;
-            } else {
-                c.enc = nullptr;
-            }
-        }
+        tg_init(c);
         if (!c.enc) return -1;
         if ((reinterpret_cast<uintptr_t>(a) & 15) || (reinterpret_cast<uintptr_t>(w) & 15) || (w2 && (reinterpret_cast<uintptr_t>(w2) & 15))) return -1;
         if (*c.h_err) { err = "a tensor-core matrix product gave up waiting on one of its barriers (device status flag set)"; return 1; }

@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "arch.h"
+#include "attn_tensor.cuh"
 #include "attn_tiles.cuh"
 #include "dense_dispatch.h"
 #include "dense_gemm.cuh"
@@ -76,7 +77,9 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
     // programmatic dependent launch of the decode chain is an option.  An architecture turns it on where it measures faster (Genetar);
     // chains of many small kernels lose a little (Tudatar, 16 steps of 3 layers: 2.96 -> 3.03 ms)
     int use_graph = 1, use_pdl = 0;
-    int attn_tiles = -1;   // option: 1 / 0 the register-tiled attention wherever it can run / nowhere, -1 by attn_large_tiles
+    int attn_tiles = -1;   // option: 2 / 1 the tensor-core / the register-tiled attention wherever it can run, 0 neither, -1 by attn_tensor and attn_large_tiles
+    uint16_t* split_planes = nullptr;   // pieces of the running call's f32 operands (attn_tensor.cuh)
+    size_t split_cap = 0;               // its elements
 
     // what an architecture implements
     virtual size_t n_layers() const = 0;
@@ -396,6 +399,50 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
         if (p.dv <= 64) return pitch == 64 ? go(attn_tile_kernel<AT, 1, 64, 2, SIG, false>, 256) : pitch == 128 ? go(attn_tile_kernel<AT, 1, 128, 2, SIG, false>, 256) : go(attn_tile_kernel<AT, 1, 0, 2, SIG, false>, 256);
         return pitch == 128 ? go(attn_tile_kernel<AT, 2, 128, 1, SIG, false>, 128) : pitch == 96 ? go(attn_tile_kernel<AT, 2, 96, 1, SIG, false>, 128) : go(attn_tile_kernel<AT, 2, 0, 1, SIG, false>, 128);
     }
+    // Room for n elements of split operands.  Every user fills and reads them on the model's stream.  Grows by half at least, so that a
+    // prompt in many portions allocates a few times; false: no memory (the caller takes a kernel that needs none).
+    bool split_room(size_t n) {
+        if (n <= split_cap) return true;
+        const size_t more = std::max(n, split_cap + split_cap / 2);
+        dfree(split_planes);
+        split_planes = nullptr; split_cap = 0;
+        void* v = nullptr;
+        for (const size_t want : {more, n})
+            if (!v && cudaMalloc(&v, want * 2) == cudaSuccess) split_cap = want;
+        (void)cudaGetLastError();
+        if (!v) return false;
+        owned.push_back(v);
+        split_planes = static_cast<uint16_t*>(v);
+        return true;
+    }
+    // Tensor-core attention of T > 1 rows: 0 launched, 1 failed, -1 not possible here (the caller takes another kernel)
+    int launch_attn_tensor(cudaStream_t st, AttnRowsParams<AT> p) {
+        dense::tg_init(gemm_ctx);
+        if (!gemm_ctx.enc) return -1;
+        if (*gemm_ctx.h_err) { error = "a tensor-core kernel gave up waiting on one of its barriers (device status flag set)"; return 1; }
+        const int kv_mul = p.H / p.G, chunks = (kv_mul + p.HC - 1) / p.HC, pos0 = (int)p.ps.pos, dkp = attn_tensor_pad(p.dk), dvp = attn_tensor_pad(p.dv);
+        p.TQ = std::max(1, AX_ROWS / p.HC);
+        p.async = p.dk % 4 == 0 && p.dv % 4 == 0 && p.k_ld % 4 == 0 && p.v_ld % 4 == 0;
+        AttnSplitParams s{};
+        s.k = p.kcache; s.v = p.vcache; s.k_ld = p.k_ld; s.v_ld = p.v_ld; s.G = p.G; s.dk = p.dk; s.dv = p.dv; s.vec = p.async;
+        s.n_keys = pos0 + p.T;
+        const int tiles = (s.n_keys + AX_KEYS - 1) / AX_KEYS;
+        s.n_pad = tiles * AX_KEYS;
+        s.first = p.window > 0 ? std::max(0, pos0 - p.window + 1) / AX_KEYS : p.chunk > 0 ? pos0 / p.chunk * p.chunk / AX_KEYS : 0;
+        s.kf = p.window > 0 && p.keep_first > 0 ? std::min(s.first, (p.keep_first + AX_KEYS - 1) / AX_KEYS) : 0;
+        const size_t k_n = (size_t)3 * p.G * s.n_pad * dkp, n = k_n + (size_t)3 * p.G * s.n_pad * dvp;
+        if (!split_room(n)) return -1;
+        s.kp = split_planes; s.vp = split_planes + k_n;
+        CUtensorMap mk, mv;
+        if (!tg_make_map(gemm_ctx, &mk, s.kp, (size_t)dkp * 2, (size_t)dkp * 2, (size_t)3 * p.G * s.n_pad, AX_KEYS) ||
+            !tg_make_map(gemm_ctx, &mv, s.vp, (size_t)s.n_pad * 2, (size_t)s.n_pad * 2, (size_t)3 * p.G * dvp, dvp))
+            return -1;
+        if (launch_k("attn_split_kernel", st, false, attn_split_kernel, dim3(2 * (s.kf + tiles - s.first), p.G, 1 + (dvp + 63) / 64), dim3(256), 0, s)) return 1;
+        const size_t smem = attn_tensor_smem(p.dk);
+        const dim3 grid(p.G * chunks, (p.T + p.TQ - 1) / p.TQ);
+        auto go = [&](auto kernel) { return optin(kernel, smem) || launch_k("attn_tensor_kernel", st, false, kernel, grid, dim3(AX_THREADS), smem, mk, mv, p, s.n_pad, gemm_ctx.d_err); };
+        return p.dv <= 64 ? go(attn_tensor_kernel<AT, 1>) : go(attn_tensor_kernel<AT, 2>);
+    }
     // attention over T query rows: the caller fills the tensors, head geometry, pitches, scale, soft-cap, window, kept first keys,
     // sink, gates and penalty;
     // the tiling, the key split of a one-row step and the merge of the splits are chosen here.  `part` is the split scratch
@@ -414,7 +461,13 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
         // a one-row step over few KV heads: fewer query heads per CTA, so that more SMs share the keys
         while (T == 1 && p.HC > 4 && p.G * ((kv_mul + p.HC - 1) / p.HC) * tiles < sms) p.HC /= 2;
         const int chunks = (kv_mul + p.HC - 1) / p.HC;
-        // Prompts and long portions: the register-tiled kernel (the values in one or two 64-column blocks), where there are tiles enough
+        // Prompts and long portions on the tensor cores: softmax weights, heads of at most 128, positions known here
+        if (!SIG && T > 1 && use_tc && p.dk <= 128 && p.dv <= 128 && !p.v_in_k && !p.ps.sp && !(p.window > 0 && p.chunk > 0) &&
+            (attn_tiles < 0 ? attn_tensor(T, p.ps.pos, p.window, p.chunk) : attn_tiles == 2) && (T + AX_ROWS / p.HC - 1) / (AX_ROWS / p.HC) <= 65535) {
+            const int rc = launch_attn_tensor(st, p);
+            if (rc >= 0) return rc;
+        }
+        // the register-tiled kernel (the values in one or two 64-column blocks), where there are tiles enough
         const bool large = attn_tiles < 0 ? (long long)T * p.HC >= TA_ROWS && attn_large_tiles(sms, T, p.G * chunks, p.HC) : attn_tiles > 0;
         if (T > 1 && large && p.dv <= 128 && attn_tile_smem(p.dk, p.dv, p.v_in_k) <= 227 * 1024) {
             p.TQ = std::max(1, TA_ROWS / p.HC);

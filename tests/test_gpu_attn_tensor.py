@@ -1,0 +1,77 @@
+"""The tensor-core prompt attention (csrc/attn_tensor.cuh) where its tiles end: query rows and keys around whole tiles of 128 (and of the
+16, 32 and 64 keys its steps take), head sizes that fill one or two operand boxes or only part of one, grouped heads that do not divide a
+tile, prompts cut in portions.  One-layer Genetar models in float32 against the float64 implementation, held to that mode's 2e-4 of the
+logits' root mean square (test_gpu_genetar.py); windows, chunks, penalties, sinks and gates through the mixed models of the other test
+files, held to theirs.  These calls are too small to take the kernel by themselves: option "attn_tiles" 2."""
+import importlib
+
+import numpy as np
+import pytest
+
+import genetar_oracle as G
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,n", [
+    (4, 1, 64, 64, 32),     # exactly one tile of rows
+    (4, 1, 64, 64, 33),     # one row more
+    (1, 1, 64, 64, 257),    # key tiles: two whole ones and one key
+    (3, 1, 128, 128, 65),   # 42 tokens x 3 heads in a tile of 128 rows; one key beyond a box of values
+    (2, 2, 128, 64, 130),   # latent attention's shape
+    (2, 2, 96, 96, 129),    # a box and a half
+    (2, 1, 72, 72, 70),     # ends inside a step of 16
+    (2, 1, 112, 20, 400),   # both groups of warps with several tiles
+    (2, 1, 20, 4, 90),      # one piece of values
+    (2, 1, 10, 6, 80),      # sizes that are not whole 16-byte pieces
+    (20, 1, 32, 32, 9),     # more grouped heads than a tile takes at once
+    (2, 2, 16, 128, 2),     # the fewest rows
+])
+def test_tile_edges(gpu_lib, tmp_path, heads, kv_heads, dim, vdim, n):
+    cfg = G.make_config([G.attention_layer("attention_2", heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, ff=0, v_mix=False, scale=0.3, rot_dims=4)])
+    W = G.random_weights(cfg, seed=dim + n, qk_gain=2.0)
+    toks = np.random.default_rng(n).integers(0, cfg["vocab"], n).tolist()
+    want, _ = G.forward(cfg, W, toks)
+    m = gpu_lib.Transformer.open(G.write_model(str(tmp_path / "m"), cfg, W), dtype="float32", max_tokens=400)
+    m.set_option("attn_tiles", 2)
+    whole = m.forward_tokens(toks, 0, list(range(n)))
+    assert G.rel_rms(whole, want) < 2e-4
+    cut = max(1, n // 2 - 3)   # a portion that starts inside a tile
+    parts = np.concatenate([m.forward_tokens(toks[:cut], 0, list(range(cut))), m.forward_tokens(toks[cut:], cut, list(range(n - cut)))])
+    assert G.rel_rms(parts, want) < 2e-4
+    m.close()
+
+
+@pytest.mark.parametrize("arch", ["tudatar", "rupenex", "badepel", "bolapel", "lutesun"])
+def test_forms_of_the_other_models(gpu_lib, tmp_path, arch):
+    """windows with and without kept keys, blocks, penalties, sinks, gates, expanded latent heads: a prompt over two key tiles whole,
+    and in portions that start inside a tile"""
+    T = importlib.import_module(f"test_gpu_{arch}")
+    n = 150
+    cfg = T.mixed_cfg()
+    toks = T.tokens_for(cfg, n)
+    W = T.weights_for(cfg, toks, seed=1) if hasattr(T, "weights_for") else T.O.random_weights(cfg, seed=1)
+    want, _ = T.O.forward(cfg, W, toks)
+    m = T.open_model(gpu_lib, tmp_path, cfg, W, "float32")
+    m.set_option("attn_tiles", 2)
+    assert T.O.rel_rms(m.forward_tokens(toks, 0, list(range(n))), want) < T.TOL["float32"]
+    cuts = [0, 67, 74, 140, n]
+    parts = [m.forward_tokens(toks[a:b], a, list(range(b - a))) for a, b in zip(cuts, cuts[1:])]
+    assert T.O.rel_rms(np.concatenate(parts), want) < T.TOL["float32"]
+    m.close()
+
+
+def test_scores_as_low_as_the_other_kernels_take_them(gpu_lib, tmp_path):
+    """a row whose only visible keys score between -1e30 and -1e30 / log2(e): still an average of their values"""
+    cfg = G.make_config([G.attention_layer("attention", heads=4, kv_heads=4, dim=16, vdim=16, ff=0, v_mix=False, scale=-5e28, softcap=None)], bigram=None)
+    W = G.random_weights(cfg, seed=3)
+    W["l0.mix.k"] = W["l0.mix.q"]   # q . k of a token with itself is 16: its score is -8e29
+    toks = np.random.default_rng(3).integers(0, cfg["vocab"], 40).tolist()
+    m = gpu_lib.Transformer.open(G.write_model(str(tmp_path / "m"), cfg, W), dtype="float32", max_tokens=64)
+    m.set_option("attn_tiles", 0)
+    want = m.forward_tokens(toks, 0, list(range(40)))
+    m.set_option("attn_tiles", 2)
+    got = m.forward_tokens(toks, 0, list(range(40)))
+    assert np.isfinite(want[0]).all() and np.isfinite(got).all()
+    assert G.rel_rms(got[0], want[0]) < 2e-4
+    m.close()
