@@ -2,11 +2,6 @@
 // f32 width: every f32 operand is split into three bf16 pieces whose sum is exact (8 + 8 + 8 significant bits), and a product is
 // the six piece products down to 2^-16 of it (what is left out is below 2^-23), each exact in the tensor cores' f32 accumulators.
 // Same parameters and arithmetic rules as attn_tile_kernel and attn_rows_kernel (dense_ops.cuh).
-// Errors against 64 bits (normal operands, f32 output; 2-norm): 2.4e-7 without a soft-cap for 2048 tokens of 128-wide heads (attn_tile_kernel 4.3e-7),
-// 7.5e-7 with one (8.1e-7; the cap's exponential is what is left).
-// What bounds it: one key tile after the other.  A tile of 128 rows x 128 keys of 128-wide heads is 96 MMAs, 6144 cycles of the tensor core, and
-// about 7500 cycles of one group's softmax (three special-function results a weight with a soft-cap), of which the other group's products hide most: 9300 cycles a tile.
-// 2048 tokens, 24 heads of 128 on 8 KV heads: 186 us and 11 for the split (attn_tile_kernel 785); 512 tokens, 32 heads of 64: 33 and 7 (62); 1000 such tokens: 57 and 8 (168).
 #pragma once
 #include "attn_tiles.cuh"
 #include "dense_gemm.cuh"
@@ -50,44 +45,6 @@ DN_DEVINL void load8(const float* row, int c, int n, bool vec, float (&v)[8]) {
 }
 
 // ---- tensor-core helpers --------------------------------------------------------------------------------------------------------------
-// MMAs of a converged warp, issued by its elected lane (`one`): operands computed by the whole warp stay in uniform registers, and the
-// upper descriptor word is a constant.  What matters is that the issue of an MMA (and the waits and commits between them) takes less than
-// the MMA itself (32 to 64 cycles here): 64-bit descriptor arithmetic in a branch of one lane took 140 - 170.
-constexpr uint32_t TG_DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);   // upper word of tg_desc_sw128
-DN_DEVINL uint32_t elect_one() {
-    uint32_t r;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(r));
-    return r;
-}
-DN_DEVINL void tg_mma_ss1(uint32_t one, uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "setp.ne.b32 q, %5, 0;\n\t"
-        "mov.b64 a, {%1, %6};\n\t"
-        "mov.b64 b, {%2, %6};\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t}"
-        ::"r"(tmem_d), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(one), "r"(TG_DESC_HI)
-        : "memory");
-}
-DN_DEVINL void tg_mma_ts1(uint32_t one, uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {   // A from TMEM
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t.reg .b64 b;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "setp.ne.b32 q, %5, 0;\n\t"
-        "mov.b64 b, {%2, %6};\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, p;\n\t}"
-        ::"r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(one), "r"(TG_DESC_HI)
-        : "memory");
-}
-DN_DEVINL void tg_commit1(uint32_t one, uint64_t* bar) {
-    asm volatile(
-        "{\n\t.reg .pred q;\n\t"
-        "setp.ne.b32 q, %1, 0;\n\t"
-        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
-        ::"r"(smem_u32(bar)), "r"(one)
-        : "memory");
-}
 // waits for the loads before it; the values pass through, so that nothing computed from them can move ahead of the wait
 DN_DEVINL void tmem_ld_wait(uint32_t (&v)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;"

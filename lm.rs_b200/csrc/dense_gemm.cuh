@@ -74,16 +74,55 @@ DN_DEVINL uint64_t tg_desc_sw128(const void* smem_tile) {
 template <int BN> __host__ __device__ constexpr uint32_t tg_idesc() {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TG_M >> 4) << 24);
 }
-DN_DEVINL void tg_mma(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+// MMAs of a converged warp, issued by its elected lane (`one`): operands computed by the whole warp stay in uniform registers, and the
+// upper descriptor word is a constant.  What matters is that the issue of an MMA (and the waits and commits between them) takes less than
+// the MMA itself (32 to 64 cycles here): 64-bit descriptor arithmetic in a branch of one lane took 140 - 170.
+constexpr uint32_t TG_DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);   // upper word of tg_desc_sw128
+DN_DEVINL uint32_t elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r;
+}
+DN_DEVINL void tg_mma_ss1(uint32_t one, uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "mov.b64 a, {%1, %6};\n\t"
+        "mov.b64 b, {%2, %6};\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(one), "r"(TG_DESC_HI)
         : "memory");
 }
-DN_DEVINL void tg_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+DN_DEVINL void tg_mma_ts1(uint32_t one, uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {   // A from TMEM
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .b64 b;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "mov.b64 b, {%2, %6};\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(one), "r"(TG_DESC_HI)
+        : "memory");
+}
+DN_DEVINL void tg_commit1(uint32_t one, uint64_t* bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
+        ::"r"(smem_u32(bar)), "r"(one)
+        : "memory");
+}
+// has the barrier's phase ended? (no waiting)
+DN_DEVINL bool mbar_test(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
 }
 DN_DEVINL void tg_tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
     asm volatile(
@@ -161,7 +200,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tfull + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     int m0 = blockIdx.y * TG_M, row_end = p.T, wrow0 = 0;
     const int n0 = blockIdx.x * OUT_COLS;
     if (p.grp) {   // tiles past the group's last row leave before anything is set up (the whole CTA takes this branch)
@@ -210,23 +249,27 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {   // ---- MMA issuer ----
-            const uint32_t idesc = tg_idesc<BN>();
-            bool ok = true;
-            for (int g = 0; g < KS && ok; g++) {
-                const int s = g % TG_STAGES;
-                ok = mbar_wait_bounded(&full[s], (g / TG_STAGES) & 1, abort_flag);
-                if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint8_t* a_t = tiles + (size_t)s * TG_STAGE_BYTES;
-                const uint64_t da = tg_desc_sw128(a_t), db = tg_desc_sw128(a_t + TG_A_BYTES);
-#pragma unroll
-                for (int k = 0; k < TG_KB / 32; k++)   // 16 bf16 = 32 bytes along K inside the swizzle atom
-                    tg_mma(tmem_base, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (g > 0 || k > 0) ? 1u : 0u);
-                tg_commit(&empty[s]);
-            }
-            if (ok) tg_commit(tfull);
+        // ---- MMA issuer: the next stage is looked at while half of this one's MMAs are still to come, so that the tensor core has work queued
+        // meanwhile.  (One lane that waited for a stage, built its descriptors and issued its four MMAs in turn: 46.1 us instead of 41.9 for 512 x 2048
+        // added to the residual, K 8192; the two-SM forms below 29.7 and 26.2, 2048 x 5120, K 3072 67.9 and 66.8) ----
+        const uint32_t one = elect_one(), idesc = tg_idesc<BN>(), t_lo = (uint32_t)tg_desc_sw128(tiles);
+        bool ok = true, landed = false;
+        for (int g = 0, s = 0, round = 0; g < KS; g++) {
+            ok = landed || mbar_wait_bounded(&full[s], round & 1, abort_flag);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t da = t_lo + s * (TG_STAGE_BYTES >> 4), db = da + (TG_A_BYTES >> 4);   // 16 bf16 = 32 bytes along K inside the swizzle atom
+            const int s2 = s + 1 == TG_STAGES ? 0 : s + 1, r2 = round + (s2 == 0);
+            tg_mma_ss1(one, tmem_base, da, db, idesc, g > 0 ? 1u : 0u);
+            tg_mma_ss1(one, tmem_base, da + 2, db + 2, idesc, 1u);
+            landed = g + 1 < KS && mbar_test(&full[s2], r2 & 1);
+            tg_mma_ss1(one, tmem_base, da + 4, db + 4, idesc, 1u);
+            tg_mma_ss1(one, tmem_base, da + 6, db + 6, idesc, 1u);
+            tg_commit1(one, &empty[s]);
+            s = s2; round = r2;
         }
+        if (ok) tg_commit1(one, tfull);
+        __syncwarp();
     } else {   // ---- epilogue: TMEM lane quadrant = warp % 4 ----
         // tcgen05.ld hands a thread one ROW of the tile (32 consecutive columns per load).  Writing rows from there would
         // touch 32 different cache lines per instruction, so each 32 x 32 block goes through shared memory (the operand
@@ -296,16 +339,24 @@ DN_DEVINL void tg_tma_load_2d_pair(void* dst, const CUtensorMap* map, int x, int
                  "l"(map), "r"(x), "r"(y), "r"(bar)
                  : "memory");
 }
-DN_DEVINL void tg_mma_pair(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+DN_DEVINL void tg_mma_pair1(uint32_t one, uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "mov.b64 a, {%1, %6};\n\t"
+        "mov.b64 b, {%2, %6};\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(one), "r"(TG_DESC_HI)
         : "memory");
 }
-DN_DEVINL void tg_commit_pair(uint64_t* bar, uint16_t mask) {   // arrives on this barrier in every CTA of the mask
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "h"(mask) : "memory");
+DN_DEVINL void tg_commit_pair1(uint32_t one, uint64_t* bar, uint16_t mask) {   // arrives on this barrier in every CTA of the mask
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %2, 0;\n\t"
+        "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+        ::"r"(smem_u32(bar)), "h"(mask), "r"(one)
+        : "memory");
 }
 template <int BN> __host__ __device__ constexpr uint32_t tg_idesc_pair() {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
@@ -328,7 +379,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_con
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tfull + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank(), side = rank & 1, split = rank >> 1;
     const int m0 = blockIdx.y * 256 + (int)side * 128, n0 = (int)(blockIdx.x / (2 * SPLIT)) * OUT_COLS;
     const int KS = (p.K * 2 + TG_KB - 1) / TG_KB;
@@ -370,22 +421,26 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_con
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && side == 0) {   // ---- MMA issuer of the pair ----
+        if (side == 0) {   // ---- MMA issuer of the pair: as above ----
             constexpr uint32_t idesc = tg_idesc_pair<BN>();
+            const uint32_t one = elect_one(), t_lo = (uint32_t)tg_desc_sw128(tiles);
             const uint16_t mask = (uint16_t)(3u << (rank & ~1u));
-            bool ok = true;
+            bool ok = true, landed = false;
             for (int i = 0, s = 0, round = 0; i < g1 - g0; i++) {
-                ok = mbar_wait_bounded(&full[s], round & 1, abort_flag);
+                ok = landed || mbar_wait_bounded(&full[s], round & 1, abort_flag);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint8_t* a_t = tiles + (size_t)s * STAGE;
-                const uint64_t da = tg_desc_sw128(a_t), db = tg_desc_sw128(a_t + TG_A_BYTES);
-#pragma unroll
-                for (int k = 0; k < TG_KB / 32; k++) tg_mma_pair(tmem_base, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (i > 0 || k > 0) ? 1u : 0u);
-                tg_commit_pair(&empty[s], mask);
-                if (++s == p.stages) { s = 0; round++; }
+                const uint32_t da = t_lo + s * (STAGE >> 4), db = da + (TG_A_BYTES >> 4);
+                const int s2 = s + 1 == p.stages ? 0 : s + 1, r2 = round + (s2 == 0);
+                tg_mma_pair1(one, tmem_base, da, db, idesc, i > 0 ? 1u : 0u);
+                tg_mma_pair1(one, tmem_base, da + 2, db + 2, idesc, 1u);
+                landed = i + 1 < g1 - g0 && mbar_test(&full[s2], r2 & 1);
+                tg_mma_pair1(one, tmem_base, da + 4, db + 4, idesc, 1u);
+                tg_mma_pair1(one, tmem_base, da + 6, db + 6, idesc, 1u);
+                tg_commit_pair1(one, &empty[s], mask);
+                s = s2; round = r2;
             }
-            if (ok) tg_commit_pair(tfull, mask);
+            if (ok) tg_commit_pair1(one, tfull, mask);
         }
     }
     __syncwarp();
