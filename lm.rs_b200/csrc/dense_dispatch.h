@@ -78,5 +78,32 @@ inline int gemm_form(bool glu, int T, int K, int O, int sms, int pairs, int quad
     return best;
 }
 
+// The float32 product of many rows, rows on 16-byte boundaries: tensor cores (dense_gemm_split.cuh) or CUDA cores (dense_gemm_f32.cuh)?  The
+// former has a second launch and fills and drains more; from 512 of K on, or where the latter's tiles do not all run at once, it wins.  CUDA cores | tensor cores, us:
+// 129 x 512 gate/up, K 256: 13 | 17; 16 x 128, K 64: 7 | 12; 5 x 96, K 260: 15 | 14; 400 x 256 added to the residual, K 512: 27 | 19; 2 x 4096, K 2048: 71 | 20.
+inline bool gemm_split_pays(bool glu, int T, int K, int O, int sms) {
+    return K >= 512 || (long long)((O + (glu ? 31 : 63)) / (glu ? 32 : 64)) * ((T + 63) / 64) > 2LL * sms;
+}
+// The tensor-core form's tiles: rows of A per CTA (N, a multiple of 16, at most 128) and CTAs that share a tile's K.  Estimated like the forms of
+// gemm_form, constants (cycles) fitted to 21 products at 16 tilings each: a 32-wide piece of K takes 800 + 4 N, a CTA 14000 besides and 7000 more when it meets others.
+// us of the choice and of the next best tilings: 301 x 8192 gate/up, K 2048: 112 rows 150, 80 rows 171, 64 rows 197; 301 x 2048, K 8192: 80 rows and K in two 93,
+// 112 and two 106, 112 and four 113; 16 x 4096, K 2048: 16 and four 20, 32 and two 27, 16 37; 200 x 3072, K 3072: 80 and two 41, 112 and two 46, 48 58.
+struct GemmSplitPlan { int N, splits; };
+inline GemmSplitPlan gemm_split_plan(bool glu, int T, int K, int O, int sms) {
+    const long long m_tiles = glu ? (O + 63) / 64 : (O + 127) / 128;
+    const int pieces = (K + 31) / 32, least = (T + 127) / 128;
+    GemmSplitPlan best{};
+    double time = 1e30;
+    for (int n_tiles = least; n_tiles <= least + 8; n_tiles++) {
+        const int N = ((T + n_tiles - 1) / n_tiles + 15) / 16 * 16;
+        for (int splits = 1; splits <= 4 && (splits == 1 || K >= 256 * splits); splits *= 2) {   // each part has 128 of K at least
+            const long long ctas = m_tiles * ((T + N - 1) / N) * splits, rounds = (ctas + sms - 1) / sms;
+            const double t = (double)rounds * ((double)((pieces + splits - 1) / splits) * (800 + 4 * N) + 14000 + (splits > 1 ? 7000 : 0));
+            if (t < time) { time = t; best = {N, splits}; }
+        }
+    }
+    return best;
+}
+
 }  // namespace dense
 }  // namespace lmrs

@@ -530,7 +530,7 @@ struct DenseGemmCtx {
     int* h_err = nullptr;   // mapped, pinned
     int* d_err = nullptr;
     std::map<std::pair<const void*, int>, CUtensorMap> wmaps;   // (weight matrix, box rows) -> tensor map
-    bool attr_set[4][2] = {}, pair_attr_set[4][3] = {};
+    bool attr_set[4][2] = {}, pair_attr_set[4][3] = {}, split_attr_set[4] = {};
     int at_once[2] = {};   // clusters of two and of four CTAs that run at the same time with one CTA per SM (0: not asked yet)
     int form = GEMM_BY_SIZE;   // option: this form for every product of more than 128 rows that it can serve
     ~DenseGemmCtx() { if (h_err) cudaFreeHost(h_err); }

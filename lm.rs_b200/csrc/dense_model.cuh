@@ -23,6 +23,7 @@
 #include "dense_dispatch.h"
 #include "dense_gemm.cuh"
 #include "dense_gemm_f32.cuh"
+#include "dense_gemm_split.cuh"
 #include "dense_ops.cuh"
 #include "safetensors.h"
 
@@ -78,6 +79,7 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
     // chains of many small kernels lose a little (Tudatar, 16 steps of 3 layers: 2.96 -> 3.03 ms)
     int use_graph = 1, use_pdl = 0;
     int attn_tiles = -1;   // option: 2 / 1 the tensor-core / the register-tiled attention wherever it can run, 0 neither, -1 by attn_tensor and attn_large_tiles
+    int gemm_split = -1;   // option: 1 / 0 float32 products on the tensor cores wherever they can run / nowhere, -1 by gemm_split_pays
     uint16_t* split_planes = nullptr;   // pieces of the running call's f32 operands (attn_tensor.cuh)
     size_t split_cap = 0;               // its elements
 
@@ -316,6 +318,12 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
         }
         GemmTiledParams<AT, WT> p{};
         p.a = a; p.lda = lda; p.w = w; p.w2 = w2; p.T = T; p.K = K; p.O = O; p.e = e;
+        if constexpr (std::is_same<AT, float>::value && std::is_same<WT, float>::value) {
+            if (use_tc && gemm_f32_usable(p) && (gemm_split == 1 || (gemm_split < 0 && gemm_split_pays(EPI == EPI_GLU, T, K, O, sms))) && split_room((size_t)3 * T * gemm_split_kp(K))) {
+                const int rc = gemm_split_launch<EPI>(gemm_ctx, st, p, gemm_split_plan(EPI == EPI_GLU, T, K, O, sms), split_planes, error);
+                if (rc >= 0) { launches += 2; return rc; }
+            }
+        }
         return launch_gemm_cores<EPI>(st, p, T, 1);
     }
     // nb products at once, one matrix per batch entry z (a head): out[:, z*o_bs ..] = a[:, z*a_bs ..] . (w + z*w_bs)^T.  The
@@ -626,6 +634,7 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
         else if (!strcmp(name, "graphs")) { use_graph = value; if (!value) drop_graphs(); }
         else if (!strcmp(name, "attn_tiles")) attn_tiles = value;
         else if (!strcmp(name, "gemm_form")) gemm_ctx.form = std::max(-2, std::min(2, value));
+        else if (!strcmp(name, "gemm_split")) gemm_split = value;
         else if (!strcmp(name, "pdl")) { use_pdl = value; drop_graphs(); }
         else set_model_option(name, value);
     }
