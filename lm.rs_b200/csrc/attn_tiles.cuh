@@ -32,11 +32,6 @@ inline size_t attn_tile_smem(int dk, int dv, bool v_in_k) {
     const size_t qs = attn_tile_pitch(dk), vs = v_in_k ? 0 : (dv <= 64 ? 64 : 128);
     return ((size_t)TA_ROWS * qs + (size_t)TA_KEYS * (qs + vs) + (size_t)TA_ROWS * TA_KEYS) * 4;
 }
-typedef unsigned long long f32pair;
-DN_DEVINL void fma2(f32pair& acc, f32pair a, f32pair b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
-DN_DEVINL f32pair mul2(f32pair a, f32pair b) { f32pair r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-DN_DEVINL f32pair dup2(float v) { f32pair r; asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v)); return r; }
-DN_DEVINL float2 unpack2(f32pair v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
 DN_DEVINL float ex2(float v) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v)); return r; }
 DN_DEVINL float lg2(float v) { float r; asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v)); return r; }
 

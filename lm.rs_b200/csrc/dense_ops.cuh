@@ -45,6 +45,14 @@ DN_DEVINL float to_f(__nv_bfloat16 v) { return __bfloat162float(v); }
 DN_DEVINL void from_f(float& d, float v) { d = v; }
 DN_DEVINL void from_f(__nv_bfloat16& d, float v) { d = __float2bfloat16_rn(v); }
 
+// two f32 in one register pair: one instruction for both, each rounded as the scalar form rounds it
+typedef unsigned long long f32pair;
+DN_DEVINL void fma2(f32pair& acc, f32pair a, f32pair b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
+DN_DEVINL f32pair mul2(f32pair a, f32pair b) { f32pair r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+DN_DEVINL f32pair dup2(float v) { f32pair r; asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v)); return r; }
+DN_DEVINL f32pair pack2(float a, float b) { f32pair r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+DN_DEVINL float2 unpack2(f32pair v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
+
 DN_DEVINL float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

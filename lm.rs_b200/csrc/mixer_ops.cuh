@@ -384,8 +384,9 @@ static __global__ void __launch_bounds__(256) delta_decay_kernel(const DeltaDeca
 // lane reads its q, k and decay entries of a token with 16-byte shared-memory loads that do not collide with its neighbours'.
 // Columns never interact: S^T k and S^T q are sums down a column, the rank-one update adds k_i u_j.  Tokens are staged
 // DELTA_TB at a time in shared memory by cp.async (q, k, decays, v, beta), the next block in flight while this one is used;
-// rows beyond dk are zero-filled, so the arithmetic needs no bounds.  Every token costs two passes over the registers and two
-// reductions across the lpc lanes.  The order of every sum is fixed, so a token's result does not depend on the portion it
+// rows beyond dk are zero-filled, so the arithmetic needs no bounds.  Every token costs two passes over the registers and one
+// reduction across the lpc lanes, which is what bounds it (the next token needs the state it leads to); the read-outs are reduced eight tokens at
+// a time (block_sums), and two rows go through one instruction: 512 tokens of 16 heads of 128 x 128 161 -> 132 us, to the same bits.  The order of every sum is fixed, so a token's result does not depend on the portion it
 // arrives in.  The state is read at the start (zeros when the step starts at position 0) and written back at the end.
 constexpr int DELTA_TB = 8, DELTA_THREADS = 128, DELTA_MAX_DK = 512;
 struct DeltaScanParams {
@@ -417,6 +418,30 @@ DN_DEVINL void cp_async4_zfill(void* smem_dst, const void* gsrc, bool valid) {
     const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem_dst);
     const int n = valid ? 4 : 0;
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(gsrc), "r"(n) : "memory");
+}
+// Sums over the LPC lanes (a power of two) of a column, lane s of them, for the eight tokens of a block at once: a stage adds the lane across and
+// leaves each with half of the tokens, 7 exchanges and one more per remaining stage instead of 8 per stage.  Every sum adds the same numbers in the
+// same order as a butterfly of its own.  Afterwards v[0 .. n) of a lane are the sums of tokens first .. first + n - 1; `writes`: one lane of those that hold them.
+struct BlockSums { int first, n; bool writes; };
+template <int LPC> DN_DEVINL BlockSums block_sums(float (&v)[DELTA_TB], int s) {
+    BlockSums r{0, DELTA_TB, true};
+#pragma unroll
+    for (int o = LPC >> 1, n = DELTA_TB; o > 0; o >>= 1, n = n > 1 ? n >> 1 : 1) {
+        const bool up = (s & o) != 0;
+        if (n > 1) {
+#pragma unroll
+            for (int i = 0; i < n / 2; i++) {
+                const float keep = up ? v[i + n / 2] : v[i], give = up ? v[i] : v[i + n / 2];
+                v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+            }
+            r.n = n / 2;
+            if (up) r.first += n / 2;
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+            if (up) r.writes = false;
+        }
+    }
+    return r;
 }
 template <int NR, int LPC, int MODE = SCAN_DELTA> __global__ void __launch_bounds__(DELTA_THREADS) delta_scan_kernel(const DeltaScanParams p) {
     extern __shared__ __align__(16) float ds_sm[];
@@ -468,12 +493,13 @@ template <int NR, int LPC, int MODE = SCAN_DELTA> __global__ void __launch_bound
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     stage(0, 0);
-    float S[NR];
+    f32pair S[NR / 2];   // neighbouring rows in pairs
     float* sp = p.state + ((size_t)h * p.dk) * p.dv + j;
 #pragma unroll
-    for (int r = 0; r < NR; r++) {
+    for (int r = 0; r < NR; r += 2) {
         const int i = ((r >> 2) * LPC + s) * 4 + (r & 3);
-        S[r] = (pos0 > 0 && col_ok && i < p.dk) ? sp[(size_t)i * p.dv] : 0.0f;
+        const bool in = pos0 > 0 && col_ok;
+        S[r / 2] = pack2(in && i < p.dk ? sp[(size_t)i * p.dv] : 0.0f, in && i + 1 < p.dk ? sp[(size_t)(i + 1) * p.dv] : 0.0f);
     }
     int buf = 0;
     for (int t0 = 0; t0 < p.T; t0 += DELTA_TB, buf ^= 1) {
@@ -486,59 +512,72 @@ template <int NR, int LPC, int MODE = SCAN_DELTA> __global__ void __launch_bound
         const float* gs = ks + DELTA_TB * dkp;
         const float* vs = gs + DELTA_TB * dkp;
         const float* bs = vs + DELTA_TB * cols;
-        for (int tt = 0; tt < nt; tt++) {
-            float o0 = 0.0f, o1 = 0.0f, o2 = 0.0f, o3 = 0.0f;
+        auto pairs = [&](const float* a, int tt, int r4) { return *reinterpret_cast<const ulonglong2*>(a + tt * dkp + (r4 * LPC + s) * 4); };
+        auto token = [&](int tt) {   // one token; this lane's share of its output
+            f32pair o01 = 0ull, o23 = 0ull;
             if (MODE == SCAN_PLAIN) {
-                const float u = vs[tt * cols + jl];
+                const f32pair u = dup2(vs[tt * cols + jl]);
 #pragma unroll
                 for (int r4 = 0; r4 < NR / 4; r4++) {
-                    const int i = (r4 * LPC + s) * 4;
-                    const float4 g4 = *reinterpret_cast<const float4*>(gs + tt * dkp + i);
-                    const float4 k4 = *reinterpret_cast<const float4*>(ks + tt * dkp + i);
-                    const float4 q4 = *reinterpret_cast<const float4*>(qs + tt * dkp + i);
-                    S[4 * r4] = fmaf(S[4 * r4], g4.x, k4.x * u); S[4 * r4 + 1] = fmaf(S[4 * r4 + 1], g4.y, k4.y * u);
-                    S[4 * r4 + 2] = fmaf(S[4 * r4 + 2], g4.z, k4.z * u); S[4 * r4 + 3] = fmaf(S[4 * r4 + 3], g4.w, k4.w * u);
-                    o0 = fmaf(S[4 * r4], q4.x, o0); o1 = fmaf(S[4 * r4 + 1], q4.y, o1);
-                    o2 = fmaf(S[4 * r4 + 2], q4.z, o2); o3 = fmaf(S[4 * r4 + 3], q4.w, o3);
+                    const ulonglong2 g4 = pairs(gs, tt, r4), k4 = pairs(ks, tt, r4), q4 = pairs(qs, tt, r4);
+                    f32pair a = mul2(k4.x, u), b = mul2(k4.y, u);
+                    fma2(a, S[2 * r4], g4.x); fma2(b, S[2 * r4 + 1], g4.y);
+                    S[2 * r4] = a; S[2 * r4 + 1] = b;
+                    fma2(o01, a, q4.x); fma2(o23, b, q4.y);
                 }
             } else {
-            float kk[NR];
-            float r0 = 0.0f, r1 = 0.0f, r2 = 0.0f, r3 = 0.0f;
-            const float gh = MODE == SCAN_DELTA_HEAD ? gs[tt] : 1.0f;
+                f32pair r01 = 0ull, r23 = 0ull;
+                const f32pair gh = dup2(MODE == SCAN_DELTA_HEAD ? gs[tt] : 1.0f);
+                ulonglong2 kk[NR / 4];
 #pragma unroll
-            for (int r4 = 0; r4 < NR / 4; r4++) {
-                const int i = (r4 * LPC + s) * 4;
-                const float4 g4 = MODE == SCAN_DELTA_HEAD ? make_float4(gh, gh, gh, gh) : *reinterpret_cast<const float4*>(gs + tt * dkp + i);
-                const float4 k4 = *reinterpret_cast<const float4*>(ks + tt * dkp + i);
-                kk[4 * r4] = k4.x; kk[4 * r4 + 1] = k4.y; kk[4 * r4 + 2] = k4.z; kk[4 * r4 + 3] = k4.w;
-                S[4 * r4] *= g4.x; S[4 * r4 + 1] *= g4.y; S[4 * r4 + 2] *= g4.z; S[4 * r4 + 3] *= g4.w;
-                r0 = fmaf(S[4 * r4], k4.x, r0); r1 = fmaf(S[4 * r4 + 1], k4.y, r1);
-                r2 = fmaf(S[4 * r4 + 2], k4.z, r2); r3 = fmaf(S[4 * r4 + 3], k4.w, r3);
-            }
-            float rsum = (r0 + r1) + (r2 + r3);
-            for (int o = LPC >> 1; o > 0; o >>= 1) rsum += __shfl_xor_sync(0xffffffffu, rsum, o);
-            const float u = bs[tt] * (vs[tt * cols + jl] - rsum);
+                for (int r4 = 0; r4 < NR / 4; r4++) {
+                    const ulonglong2 g4 = MODE == SCAN_DELTA_HEAD ? make_ulonglong2(gh, gh) : pairs(gs, tt, r4);
+                    kk[r4] = pairs(ks, tt, r4);
+                    S[2 * r4] = mul2(S[2 * r4], g4.x); S[2 * r4 + 1] = mul2(S[2 * r4 + 1], g4.y);
+                    fma2(r01, S[2 * r4], kk[r4].x); fma2(r23, S[2 * r4 + 1], kk[r4].y);
+                }
+                const float2 ra = unpack2(r01), rb = unpack2(r23);
+                float rsum = (ra.x + ra.y) + (rb.x + rb.y);
 #pragma unroll
-            for (int r4 = 0; r4 < NR / 4; r4++) {
-                const int i = (r4 * LPC + s) * 4;
-                const float4 q4 = *reinterpret_cast<const float4*>(qs + tt * dkp + i);
-                S[4 * r4] = fmaf(kk[4 * r4], u, S[4 * r4]); S[4 * r4 + 1] = fmaf(kk[4 * r4 + 1], u, S[4 * r4 + 1]);
-                S[4 * r4 + 2] = fmaf(kk[4 * r4 + 2], u, S[4 * r4 + 2]); S[4 * r4 + 3] = fmaf(kk[4 * r4 + 3], u, S[4 * r4 + 3]);
-                o0 = fmaf(S[4 * r4], q4.x, o0); o1 = fmaf(S[4 * r4 + 1], q4.y, o1);
-                o2 = fmaf(S[4 * r4 + 2], q4.z, o2); o3 = fmaf(S[4 * r4 + 3], q4.w, o3);
+                for (int o = LPC >> 1; o > 0; o >>= 1) rsum += __shfl_xor_sync(0xffffffffu, rsum, o);
+                const f32pair u = dup2(bs[tt] * (vs[tt * cols + jl] - rsum));
+#pragma unroll
+                for (int r4 = 0; r4 < NR / 4; r4++) {
+                    const ulonglong2 q4 = pairs(qs, tt, r4);
+                    fma2(S[2 * r4], kk[r4].x, u); fma2(S[2 * r4 + 1], kk[r4].y, u);
+                    fma2(o01, S[2 * r4], q4.x); fma2(o23, S[2 * r4 + 1], q4.y);
+                }
             }
+            const float2 oa = unpack2(o01), ob = unpack2(o23);
+            return (oa.x + oa.y) + (ob.x + ob.y);
+        };
+        float* dst = p.out + (size_t)t0 * p.H * p.dv + (size_t)h * p.dv + j;
+        if (nt == DELTA_TB) {
+            float ov[DELTA_TB];
+#pragma unroll
+            for (int tt = 0; tt < DELTA_TB; tt++) ov[tt] = token(tt);
+            const BlockSums b = block_sums<LPC>(ov, s);
+            if (b.writes && col_ok)
+#pragma unroll
+                for (int i = 0; i < DELTA_TB; i++)
+                    if (i < b.n) dst[(size_t)(b.first + i) * p.H * p.dv] = p.q_scale != 0.0f ? ov[i] * p.q_scale : ov[i];
+        } else {
+#pragma unroll 1
+            for (int tt = 0; tt < nt; tt++) {
+                float osum = token(tt);
+#pragma unroll
+                for (int o = LPC >> 1; o > 0; o >>= 1) osum += __shfl_xor_sync(0xffffffffu, osum, o);
+                if (s == 0 && col_ok) dst[(size_t)tt * p.H * p.dv] = p.q_scale != 0.0f ? osum * p.q_scale : osum;
             }
-            float osum = (o0 + o1) + (o2 + o3);
-            for (int o = LPC >> 1; o > 0; o >>= 1) osum += __shfl_xor_sync(0xffffffffu, osum, o);
-            if (p.q_scale != 0.0f) osum *= p.q_scale;
-            if (s == 0 && col_ok) p.out[(size_t)(t0 + tt) * p.H * p.dv + (size_t)h * p.dv + j] = osum;
         }
     }
     if (col_ok) {
 #pragma unroll
-        for (int r = 0; r < NR; r++) {
+        for (int r = 0; r < NR; r += 2) {
             const int i = ((r >> 2) * LPC + s) * 4 + (r & 3);
-            if (i < p.dk) sp[(size_t)i * p.dv] = S[r];
+            const float2 v = unpack2(S[r / 2]);
+            if (i < p.dk) sp[(size_t)i * p.dv] = v.x;
+            if (i + 1 < p.dk) sp[(size_t)(i + 1) * p.dv] = v.y;
         }
     }
 }
@@ -1116,7 +1155,9 @@ static __global__ void __launch_bounds__(128) ssm_pre_kernel(const SsmPreParams 
 // The scan.  CTA = (block of state columns, head); a column j (one of the head's P value channels) of the state S [N][P]
 // belongs to `lpc` adjacent lanes, lane s of them holding NR rows in registers, in the row order of delta_scan_kernel so
 // that B and C entries are read with 16-byte shared-memory loads; a thread may own CPT adjacent columns, which share those reads.  Per token and row: S <- decay * S + (dt x_j) B_i, and
-// y_j += S C_i; one reduction across the lpc lanes, then + D x_j.  Tokens are staged DELTA_TB at a time by cp.async, the
+// y_j += S C_i; a reduction across the lpc lanes, eight tokens at a time (block_sums), then + D x_j.  Two rows go through one instruction.  What bounds it:
+// one or two warps per scheduler that issue every 3.8 cycles, waiting for shared memory and for their own results (1000 tokens of 64 heads of 64 x 128: 251 us with a
+// reduction per token, 214 without, 171 with 16 lanes per column instead of 8, 166 with four columns per thread instead of two).  Tokens are staged DELTA_TB at a time by cp.async, the
 // next block in flight while this one is used.  The order of every sum is fixed, so a token's result does not depend on the
 // portion it arrives in.  The state is read at the start (zeros when the step starts at position 0) and written back at
 // the end.
@@ -1178,14 +1219,15 @@ template <int NR, int LPC, int CPT> __global__ void __launch_bounds__(DELTA_THRE
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     stage(0, 0);
-    float S[CPT][NR];
+    f32pair S[CPT][NR / 2];   // neighbouring rows in pairs
     float* sp = p.state + ((size_t)h * p.N) * p.P + j;
 #pragma unroll
     for (int cc = 0; cc < CPT; cc++)
 #pragma unroll
-        for (int r = 0; r < NR; r++) {
+        for (int r = 0; r < NR; r += 2) {
             const int i = ((r >> 2) * LPC + s) * 4 + (r & 3);
-            S[cc][r] = (pos0 > 0 && j + cc < p.P && i < p.N) ? sp[(size_t)i * p.P + cc] : 0.0f;
+            const bool in = pos0 > 0 && j + cc < p.P;
+            S[cc][r / 2] = pack2(in && i < p.N ? sp[(size_t)i * p.P + cc] : 0.0f, in && i + 1 < p.N ? sp[(size_t)(i + 1) * p.P + cc] : 0.0f);
         }
     const float dskip = p.D ? p.D[h] : 0.0f;
     int buf = 0;
@@ -1199,43 +1241,74 @@ template <int NR, int LPC, int CPT> __global__ void __launch_bounds__(DELTA_THRE
         const float* xs = cs + DELTA_TB * dkp;
         const float* dts = xs + DELTA_TB * cols;
         const float* des = dts + DELTA_TB;
-        for (int tt = 0; tt < nt; tt++) {
-            const float a = des[tt], dtv = dts[tt];
-            float xv[CPT], dtx[CPT], y[CPT][4];
+        auto token = [&](int tt, float (&share)[CPT]) {   // one token; this lane's share of its outputs
+            const f32pair a = dup2(des[tt]);
+            f32pair dtx[CPT], y[CPT][2];
 #pragma unroll
             for (int cc = 0; cc < CPT; cc++) {
-                xv[cc] = xs[tt * cols + jl + cc];
-                dtx[cc] = dtv * xv[cc];
-                y[cc][0] = y[cc][1] = y[cc][2] = y[cc][3] = 0.0f;
+                dtx[cc] = dup2(dts[tt] * xs[tt * cols + jl + cc]);
+                y[cc][0] = y[cc][1] = 0ull;
             }
 #pragma unroll
             for (int r4 = 0; r4 < NR / 4; r4++) {
                 const int i = (r4 * LPC + s) * 4;
-                const float4 b4 = *reinterpret_cast<const float4*>(bs + tt * dkp + i);
-                const float4 c4 = *reinterpret_cast<const float4*>(cs + tt * dkp + i);
-                const float bv[4] = {b4.x, b4.y, b4.z, b4.w}, cv[4] = {c4.x, c4.y, c4.z, c4.w};
+                const ulonglong2 b4 = *reinterpret_cast<const ulonglong2*>(bs + tt * dkp + i);
+                const ulonglong2 c4 = *reinterpret_cast<const ulonglong2*>(cs + tt * dkp + i);
 #pragma unroll
-                for (int cc = 0; cc < CPT; cc++)
-#pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        S[cc][4 * r4 + k] = fmaf(a, S[cc][4 * r4 + k], dtx[cc] * bv[k]);
-                        y[cc][k] = fmaf(S[cc][4 * r4 + k], cv[k], y[cc][k]);
-                    }
+                for (int cc = 0; cc < CPT; cc++) {
+                    f32pair n0 = mul2(dtx[cc], b4.x), n1 = mul2(dtx[cc], b4.y);
+                    fma2(n0, a, S[cc][2 * r4]); fma2(n1, a, S[cc][2 * r4 + 1]);
+                    S[cc][2 * r4] = n0; S[cc][2 * r4 + 1] = n1;
+                    fma2(y[cc][0], n0, c4.x); fma2(y[cc][1], n1, c4.y);
+                }
             }
 #pragma unroll
             for (int cc = 0; cc < CPT; cc++) {
-                float ysum = (y[cc][0] + y[cc][1]) + (y[cc][2] + y[cc][3]);
-                for (int o = LPC >> 1; o > 0; o >>= 1) ysum += __shfl_xor_sync(0xffffffffu, ysum, o);
-                if (s == 0 && j + cc < p.P) p.out[(size_t)(t0 + tt) * p.H * p.P + (size_t)h * p.P + j + cc] = fmaf(dskip, xv[cc], ysum);
+                const float2 ya = unpack2(y[cc][0]), yb = unpack2(y[cc][1]);
+                share[cc] = (ya.x + ya.y) + (yb.x + yb.y);
+            }
+        };
+        float* dst = p.out + (size_t)t0 * p.H * p.P + (size_t)h * p.P + j;
+        if (nt == DELTA_TB) {
+            float yv[CPT][DELTA_TB];
+#pragma unroll
+            for (int tt = 0; tt < DELTA_TB; tt++) {
+                float share[CPT];
+                token(tt, share);
+#pragma unroll
+                for (int cc = 0; cc < CPT; cc++) yv[cc][tt] = share[cc];
+            }
+#pragma unroll
+            for (int cc = 0; cc < CPT; cc++) {
+                const BlockSums b = block_sums<LPC>(yv[cc], s);
+                if (b.writes && j + cc < p.P)
+#pragma unroll
+                    for (int i = 0; i < DELTA_TB; i++)
+                        if (i < b.n) dst[(size_t)(b.first + i) * p.H * p.P + cc] = fmaf(dskip, xs[(b.first + i) * cols + jl + cc], yv[cc][i]);
+            }
+        } else {
+#pragma unroll 1
+            for (int tt = 0; tt < nt; tt++) {
+                float share[CPT];
+                token(tt, share);
+#pragma unroll
+                for (int cc = 0; cc < CPT; cc++) {
+                    float ysum = share[cc];
+#pragma unroll
+                    for (int o = LPC >> 1; o > 0; o >>= 1) ysum += __shfl_xor_sync(0xffffffffu, ysum, o);
+                    if (s == 0 && j + cc < p.P) dst[(size_t)tt * p.H * p.P + cc] = fmaf(dskip, xs[tt * cols + jl + cc], ysum);
+                }
             }
         }
     }
 #pragma unroll
     for (int cc = 0; cc < CPT; cc++)
 #pragma unroll
-        for (int r = 0; r < NR; r++) {
+        for (int r = 0; r < NR; r += 2) {
             const int i = ((r >> 2) * LPC + s) * 4 + (r & 3);
-            if (j + cc < p.P && i < p.N) sp[(size_t)i * p.P + cc] = S[cc][r];
+            const float2 v = unpack2(S[cc][r / 2]);
+            if (j + cc < p.P && i < p.N) sp[(size_t)i * p.P + cc] = v.x;
+            if (j + cc < p.P && i + 1 < p.N) sp[(size_t)(i + 1) * p.P + cc] = v.y;
         }
 }
 

@@ -354,19 +354,19 @@ template <typename AT, typename WT> class RupenexModel : public DenseModel<AT, W
         SsmScanParams sp{};
         sp.xbc = qa; sp.ld = C; sp.b_off = inner; sp.c_off = inner + gn; sp.dt = dt; sp.decay = decay; sp.D = L.dskip; sp.state = L.state; sp.out = ys;
         sp.T = T; sp.H = c.H; sp.G = c.G; sp.N = c.N; sp.P = c.dv; sp.ps = ps;
-        // (rows per lane, lanes per column) with rows * lanes >= N.  The read-out's lane reduction is not on the path to the next
-        // token's state (unlike the delta rule's), so fewer lanes with more rows each do better here: 8 lanes of 16 rows at 128
-        // state rows measured 5 % under 16 lanes of 8, and 4 lanes of 32 another 1 % at half as many CTAs
-        int lpc = ssm_lanes > 0 ? ssm_lanes : (c.N <= 16 ? 1 : c.N <= 32 ? 2 : c.N <= 64 ? 4 : c.N <= 128 ? 8 : c.N <= 256 ? 16 : 32);
+        // (rows per lane, lanes per column) with rows * lanes >= N.  1000 tokens of 64 heads of 64 x 128, one column per thread: 8 rows on 16 lanes
+        // 243 us, 16 on 8 246, 32 on 4 240; what decides is how many columns share each read of a token's B and C entries (below): two 171 and
+        // 214 (8 and 16 rows), four 166 (8 rows)
+        int lpc = ssm_lanes > 0 ? ssm_lanes : (c.N <= 16 ? 1 : c.N <= 32 ? 2 : c.N <= 64 ? 4 : c.N <= 256 ? 16 : 32);
         while (lpc < 32 && 32 * lpc < c.N) lpc *= 2;
         const int nr = 8 * lpc >= c.N ? 8 : (16 * lpc >= c.N ? 16 : 32);
         int rc = 1;
 #define RP_SCAN(NR_, LPC_) if (nr == NR_ && lpc == LPC_) rc = launch_scan<NR_, LPC_, 1>(st, sp); else
-        // two columns per thread share each read of a token's B and C entries (12 % off the scan at 64 heads of 64 x 128); taken
-        // when the grid still has a CTA for at least half of the SMs
-        const bool two_ok = (nr == 8 && (lpc == 8 || lpc == 16)) || (nr == 16 && lpc == 8);
-        const int ctas2 = ((c.dv + 2 * (DELTA_THREADS / lpc) - 1) / (2 * (DELTA_THREADS / lpc))) * c.H;
-        const int cpt = ssm_cols > 0 ? ssm_cols : (two_ok && 2 * ctas2 >= sms ? 2 : 1);
+        // two or four columns per thread; taken when the grid still has a CTA for at least half of the SMs
+        const bool two_ok = (nr == 8 && (lpc == 8 || lpc == 16)) || (nr == 16 && lpc == 8), four_ok = nr == 8 && lpc == 16;
+        auto ctas = [&](int n) { const int cols = n * (DELTA_THREADS / lpc); return (c.dv + cols - 1) / cols * c.H; };
+        const int cpt = ssm_cols > 0 ? ssm_cols : four_ok && 2 * ctas(4) >= sms ? 4 : two_ok && 2 * ctas(2) >= sms ? 2 : 1;
+        if (cpt == 4 && four_ok) rc = launch_scan<8, 16, 4>(st, sp); else
         if (cpt == 2 && nr == 8 && lpc == 16) rc = launch_scan<8, 16, 2>(st, sp);
         else if (cpt == 2 && nr == 16 && lpc == 8) rc = launch_scan<16, 8, 2>(st, sp);
         else if (cpt == 2 && nr == 8 && lpc == 8) rc = launch_scan<8, 8, 2>(st, sp);

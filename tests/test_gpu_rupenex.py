@@ -188,6 +188,24 @@ def test_scan_with_two_columns_per_thread(gpu_lib, tmp_path, state, vdim):
     m.close()
 
 
+@pytest.mark.parametrize("state,vdim,n", [(72, 6, 8), (100, 35, 17), (128, 40, 50), (128, 64, 7)])
+def test_scan_with_four_columns_per_thread(gpu_lib, tmp_path, state, vdim, n):
+    """the same with four columns, around whole blocks of eight tokens (whose read-outs are reduced together) and rests of them"""
+    cfg = O.make_config([S(heads=2, vdim=vdim, state=state, groups=1, norm_groups=1, mlp=None), S(heads=4, vdim=vdim, state=state, groups=2, conv=2, mlp=None)])
+    toks = tokens_for(cfg, n, seed=5)
+    W = O.random_weights(cfg, seed=14, gain=2.0)
+    want, _ = O.forward(cfg, W, toks)
+    m = open_model(gpu_lib, tmp_path, cfg, W, "float32")
+    m.set_option("ssm_cols", 1)
+    one = m.forward_tokens(toks, 0, list(range(n)))
+    m.set_option("ssm_cols", 4)
+    four = m.forward_tokens(toks, 0, list(range(n)))
+    assert O.rel_rms(four, want) < TOL["float32"] and np.array_equal(one, four)   # the same sums in the same order
+    parts = np.concatenate([m.forward_tokens(toks[:5], 0, list(range(5)))] + [m.forward(toks[i], i).copy()[None] for i in range(5, n)])
+    assert O.rel_rms(parts, want) < TOL["float32"]
+    m.close()
+
+
 def test_wanted_rows_in_any_order(gpu_lib, tmp_path):
     cfg = mixed_cfg()
     toks = tokens_for(cfg, 40)
