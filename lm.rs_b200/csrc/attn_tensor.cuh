@@ -75,6 +75,8 @@ struct AttnSplitParams {
 };
 static __global__ void __launch_bounds__(256) attn_split_kernel(const AttnSplitParams p) {
     __shared__ float tile[64][65];
+    pdl_launch();
+    pdl_wait();
     const int u = blockIdx.x >> 1, g = blockIdx.y, part = blockIdx.z;
     const int key0 = (u < p.kf ? u : p.first + u - p.kf) * AX_KEYS + (blockIdx.x & 1) * 64;
     float v[8];
@@ -173,6 +175,8 @@ attn_tensor_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
+    pdl_wait();
+    pdl_launch();   // (not before this CTA has its TMEM)
     // registers: 384 x 168 at launch = 256 x 232 for the rows of the groups + 128 x 40
     if (warp >= 8) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");

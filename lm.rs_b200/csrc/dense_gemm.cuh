@@ -204,6 +204,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     int m0 = blockIdx.y * TG_M, row_end = p.T, wrow0 = 0;
     const int n0 = blockIdx.x * OUT_COLS;
     if (p.grp) {   // tiles past the group's last row leave before anything is set up (the whole CTA takes this branch)
+        pdl_wait();
         m0 += p.grp[blockIdx.z];
         row_end = p.grp[blockIdx.z + 1];
         wrow0 = (int)blockIdx.z * p.O;
@@ -225,6 +226,8 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
+    pdl_wait();
+    pdl_launch();   // (not before this CTA has its TMEM: a successor that took it would hold it until this kernel ends)
 
     if (warp == 0) {
         if (lane == 0) {   // ---- TMA producer ----
@@ -400,6 +403,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_con
     cluster_sync();   // the other CTAs' barriers exist before anything is signalled there
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
+    pdl_wait();
+    pdl_launch();
 
     if (warp == 0) {
         if (lane == 0) {   // ---- TMA producer: this CTA's rows of A and of W ----
@@ -532,6 +537,7 @@ struct DenseGemmCtx {
     std::map<std::pair<const void*, int>, CUtensorMap> wmaps;   // (weight matrix, box rows) -> tensor map
     bool attr_set[4][2] = {}, pair_attr_set[4][3] = {}, split_attr_set[4] = {};
     int at_once[2] = {};   // clusters of two and of four CTAs that run at the same time with one CTA per SM (0: not asked yet)
+    bool pdl = false;          // chain the launches (programmatic dependent launch)
     int form = GEMM_BY_SIZE;   // option: this form for every product of more than 128 rows that it can serve
     ~DenseGemmCtx() { if (h_err) cudaFreeHost(h_err); }
 };
@@ -637,10 +643,12 @@ inline int dense_gemm_launch(DenseGemmCtx& c, cudaStream_t st, int T, const AT* 
             cfg.gridDim = dim3((O + oc - 1) / oc * cluster, (T + 255) / 256); cfg.blockDim = dim3(TG_THREADS); cfg.stream = st;
             p.stages = tg_pair_stages(bn, form == 2 ? 2 : 1, gemm_whole_sm((long long)cfg.gridDim.x / cluster * cfg.gridDim.y, c.at_once[form == GEMM_SPLIT]));
             cfg.dynamicSmemBytes = tg_pair_smem(bn, p.stages);
-            cudaLaunchAttribute attr[1];
+            cudaLaunchAttribute attr[2];
             attr[0].id = cudaLaunchAttributeClusterDimension;
             attr[0].val.clusterDim.x = cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-            cfg.attrs = attr; cfg.numAttrs = 1;
+            attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[1].val.programmaticStreamSerializationAllowed = 1;
+            cfg.attrs = attr; cfg.numAttrs = c.pdl ? 2 : 1;
             const cudaError_t ce = cudaLaunchKernelEx(&cfg, kernel, ta, tb, tb2, p);
             if (ce != cudaSuccess) { err = std::string("gemm_bf16_pair_kernel: ") + cudaGetErrorString(ce); return 1; }
             return 0;
@@ -656,9 +664,14 @@ inline int dense_gemm_launch(DenseGemmCtx& c, cudaStream_t st, int T, const AT* 
         const int out_cols = (GLU || narrow) ? 64 : TG_N;
         const int rows_y = n_groups > 0 ? std::min(T, max_group_rows) : T;
         const dim3 grid((O + out_cols - 1) / out_cols, (rows_y + TG_M - 1) / TG_M, n_groups > 0 ? n_groups : 1);
-        if (narrow) gemm_bf16_tc_kernel<EPI, GLU ? 128 : 64><<<grid, TG_THREADS, TG_SMEM, st>>>(ta, tb, tb2, p);
-        else gemm_bf16_tc_kernel<EPI, 128><<<grid, TG_THREADS, TG_SMEM, st>>>(ta, tb, tb2, p);
-        cudaError_t ce = cudaGetLastError();
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = grid; cfg.blockDim = dim3(TG_THREADS); cfg.stream = st; cfg.dynamicSmemBytes = TG_SMEM;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr; cfg.numAttrs = c.pdl ? 1 : 0;
+        const cudaError_t ce = narrow ? cudaLaunchKernelEx(&cfg, gemm_bf16_tc_kernel<EPI, GLU ? 128 : 64>, ta, tb, tb2, p)
+                                      : cudaLaunchKernelEx(&cfg, gemm_bf16_tc_kernel<EPI, 128>, ta, tb, tb2, p);
         if (ce != cudaSuccess) { err = std::string("gemm_bf16_tc_kernel: ") + cudaGetErrorString(ce); return 1; }
         return 0;
     }

@@ -16,6 +16,8 @@ namespace dense {
 // The rows of A, split once per product: [plane][T][kp], kp = K padded to 8, zeros in the padding
 struct SplitRowsParams { const float* a; int lda, T, K, kp; uint16_t* out; };
 static __global__ void __launch_bounds__(256) split_rows_kernel(const SplitRowsParams p) {
+    pdl_launch();
+    pdl_wait();
     const int pieces = p.kp >> 3;
     const size_t plane = (size_t)p.T * p.kp;
     for (long long e = (long long)blockIdx.x * 256 + threadIdx.x; e < (long long)p.T * pieces; e += (long long)gridDim.x * 256) {
@@ -91,6 +93,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
+    pdl_wait();
+    pdl_launch();   // (not before this CTA has its TMEM)
     // registers: 512 x 128 at launch = 128 x 232 for the sums + 256 x 104 + 128 x 72
     if (warp >= 12) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
@@ -318,15 +322,18 @@ inline int gemm_split_launch(DenseGemmCtx& c, cudaStream_t st, const GemmTiledPa
     }
     SplitRowsParams sp{q.a, q.lda, q.T, q.K, kp, planes};
     const long long pieces = (long long)q.T * (kp / 8);
-    split_rows_kernel<<<(unsigned)std::min<long long>((pieces + 255) / 256, 8LL * c.sms), 256, 0, st>>>(sp);
-    cudaError_t ce = cudaGetLastError();
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = dim3((unsigned)std::min<long long>((pieces + 255) / 256, 8LL * c.sms)); cfg.blockDim = dim3(256); cfg.stream = st;
+    cfg.attrs = attr; cfg.numAttrs = c.pdl ? 1 : 0;
+    cudaError_t ce = cudaLaunchKernelEx(&cfg, split_rows_kernel, sp);
     if (ce == cudaSuccess) {
-        cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3((unsigned)((q.O + (GLU ? 63 : 127)) / (GLU ? 64 : 128) * p.n_tiles * p.splits)); cfg.blockDim = dim3(FX_THREADS); cfg.stream = st; cfg.dynamicSmemBytes = FX_SMEM;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = p.splits; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr; cfg.numAttrs = 1;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = p.splits; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+        cfg.attrs = c.pdl ? attr : attr + 1; cfg.numAttrs = c.pdl ? 2 : 1;
         ce = cudaLaunchKernelEx(&cfg, gemm_split_kernel<EPI>, tw, tw2, tx, p);
     }
     if (ce != cudaSuccess) { err = std::string("gemm_split_kernel: ") + cudaGetErrorString(ce); return 1; }

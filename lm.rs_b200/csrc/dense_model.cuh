@@ -78,6 +78,9 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
     // programmatic dependent launch of the decode chain is an option.  An architecture turns it on where it measures faster (Genetar);
     // chains of many small kernels lose a little (Tudatar, 16 steps of 3 layers: 2.96 -> 3.03 ms)
     int use_graph = 1, use_pdl = 0;
+    // ... and of a prompt portion's.  Most of its kernels are short (512 tokens, 3 layers: 25 of them in 600 us), and the next one's launch, barriers and TMEM
+    // are ready when one ends: 512 tokens, Llama-3.2-1B shapes, Genetar 600 -> 524 us, Tudatar 1125 -> 1037, 2048 tokens of 3B shapes 1602 -> 1584.  Rupenex loses (1084 -> 1105).
+    int prompt_pdl = 0;
     int attn_tiles = -1;   // option: 2 / 1 the tensor-core / the register-tiled attention wherever it can run, 0 neither, -1 by attn_tensor and attn_large_tiles
     int gemm_split = -1;   // option: 1 / 0 float32 products on the tensor cores wherever they can run / nowhere, -1 by gemm_split_pays
     uint16_t* split_planes = nullptr;   // pieces of the running call's f32 operands (attn_tensor.cuh)
@@ -249,7 +252,12 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
         if (e != cudaSuccess) { error = std::string(what) + ": " + cudaGetErrorString(e); return 1; }
         return 0;
     }
-    bool pdl_now = false;   // set while a decode step is being enqueued
+    bool pdl_now = false;   // set while a decode step or a prompt portion is being enqueued
+    struct Chained {        // ... and cleared however that ends
+        DenseModel& m;
+        Chained(DenseModel& model, bool on) : m(model) { m.pdl_now = m.gemm_ctx.pdl = on; }
+        ~Chained() { m.pdl_now = m.gemm_ctx.pdl = false; }
+    };
     // Lets a kernel ask for `smem` bytes of dynamic shared memory.  Without it a launch may use 48 KB, the kernel's own static arrays
     // included (a one-row product 12288 floats wide asks for exactly 48 KB beside a few hundred static bytes).
     std::map<const void*, size_t> smem_limit;   // dynamic bytes each kernel may ask for so far
@@ -298,7 +306,7 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
             if (gemm_f32_usable(p)) {
                 constexpr int cols = EPI == EPI_GLU ? FG_N / 2 : FG_N;
                 return optin(gemm_f32_kernel<EPI>, FG_SMEM) ||
-                       launch_k("gemm_f32_kernel", st, false, gemm_f32_kernel<EPI>, dim3((p.O + cols - 1) / cols, (rows + FG_M - 1) / FG_M, nb), dim3(FG_THREADS), FG_SMEM, p);
+                       launch_k("gemm_f32_kernel", st, pdl_now, gemm_f32_kernel<EPI>, dim3((p.O + cols - 1) / cols, (rows + FG_M - 1) / FG_M, nb), dim3(FG_THREADS), FG_SMEM, p);
             }
         }
         gemm_tiled_kernel<AT, WT, EPI><<<dim3((p.O + 63) / 64, (rows + 63) / 64, nb), 256, 0, st>>>(p);
@@ -445,10 +453,10 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
         if (!tg_make_map(gemm_ctx, &mk, s.kp, (size_t)dkp * 2, (size_t)dkp * 2, (size_t)3 * p.G * s.n_pad, AX_KEYS) ||
             !tg_make_map(gemm_ctx, &mv, s.vp, (size_t)s.n_pad * 2, (size_t)s.n_pad * 2, (size_t)3 * p.G * dvp, dvp))
             return -1;
-        if (launch_k("attn_split_kernel", st, false, attn_split_kernel, dim3(2 * (s.kf + tiles - s.first), p.G, 1 + (dvp + 63) / 64), dim3(256), 0, s)) return 1;
+        if (launch_k("attn_split_kernel", st, pdl_now, attn_split_kernel, dim3(2 * (s.kf + tiles - s.first), p.G, 1 + (dvp + 63) / 64), dim3(256), 0, s)) return 1;
         const size_t smem = attn_tensor_smem(p.dk);
         const dim3 grid(p.G * chunks, (p.T + p.TQ - 1) / p.TQ);
-        auto go = [&](auto kernel) { return optin(kernel, smem) || launch_k("attn_tensor_kernel", st, false, kernel, grid, dim3(AX_THREADS), smem, mk, mv, p, s.n_pad, gemm_ctx.d_err); };
+        auto go = [&](auto kernel) { return optin(kernel, smem) || launch_k("attn_tensor_kernel", st, pdl_now, kernel, grid, dim3(AX_THREADS), smem, mk, mv, p, s.n_pad, gemm_ctx.d_err); };
         return p.dv <= 64 ? go(attn_tensor_kernel<AT, 1>) : go(attn_tensor_kernel<AT, 2>);
     }
     // attention over T query rows: the caller fills the tensors, head geometry, pitches, scale, soft-cap, window, kept first keys,
@@ -596,6 +604,7 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
                 GCK(cudaMemcpyAsync(d_rows, rows.data(), (size_t)m * 4, cudaMemcpyHostToDevice, st));
                 GCK(cudaStreamSynchronize(st));   // `rows` is a local
             }
+            const Chained chained(*this, T > 1 && prompt_pdl);   // (for this portion's layers and head)
             if (run_layers(st, T, ps, pos + (uint32_t)c0)) return 1;
             if (m == 0) continue;
             if (T == 1) {
@@ -635,6 +644,7 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
         else if (!strcmp(name, "attn_tiles")) attn_tiles = value;
         else if (!strcmp(name, "gemm_form")) gemm_ctx.form = std::max(-2, std::min(2, value));
         else if (!strcmp(name, "gemm_split")) gemm_split = value;
+        else if (!strcmp(name, "prompt_pdl")) prompt_pdl = value;
         else if (!strcmp(name, "pdl")) { use_pdl = value; drop_graphs(); }
         else set_model_option(name, value);
     }

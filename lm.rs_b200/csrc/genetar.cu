@@ -132,6 +132,7 @@ template <typename AT, typename WT> class GenetarModel : public DenseModel<AT, W
     int load(const std::string& dir, const Json& cfg, const ArchOptions& opt) {
         sms = opt.sms;
         gemm_ctx.sms = opt.sms;
+        B::prompt_pdl = 1;
         B::use_pdl = 1;   // its decode chain is mostly one-row products that have their first weights in flight while they wait: 370 -> 346 us
                           // per step (6 layers at width 2048, waited for on the host), 96 -> 85 (3 layers at width 256)
         width = (int)cfg.at("width").number(0);
@@ -256,8 +257,7 @@ template <typename AT, typename WT> class GenetarModel : public DenseModel<AT, W
             } else {
                 NormRowsParams<AT> np{};
                 np.x = x; np.ldx = width; np.w = L.norm1; np.out = h; np.ldo = width; np.n = width; np.eps = info.eps;
-                rmsnorm_rows_kernel<AT><<<T, 256, 0, st>>>(np);
-                if (check_launch("rmsnorm_rows_kernel")) return 1;
+                if (launch_k("rmsnorm_rows_kernel", st, pdl_now, rmsnorm_rows_kernel<AT>, dim3(T), dim3(256), 0, np)) return 1;
                 if (this->template matmul<EPI_STORE>(st, T, h, width, L.wqkv, nullptr, width, L.qkv_rows, e_qkv)) return 1;
                 if (c.has_mlp && this->template matmul<EPI_GLU>(st, T, h, width, L.wgate, L.wup, width, c.ff, e_glu)) return 1;
             }
@@ -293,8 +293,7 @@ template <typename AT, typename WT> class GenetarModel : public DenseModel<AT, W
         }
         NormRowsParams<AT> np{};
         np.x = x; np.ldx = width; np.rows = rows_dev; np.w = final_norm; np.out = hn; np.ldo = width; np.n = width; np.eps = info.eps;
-        rmsnorm_rows_kernel<AT><<<m, 256, 0, st>>>(np);
-        if (check_launch("rmsnorm_rows_kernel")) return 1;
+        if (launch_k("rmsnorm_rows_kernel", st, pdl_now, rmsnorm_rows_kernel<AT>, dim3(m), dim3(256), 0, np)) return 1;
         return this->template matmul<EPI_STORE>(st, m, hn, width, head, nullptr, width, vocab, e);
     }
 
