@@ -1,6 +1,7 @@
 // attn_tiles.cuh -- attention of many query rows (prompts and long portions) in f32 on CUDA cores, as two register-tiled
 // products per key tile.  Same parameters and arithmetic rules as attn_rows_kernel (dense_ops.cuh), which serves one-row steps and the
-// portions that would leave SMs idle here (attn_large_tiles).
+// portions that would leave SMs idle here (attn_large_tiles).  Long portions of heads up to 128 run on the tensor cores (attn_tensor.cuh); here: fewer than
+// 512 keys, sigmoid weights, shared latents, wider keys.
 #pragma once
 #include "dense_ops.cuh"
 

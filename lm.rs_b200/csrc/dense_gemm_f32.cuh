@@ -1,5 +1,6 @@
 // dense_gemm_f32.cuh -- many-row products of the float32 operand mode on CUDA cores:
 //     out[T][O] = A[T][K] . W[O][K]^T, all f32,  then one of the epilogues of dense_ops.cuh
+// (the small ones, the batched and the grouped ones: the rest runs on the tensor cores, dense_gemm_split.cuh, by gemm_split_pays)
 // for rows that start on 16-byte boundaries (K, the pitch of A and the batch strides multiples of 4); gemm_tiled_kernel serves every
 // other shape and the bf16 shapes the tensor-core kernel cannot take.
 //

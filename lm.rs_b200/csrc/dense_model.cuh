@@ -97,8 +97,33 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
     // called before a step of n tokens at position pos is enqueued (models with state that is not addressed by position check it here)
     virtual int begin_step(uint32_t pos, size_t n) { (void)pos; (void)n; return 0; }
 
+    // A second stream for what may run beside the main one within a step: side_fork lets it start after what is in `st` so far, side_join makes `st` wait
+    // for it.  Captured steps become graphs with two branches.  side_fork is false where the stream cannot be had (the caller then stays on `st`).
+    cudaStream_t side = nullptr;
+    cudaEvent_t side_from = nullptr, side_to = nullptr;
+    bool side_fork(cudaStream_t st) {
+        if (!side) {
+            if ((!side_from && cudaEventCreateWithFlags(&side_from, cudaEventDisableTiming) != cudaSuccess) ||
+                (!side_to && cudaEventCreateWithFlags(&side_to, cudaEventDisableTiming) != cudaSuccess) ||
+                cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking) != cudaSuccess) {
+                (void)cudaGetLastError();
+                side = nullptr;
+                return false;
+            }
+        }
+        return cudaEventRecord(side_from, st) == cudaSuccess && cudaStreamWaitEvent(side, side_from, 0) == cudaSuccess;
+    }
+    int side_join(cudaStream_t st) {
+        GCK(cudaEventRecord(side_to, side));
+        GCK(cudaStreamWaitEvent(st, side_to, 0));
+        return 0;
+    }
+
     ~DenseModel() override {
         drop_graphs();
+        if (side) cudaStreamDestroy(side);
+        if (side_from) cudaEventDestroy(side_from);
+        if (side_to) cudaEventDestroy(side_to);
         for (void* p : owned) cudaFree(p);
     }
     template <typename T> int dalloc(T** p, size_t n) {

@@ -189,6 +189,25 @@ def test_first_tokens_and_a_prompt_of_one(gpu_lib, tmp_path):
     m.close()
 
 
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+def test_feed_forward_beside_the_mixer(gpu_lib, tmp_path, dtype):
+    """one-token steps with the feed-forward on a second stream and on the main one, as plain launches and replayed, chained and not, with layers
+    without a feed-forward between: the same logits to the bit over a run of steps (a product that started too early or too late would show)"""
+    cfg = mixed_cfg()
+    W = G.random_weights(cfg, seed=21)
+    toks = np.random.default_rng(8).integers(0, cfg["vocab"], 90).tolist()
+    m = gpu_lib.Transformer.open(G.write_model(str(tmp_path / "m"), cfg, W), dtype=dtype, max_tokens=128)
+    runs = []
+    for beside, graphs, pdl in ((0, 0, 0), (1, 0, 0), (1, 0, 1), (1, 1, 0), (1, 1, 1), (0, 1, 1)):
+        m.set_option("mlp_beside", beside)
+        m.set_option("graphs", graphs)
+        m.set_option("pdl", pdl)
+        m.forward_tokens(toks[:50], 0)
+        runs.append(np.stack([m.forward(t, i).copy() for i, t in enumerate(toks) if i >= 50]))
+    assert all(np.array_equal(runs[0], r) for r in runs[1:])
+    m.close()
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_long_greedy_generation_through_the_generate_loop(gpu_lib, tmp_path, dtype):
     cfg = mixed_cfg(logit_scale=3.0)
