@@ -352,7 +352,7 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
         GemmTiledParams<AT, WT> p{};
         p.a = a; p.lda = lda; p.w = w; p.w2 = w2; p.T = T; p.K = K; p.O = O; p.e = e;
         if constexpr (std::is_same<AT, float>::value && std::is_same<WT, float>::value) {
-            if (use_tc && gemm_f32_usable(p) && (gemm_split == 1 || (gemm_split < 0 && gemm_split_pays(EPI == EPI_GLU, T, K, O, sms))) && split_room((size_t)3 * T * gemm_split_kp(K))) {
+            if (use_tc && gemm_f32_usable(p) && (gemm_split == 1 || (gemm_split < 0 && gemm_split_pays(EPI == EPI_GLU, T, K, O, sms))) && split_room(st, (size_t)3 * T * gemm_split_kp(K))) {
                 const int rc = gemm_split_launch<EPI>(gemm_ctx, st, p, gemm_split_plan(EPI == EPI_GLU, T, K, O, sms), split_planes, error);
                 if (rc >= 0) { launches += 2; return rc; }
             }
@@ -442,8 +442,13 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
     }
     // Room for n elements of split operands.  Every user fills and reads them on the model's stream.  Grows by half at least, so that a
     // prompt in many portions allocates a few times; false: no memory (the caller takes a kernel that needs none).
-    bool split_room(size_t n) {
+    // Captured steps hold the buffer's address (a latent too wide for the shared form is up-projected by products of many rows in every step), so they go
+    // when it moves.  While a step is being captured nothing can be allocated: it has what its uncaptured first step got.
+    bool split_room(cudaStream_t st, size_t n) {
         if (n <= split_cap) return true;
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return false;
+        drop_graphs();
         const size_t more = std::max(n, split_cap + split_cap / 2);
         dfree(split_planes);
         split_planes = nullptr; split_cap = 0;
@@ -472,7 +477,7 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
         s.first = p.window > 0 ? std::max(0, pos0 - p.window + 1) / AX_KEYS : p.chunk > 0 ? pos0 / p.chunk * p.chunk / AX_KEYS : 0;
         s.kf = p.window > 0 && p.keep_first > 0 ? std::min(s.first, (p.keep_first + AX_KEYS - 1) / AX_KEYS) : 0;
         const size_t k_n = (size_t)3 * p.G * s.n_pad * dkp, n = k_n + (size_t)3 * p.G * s.n_pad * dvp;
-        if (!split_room(n)) return -1;
+        if (!split_room(st, n)) return -1;
         s.kp = split_planes; s.vp = split_planes + k_n;
         CUtensorMap mk, mv;
         if (!tg_make_map(gemm_ctx, &mk, s.kp, (size_t)dkp * 2, (size_t)dkp * 2, (size_t)3 * p.G * s.n_pad, AX_KEYS) ||

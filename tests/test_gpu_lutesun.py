@@ -405,6 +405,33 @@ def test_long_decoding_with_a_latent_that_is_always_up_projected(gpu_lib, tmp_pa
     m.close()
 
 
+def test_replayed_steps_when_the_workspace_of_wide_latents_has_moved(gpu_lib, tmp_path):
+    """steps captured for early positions, then a prompt so long that the pieces of the up-projected latents need more room than those steps
+    had, then the early positions again: the same logits to the bit as without graphs"""
+    n = 2200   # a second portion, with more rows to up-project than any step or portion before
+    cfg = O.make_config([G(heads=2, dim=8, rot_dim=4, vdim=8, kv_rank=528, q_rank=16, size=70, mlp=None), D(heads=2, dim=8, rot_dim=4, vdim=8, kv_rank=520, size=0, mlp=None)],
+                        width=24, vocab=40)
+    W = O.random_weights(cfg, seed=4, gain=1.5)
+    toks = tokens_for(cfg, n, seed=9)
+    want, _ = O.forward(cfg, W, toks[:80])
+    got = []
+    for graphs in (0, 1):
+        m = open_model(gpu_lib, tmp_path, cfg, W, "float32", max_tokens=n, name=f"m{graphs}")
+        m.set_option("graphs", graphs)
+        early = [[m.forward(toks[i], i).copy() for i in range(80)] for _ in range(2)]
+        whole = m.forward_tokens(toks, 0, [n - 1])
+        late = [m.forward(toks[i], i).copy() for i in range(n - 4, n)]
+        other = open_model(gpu_lib, tmp_path, cfg, W, "float32", max_tokens=n, name=f"o{graphs}")   # takes what was given back
+        other.forward_tokens(toks, 0, [n - 1])
+        early += [[m.forward(toks[i], i).copy() for i in range(80)]]
+        for e in early:
+            assert O.rel_rms(np.array(e), want) < TOL["float32"]
+        got.append(np.concatenate([np.array(early).reshape(240, -1), whole, np.array(late)]))
+        other.close()
+        m.close()
+    assert np.array_equal(got[0], got[1])
+
+
 TC_LAYERS = [
     D(heads=5, dim=24, rot_dim=8, vdim=24, kv_rank=40, size=50, mlp=O.dense(ff=200)),
     G(heads=6, dim=32, rot_dim=16, vdim=20, kv_rank=48, q_rank=56, size=100, mlp=M(7, 2, 2, ff=72, shared=56, groups=3, keep=2)),
