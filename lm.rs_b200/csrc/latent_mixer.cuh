@@ -132,7 +132,11 @@ template <typename AT, typename WT> class LatentModel : public DenseModel<AT, WT
                 first = bounded ? (int)(pos_hint / ATT_KT * ATT_KT) : -1;
                 n = bounded ? (int)std::min<uint32_t>(max_tokens, (pos_hint / ATT_KT + 1) * ATT_KT) : (int)max_tokens;
             }
-            const int j0 = c.window > 0 && first >= c.window ? (first - c.window + 1) / ATT_KT * ATT_KT : 0;   // the attention walks whole key tiles
+            // the attention reads whole key tiles from the first visible key's on (hidden keys of theirs with weight 0: they must be numbers): the widest
+            // tiles any kernel of several rows takes, those of attn_rows_kernel for one row
+            static_assert(AX_KEYS % TA_KEYS == 0 && AX_KEYS % ATT_KT == 0, "the widest key tile covers the others");
+            const int tile = T > 1 ? AX_KEYS : ATT_KT;
+            const int j0 = c.window > 0 && first >= c.window ? (first - c.window + 1) / tile * tile : 0;
             if (!kfull && (dalloc(&kfull, (size_t)max_tokens * max_kfull) || dalloc(&vfull, (size_t)max_tokens * max_vfull) || dalloc(&knope, (size_t)max_tokens * max_knope)))
                 return 1;
             qp.qfull = l_q;

@@ -432,6 +432,28 @@ def test_replayed_steps_when_the_workspace_of_wide_latents_has_moved(gpu_lib, tm
     assert np.array_equal(got[0], got[1])
 
 
+@pytest.mark.parametrize("window", [100, 512])
+def test_a_portion_behind_single_steps_reads_no_row_that_it_did_not_expand(gpu_lib, tmp_path, window):
+    """single steps attend in the latent space and leave no per-head keys and values; what an earlier sequence left there (NaN here) must not
+    enter a later portion, whose key tiles start below its window's first key"""
+    n0, pos = 30, window + 100   # (pos - window + 1) / 64 is odd: the first visible key lies in the second half of its tile of 128
+    cfg = O.make_config([D(heads=2, dim=8, rot_dim=4, vdim=8, kv_rank=24, size=window, mlp=None)], width=16, vocab=51)
+    W = O.random_weights(cfg, seed=7, gain=1.5)
+    bad = dict(W, embed=W["embed"].copy())
+    bad["embed"][50] = np.nan
+    toks = np.random.default_rng(3).integers(0, 50, pos + 40).tolist()
+    want, _ = O.forward(cfg, W, toks)
+    m = open_model(gpu_lib, tmp_path, cfg, bad, "float32", max_tokens=pos + 40)
+    m.set_option("attn_tiles", 2)
+    m.forward_tokens(toks[:n0] + [50] * 34, 0, [0])
+    m.forward_tokens(toks[:n0], 0, [0])
+    for i in range(n0, pos):
+        m.forward_device(toks[i], i)
+    got = m.forward_tokens(toks[pos:], pos, list(range(40)))
+    assert O.rel_rms(got[:, :50], want[pos:, :50]) < TOL["float32"]   # (the table is the head too: column 50 is NaN)
+    m.close()
+
+
 TC_LAYERS = [
     D(heads=5, dim=24, rot_dim=8, vdim=24, kv_rank=40, size=50, mlp=O.dense(ff=200)),
     G(heads=6, dim=32, rot_dim=16, vdim=20, kv_rank=48, q_rank=56, size=100, mlp=M(7, 2, 2, ff=72, shared=56, groups=3, keep=2)),
