@@ -299,8 +299,9 @@ attn_tensor_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
         const int t = t0 + r / p.HC, hl = h0 + r % p.HC, h = g * kv_mul + min(hl, kv_mul - 1);
         const bool row_ok = r / p.HC < p.TQ && t < p.T && hl < kv_mul;
         const int last = row_ok ? pos0 + t : -1;   // last visible key
-        float m = p.sink && row_ok && grp == 0 ? p.sink[h] * LOG2E : MASKED;
-        float l = p.sink && row_ok && grp == 0 ? 1.0f : 0.0f;
+        // a sink is a key without a value.  Below a hidden key's score it weighs nothing, and the maximum stays finite: the first tiles may be hidden
+        const float sink = p.sink && row_ok && grp == 0 ? p.sink[h] * LOG2E : -INFINITY;
+        float m = fmaxf(sink, MASKED), l = ex2(sink - m);
         const float r1 = p.r1 ? p.r1[h] : 0.0f, r2 = p.r1 ? p.r2[h] : 0.0f;
         const float scale2 = p.scale * LOG2E, cap2 = p.softcap * LOG2E;
         const float unit = p.softcap > 0.0f ? 2.0f / p.softcap * scale2 : scale2;   // with a cap: e^(2 s scale / cap) as a power of two

@@ -9,6 +9,7 @@ import numpy as np
 import pytest
 
 import genetar_oracle as G
+import rupenex_oracle as R
 
 pytestmark = pytest.mark.gpu
 
@@ -74,4 +75,22 @@ def test_scores_as_low_as_the_other_kernels_take_them(gpu_lib, tmp_path):
     got = m.forward_tokens(toks, 0, list(range(40)))
     assert np.isfinite(want[0]).all() and np.isfinite(got).all()
     assert G.rel_rms(got[0], want[0]) < 2e-4
+    m.close()
+
+
+@pytest.mark.parametrize("keep_first", [0, 200])
+def test_hidden_tiles_and_sinks_that_are_off(gpu_lib, tmp_path, keep_first):
+    """a prompt longer than its window by several key tiles, which both groups of warps skip or walk (those of kept first keys included), in heads
+    whose sink adds nothing (-inf, the lowest value of the weights' type) or something; whole, and in portions behind hidden tiles"""
+    n = 900
+    cfg = R.make_config([R.attention_layer(heads=8, kv_heads=2, dim=16, vdim=20, size=400, keep_first=keep_first, mlp=None)])
+    W = R.random_weights(cfg, seed=6, gain=2.0)
+    W["l0.mix.sink"] = np.array([-np.inf, -3.3895313892515355e38, 0.0, 2.0, -1e30, -np.inf, 5.0, -40.0])
+    toks = np.random.default_rng(keep_first).integers(0, cfg["vocab"], n).tolist()
+    want, _ = R.forward(cfg, W, toks)
+    m = gpu_lib.Transformer.open(R.write_model(str(tmp_path / "m"), cfg, W), dtype="float32", max_tokens=n)
+    assert R.rel_rms(m.forward_tokens(toks, 0, list(range(n))), want) < 2e-4
+    cuts = [0, 520, 580, 582, 850, n]
+    parts = [m.forward_tokens(toks[a:b], a, list(range(b - a))) for a, b in zip(cuts, cuts[1:])]
+    assert R.rel_rms(np.concatenate(parts), want) < 2e-4
     m.close()
