@@ -112,6 +112,35 @@ static __global__ void __launch_bounds__(256) attn_split_kernel(const AttnSplitP
     }
 }
 
+// A row whose result is not finite, once more with multiply-adds: an infinity has no pieces (theirs sum to NaN), and a NaN or an infinity spoils through
+// its weight 0 also the rows of the tile that do not see it.  Here only visible keys count, with the same arithmetic otherwise: a score of -inf weighs
+// nothing, one of +inf or NaN makes the row NaN.  acc: n of the row's columns from c0 on, unnormalised, AX_ROWS floats apart in shared memory; returns
+// the sum of the weights.  Slow (a thread, a row), and out of line for the registers: finite operands come here only if a sum leaves f32.
+template <typename AT>
+static __device__ __noinline__ float attn_row_again(const AttnRowsParams<AT>& p, int t, int g, int h, int c0, int n, float* acc) {
+    constexpr float LOG2E = 1.4426950408889634f, MASKED = -1e30f * LOG2E;
+    const float* q = p.q + ((size_t)t * p.H + h) * p.dk;
+    const int last = (int)p.ps.pos + t, from = max(0, p.window > 0 ? last - p.window + 1 : p.chunk > 0 ? last / p.chunk * p.chunk : 0);
+    const int keep = p.window > 0 ? min(p.keep_first, from) : 0;   // the row sees keys 0 .. keep and from .. last
+    const float sink = p.sink ? p.sink[h] * LOG2E : -INFINITY, scale2 = p.scale * LOG2E, cap2 = p.softcap * LOG2E;
+    float m = fmaxf(sink, MASKED), l = ex2(sink - m);
+    for (int c = 0; c < n; c++) acc[c * AX_ROWS] = 0.0f;
+    for (int j = keep > 0 ? 0 : from; j <= last; j = j + 1 == keep ? from : j + 1) {
+        const float* k = p.kcache + (size_t)j * p.k_ld + (size_t)g * p.dk;
+        float a = 0.0f;
+        for (int d = 0; d < p.dk; d++) a = fmaf(q[d], k[d], a);
+        a = p.softcap > 0.0f ? fmaf(-2.0f * cap2, rcp(ex2(a * (2.0f / p.softcap * scale2)) + 1.0f), cap2) : a * scale2;
+        if (p.r1) a -= p.r1[h] * lg2(1.0f + p.r2[h] * (float)(last - j));
+        const float mn = fmaxf(m, a), corr = ex2(m - mn), w = ex2(a - mn);
+        m = mn;
+        l = l * corr + w;
+        if (l != l) break;   // so is the whole row
+        const float* v = p.vcache + (size_t)j * p.v_ld + (size_t)g * p.dv + c0;
+        for (int c = 0; c < n; c++) acc[c * AX_ROWS] = fmaf(acc[c * AX_ROWS], corr, w * v[c]);
+    }
+    return l;
+}
+
 // ---- the kernel ---------------------------------------------------------------------------------------------------------------------
 // CTA = 128 query rows (tokens x grouped heads of one KV head, one row per TMEM lane) against the KV head's keys in tiles of 128; one CTA per SM.
 //   warps 0-3, 4-7   two groups that take alternate key tiles, a thread one row: the tile's scores from TMEM (once for the maximum, once
@@ -126,7 +155,7 @@ static __global__ void __launch_bounds__(256) attn_split_kernel(const AttnSplitP
 // NV: 64-column blocks of the values
 template <typename AT, int NV>
 static __global__ void __launch_bounds__(AX_THREADS, 1)
-attn_tensor_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const AttnRowsParams<AT> p, int n_pad, int* err) {
+attn_tensor_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ AttnRowsParams<AT> p, int n_pad, int* err) {
     constexpr int DV = 64 * NV, S_AT = 64, PV_AT = 384;   // TMEM columns: group x 192 + [weights 0 .. 191 over scores 64 .. 191], then the values' sums
     extern __shared__ uint8_t ax_raw[];
     uint8_t* sm = ax_raw + (((smem_u32(ax_raw) + 1023u) & ~1023u) - smem_u32(ax_raw));
@@ -421,7 +450,19 @@ attn_tensor_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
         if (ok && row_ok) {
             const float m2 = ml[(1 - grp) * 256 + r], l2 = ml[(1 - grp) * 256 + 128 + r];
             const float mn = fmaxf(m, m2), ca = ex2(m - mn), cb = ex2(m2 - mn);
-            const float ls = grp ? l2 * cb + l * ca : l * ca + l2 * cb;
+            float ls = grp ? l2 * cb + l * ca : l * ca + l2 * cb;
+            float numbers = ls * 0.0f;   // zero, unless something is an infinity or NaN
+#pragma unroll
+            for (int c = 0; c < HALF; c++) {
+                const float a = xch[(grp * HALF + c) * AX_ROWS + r], own = grp ? o[HALF + c] : o[c];
+                o[c] = own * ca + a * cb;
+                if (grp * HALF + c < p.dv) numbers = fmaf(o[c], 0.0f, numbers);
+            }
+            if (!(numbers == 0.0f)) {
+                ls = attn_row_again(p, t, g, h, grp * HALF, min(HALF, p.dv - grp * HALF), xch + grp * HALF * AX_ROWS + r);
+#pragma unroll
+                for (int c = 0; c < HALF; c++) o[c] = xch[(grp * HALF + c) * AX_ROWS + r];
+            }
             const float inv = (p.gate ? p.gate[(size_t)t * p.H + h] : 1.0f) * p.out_scale / ls;
             AT* dst = p.out + (size_t)t * p.out_ld + (size_t)h * p.dv;
             const float* gl = p.gate_logits ? p.gate_logits + (size_t)t * p.gate_ld + (size_t)h * p.dv : nullptr;
@@ -433,9 +474,7 @@ attn_tensor_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
                 float y[8];
 #pragma unroll
                 for (int j = 0; j < 8; j++) {
-                    const float a = xch[(grp * HALF + c8 + j) * AX_ROWS + r];
-                    const float own = grp ? o[HALF + c8 + j] : o[c8 + j];
-                    y[j] = (own * ca + a * cb) * inv;
+                    y[j] = o[c8 + j] * inv;
                     if (gl && c0 + j < p.dv) y[j] = y[j] / (1.0f + expf(-gl[c0 + j]));
                 }
                 if (vec) {

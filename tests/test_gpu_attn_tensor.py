@@ -94,3 +94,44 @@ def test_hidden_tiles_and_sinks_that_are_off(gpu_lib, tmp_path, keep_first):
     parts = [m.forward_tokens(toks[a:b], a, list(range(b - a))) for a, b in zip(cuts, cuts[1:])]
     assert R.rel_rms(np.concatenate(parts), want) < 2e-4
     m.close()
+
+
+@pytest.mark.parametrize("softcap", [None, 8.0])
+@pytest.mark.parametrize("dim", [10, 72])
+def test_a_key_that_scores_minus_infinity(gpu_lib, tmp_path, dim, softcap):
+    """a token whose key is beyond f32 in one dimension and scores -inf for every row: no weight (or, capped, the least one), as in 64 bits"""
+    n = 560   # long enough to take the kernel by itself
+    cfg = G.make_config([G.attention_layer("attention_2", heads=4, kv_heads=2, dim=dim, vdim=dim, ff=0, v_mix=False, scale=0.3, softcap=softcap, rot_dims=4)], bigram=None)
+    W = G.random_weights(cfg, seed=8, qk_gain=2.0)
+    W["embed"][:, 0], W["embed"][:, 1], W["l0.norm1"][0] = 1.0, 0.0, 1.0
+    W["embed"][60, 1] = -8.0
+    for name, column, value in (("q", 0, 1.0), ("k", 1, 2.0 ** 127)):
+        for h in range(4 if name == "q" else 2):
+            row = W["l0.mix." + name][h * dim + 7]
+            row[:] = 0.0
+            row[column] = value
+    toks = np.random.default_rng(n).integers(0, 60, n)
+    toks[[5, 130, 131, 300, 558]] = 60
+    toks = toks.tolist()
+    want, _ = G.forward(cfg, W, toks)
+    m = gpu_lib.Transformer.open(G.write_model(str(tmp_path / "m"), cfg, W), dtype="float32", max_tokens=n)
+    assert G.rel_rms(m.forward_tokens(toks, 0, list(range(n))), want) < 2e-4
+    parts = [m.forward_tokens(toks[a:b], a, list(range(b - a))) for a, b in ((0, 531), (531, n))]
+    assert G.rel_rms(np.concatenate(parts), want) < 2e-4
+    m.close()
+
+
+def test_rows_do_not_see_later_tokens_that_are_no_numbers(gpu_lib, tmp_path):
+    """a NaN among the keys and values of a later token of the same tile: the rows before it are what they are without it"""
+    n, at = 700, 600
+    cfg = G.make_config([G.attention_layer("attention_2", heads=4, kv_heads=2, dim=24, vdim=40, ff=0, v_mix=False, scale=0.3, rot_dims=4)], bigram=None)
+    W = G.random_weights(cfg, seed=9, qk_gain=2.0)
+    W["embed"][60, 3] = np.nan
+    toks = np.random.default_rng(n).integers(0, 60, n).tolist()
+    want, _ = G.forward(cfg, W, toks[:at])
+    m = gpu_lib.Transformer.open(G.write_model(str(tmp_path / "m"), cfg, W), dtype="float32", max_tokens=n)
+    toks[at] = 60
+    got = m.forward_tokens(toks, 0, list(range(n)))
+    assert G.rel_rms(got[:at], want) < 2e-4
+    assert np.isnan(got[at:]).all()
+    m.close()
