@@ -253,6 +253,7 @@ template <typename AT, typename WT> class BadepelModel : public DenseModel<AT, W
                 }
                 if (load_vec(st, l + "q.norm", nq, &L.qnorm) || load_vec(st, l + "k.norm", nk, &L.knorm)) return 1;
                 if (dalloc(&L.kcache, (size_t)max_tokens * nk) || dalloc(&L.vcache, (size_t)max_tokens * nv) || dalloc(&L.sink, (size_t)c.H)) return 1;
+                this->will_attend(c.G, c.dk, c.dv);
                 GCK(cudaMemset(L.sink, 0, (size_t)c.H * 4));   // the extra softmax entry has score 0 for every head
                 if (c.rot_dims > 0) {
                     std::vector<double> f;
@@ -325,7 +326,7 @@ template <typename AT, typename WT> class BadepelModel : public DenseModel<AT, W
         info.vocab = (uint32_t)vocab; info.width = (uint32_t)width; info.n_layers = (uint32_t)layers.size(); info.max_tokens = max_tokens;
         info.heads = (uint32_t)layers[0].c.H; info.kv_heads = (uint32_t)layers[0].c.G; info.head_dim = (uint32_t)layers[0].c.dk;
         info.ff = (uint32_t)layers[0].c.ff; info.dtype = opt.dtype; info.eps = eps;
-        return ensure_scratch(1);
+        return ensure_scratch(1) || this->reserve_split();
     }
 
     int ensure_scratch(size_t rows) override {

@@ -197,7 +197,7 @@ template <typename AT, typename WT> class BolapelModel : public DenseModel<AT, W
         info.vocab = (uint32_t)vocab; info.width = (uint32_t)width; info.n_layers = (uint32_t)nl; info.max_tokens = max_tokens;
         info.heads = (uint32_t)c0.H; info.kv_heads = (uint32_t)(c0.kind == BO_DELTA ? c0.H : c0.G); info.head_dim = (uint32_t)(c0.kind == BO_DELTA ? c0.d : c0.dk);
         info.ff = (uint32_t)c0.ff; info.dtype = opt.dtype; info.eps = eps;
-        return ensure_scratch(1);
+        return ensure_scratch(1) || this->reserve_split();
     }
 
     int ensure_scratch(size_t rows) override {

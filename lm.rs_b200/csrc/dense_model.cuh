@@ -85,6 +85,8 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
     int gemm_split = -1;   // option: 1 / 0 float32 products on the tensor cores wherever they can run / nowhere, -1 by gemm_split_pays
     uint16_t* split_planes = nullptr;   // pieces of the running call's f32 operands (attn_tensor.cuh)
     size_t split_cap = 0;               // its elements
+    size_t split_key = 0;               // what a key of the widest attention layer takes of them, what a row of the widest float32 product (its length): will_attend, load_stack
+    int split_k = 0;
 
     // what an architecture implements
     virtual size_t n_layers() const = 0;
@@ -240,6 +242,7 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
     }
     // matrices stacked into one: rows of `parts` in order, then zero rows up to a multiple of `row_multiple`
     int load_stack(const SafeTensors& st, const std::vector<std::pair<std::string, int>>& parts, int K, WT** out, int* rows_out, int row_multiple = 1) {
+        split_k = std::max(split_k, K);
         int rows = 0;
         for (const auto& pr : parts) rows += pr.second;
         const int padded = (rows + row_multiple - 1) / row_multiple * row_multiple;
@@ -440,8 +443,9 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
         if (p.dv <= 64) return pitch == 64 ? go(attn_tile_kernel<AT, 1, 64, 2, SIG, false>, 256) : pitch == 128 ? go(attn_tile_kernel<AT, 1, 128, 2, SIG, false>, 256) : go(attn_tile_kernel<AT, 1, 0, 2, SIG, false>, 256);
         return pitch == 128 ? go(attn_tile_kernel<AT, 2, 128, 1, SIG, false>, 128) : pitch == 96 ? go(attn_tile_kernel<AT, 2, 96, 1, SIG, false>, 128) : go(attn_tile_kernel<AT, 2, 0, 1, SIG, false>, 128);
     }
-    // Room for n elements of split operands.  Every user fills and reads them on the model's stream.  Grows by half at least, so that a
-    // prompt in many portions allocates a few times; false: no memory (the caller takes a kernel that needs none).
+    // Room for n elements of split operands.  Every user fills and reads them on the model's stream.  A model asks for what a first prompt can need when it is
+    // loaded (reserve_split); beyond that it grows by half at least, so that a prompt in many portions allocates a few times; false: no memory (the caller
+    // takes a kernel that needs none).
     // Captured steps hold the buffer's address (a latent too wide for the shared form is up-projected by products of many rows in every step), so they go
     // when it moves.  While a step is being captured nothing can be allocated: it has what its uncaptured first step got.
     bool split_room(cudaStream_t st, size_t n) {
@@ -460,6 +464,21 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
         owned.push_back(v);
         split_planes = static_cast<uint16_t*>(v);
         return true;
+    }
+    // an attention layer with softmax weights over G heads of keys and values of their own, as attention_launch will get it
+    void will_attend(int G, int dk, int dv) {
+        if (dk <= 128 && dv <= 128) split_key = std::max(split_key, (size_t)3 * G * (attn_tensor_pad(dk) + attn_tensor_pad(dv)));
+    }
+    // The last step of loading.  One allocation here instead of one to three in the first prompt: cudaMalloc and cudaFree take 0.3 to 2 ms each.  First prompt of a
+    // fresh model, the shortest of a dozen (ms; CUDA-core kernels | room made within the call | here): 512 tokens of Llama-3.2-1B shapes 3.2 | 3.3 | 3.1, Tudatar 8.2 | 8.5 | 7.8,
+    // 301 tokens in float32 5.3 | 4.4 | 3.3.  Only a convenience: never more than an eighth of what is free.
+    int reserve_split() {
+        const size_t rows = std::min<size_t>(max_tokens, chunk_rows), keys = (rows + AX_KEYS - 1) / AX_KEYS * AX_KEYS;
+        size_t n = attn_tensor((int)rows, 0, 0, 0) ? split_key * keys : 0, free_bytes = 0, all = 0;
+        if (std::is_same<WT, float>::value && rows > 1) n = std::max(n, 3 * rows * gemm_split_kp(std::max(split_k, width)));
+        if (n > 0 && cudaMemGetInfo(&free_bytes, &all) == cudaSuccess && 2 * n <= free_bytes / 8) split_room(nullptr, n);
+        (void)cudaGetLastError();
+        return 0;
     }
     // Tensor-core attention of T > 1 rows: 0 launched, 1 failed, -1 not possible here (the caller takes another kernel)
     int launch_attn_tensor(cudaStream_t st, AttnRowsParams<AT> p) {

@@ -199,6 +199,8 @@ template <typename AT, typename WT> class GenetarModel : public DenseModel<AT, W
                 if (need(st, p + "ls2", {width}, &t) || upload_f32(t, &L.ls2)) return 1;
             }
             if (dalloc(&L.kcache, (size_t)max_tokens * nk) || dalloc(&L.vcache, (size_t)max_tokens * nv)) return 1;
+            this->will_attend(c.G, c.dk, c.dv);
+            B::split_k = std::max({B::split_k, c.H * c.dv, c.has_mlp ? c.ff : 0});
             if (c.rotary && rot_table(c.rot, &L.rot_cos, &L.rot_sin)) return 1;
             max_qkv = std::max(max_qkv, L.qkv_rows); max_q = std::max(max_q, nq); max_att = std::max(max_att, c.H * c.dv);
             max_ff = std::max(max_ff, c.ff); max_v = std::max(max_v, nv); max_H = std::max(max_H, c.H); max_dv = std::max(max_dv, c.dv);
@@ -209,8 +211,7 @@ template <typename AT, typename WT> class GenetarModel : public DenseModel<AT, W
         info.vocab = (uint32_t)vocab; info.width = (uint32_t)width; info.n_layers = (uint32_t)layers.size(); info.max_tokens = max_tokens;
         info.heads = (uint32_t)layers[0].c.H; info.kv_heads = (uint32_t)layers[0].c.G; info.head_dim = (uint32_t)layers[0].c.dk;
         info.ff = (uint32_t)layers[0].c.ff; info.dtype = opt.dtype; info.eps = eps;
-        if (ensure_scratch(1)) return 1;
-        return 0;
+        return ensure_scratch(1) || this->reserve_split();
     }
 
     int ensure_scratch(size_t rows) {

@@ -84,6 +84,7 @@ template <typename AT, typename WT> class LatentModel : public DenseModel<AT, WT
                 }
         if (dalloc(&L.wukT, tr.size()) || this->upload_host(tr, L.wukT)) return 1;
         if (dalloc(&L.cache, (size_t)max_tokens * (c.rk + c.dr)) || dalloc(&L.cache_op, (size_t)max_tokens * c.rk)) return 1;
+        if (c.per_head_ok) this->will_attend(c.H, dq, c.dv);
         L.rot.dims = c.rot_dims; L.rot.halves = c.halves;
         if (c.rot_dims > 0 && this->angle_tables(c.rot_key, c.rot_f, c.rot_mult, &L.rot.cos, &L.rot.sin)) return 1;
         max_cq = std::max(max_cq, c.rq); max_qraw = std::max(max_qraw, c.rq > 0 ? c.H * dq : 0); max_qn = std::max(max_qn, c.H * c.dn);

@@ -159,7 +159,7 @@ template <typename AT, typename WT> class LutesunModel : public LatentModel<AT, 
         info.vocab = (uint32_t)vocab; info.width = (uint32_t)width; info.n_layers = (uint32_t)layers.size(); info.max_tokens = max_tokens;
         info.heads = (uint32_t)layers[0].mix.c.H; info.kv_heads = 1; info.head_dim = (uint32_t)layers[0].mix.c.dn;
         info.ff = (uint32_t)layers[0].f.ff; info.dtype = opt.dtype; info.eps = eps;
-        return ensure_scratch(1);
+        return ensure_scratch(1) || this->reserve_split();
     }
 
     int ensure_scratch(size_t rows) override {

@@ -183,6 +183,7 @@ template <typename AT, typename WT> class RupenexModel : public DenseModel<AT, W
                 if (load_vec(st, q + "q.norm", c.dk, &L.qnorm) || load_vec(st, q + "k.norm", c.dk, &L.knorm)) return 1;
                 if (st.find(q + "sink") && load_vec(st, q + "sink", c.H, &L.sink)) return 1;
                 if (dalloc(&L.kcache, (size_t)max_tokens * nk) || dalloc(&L.vcache, (size_t)max_tokens * nv)) return 1;
+                this->will_attend(c.G, c.dk, c.dv);
                 if (c.rot_dims > 0) {
                     std::vector<double> f;
                     for (int i = 0; i < c.rot_dims / 2; i++) f.push_back(pow(c.rot_base, -2.0 * (double)i / (double)c.rot_dims) / c.rot_factor);
@@ -244,7 +245,7 @@ template <typename AT, typename WT> class RupenexModel : public DenseModel<AT, W
         info.vocab = (uint32_t)vocab; info.width = (uint32_t)width; info.n_layers = (uint32_t)layers.size(); info.max_tokens = max_tokens;
         info.heads = (uint32_t)layers[0].c.H; info.kv_heads = (uint32_t)layers[0].c.G; info.head_dim = (uint32_t)(layers[0].c.kind == RP_ATTENTION ? layers[0].c.dk : layers[0].c.dv);
         info.ff = (uint32_t)layers[0].c.ff; info.dtype = opt.dtype; info.eps = eps;
-        return ensure_scratch(1);
+        return ensure_scratch(1) || this->reserve_split();
     }
 
     int ensure_scratch(size_t rows) override {

@@ -222,6 +222,7 @@ template <typename AT, typename WT> class TudatarModel : public LatentModel<AT, 
                     load_vec(st, q + "r2", c.H, &L.r2))
                     return 1;
                 if (dalloc(&L.kcache, (size_t)max_tokens * nk) || dalloc(&L.vcache, (size_t)max_tokens * nv)) return 1;
+                this->will_attend(c.G, c.dk, c.dv);
                 max_qa = std::max(max_qa, nq);
                 max_att = std::max(max_att, att_cols);
             } else if (c.kind == MIX_LATENT) {
@@ -276,7 +277,7 @@ template <typename AT, typename WT> class TudatarModel : public LatentModel<AT, 
         info.vocab = (uint32_t)vocab; info.width = (uint32_t)width; info.n_layers = (uint32_t)layers.size(); info.max_tokens = max_tokens;
         info.heads = (uint32_t)layers[0].c.H; info.kv_heads = (uint32_t)layers[0].c.G; info.head_dim = (uint32_t)layers[0].c.dk;
         info.ff = (uint32_t)layers[0].c.moe.ff; info.dtype = opt.dtype; info.eps = eps;
-        return ensure_scratch(1);
+        return ensure_scratch(1) || this->reserve_split();
     }
 
     int ensure_scratch(size_t rows) override {

@@ -7,6 +7,7 @@ import importlib
 
 import numpy as np
 import pytest
+import torch
 
 import genetar_oracle as G
 import rupenex_oracle as R
@@ -135,3 +136,26 @@ def test_rows_do_not_see_later_tokens_that_are_no_numbers(gpu_lib, tmp_path):
     assert G.rel_rms(got[:at], want) < 2e-4
     assert np.isnan(got[at:]).all()
     m.close()
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_the_first_prompt_finds_the_room_for_its_pieces(gpu_lib, tmp_path, dtype):
+    """the pieces of keys, values and (float32) rows are given room when the model is loaded: where everything else is allocated already, the first
+    prompt that takes the tensor-core kernels leaves the free memory as it is"""
+    n = 600
+    cfg = G.make_config([G.attention_layer("attention_2", heads=8, kv_heads=8, dim=64, vdim=64, ff=4096)], width=1024, vocab=64)
+    folder = G.write_model(str(tmp_path / "m"), cfg, G.random_weights(cfg, seed=1))
+    toks = np.random.default_rng(1).integers(0, 64, n).tolist()
+    loads_the_kernels = gpu_lib.Transformer.open(folder, dtype=dtype, max_tokens=n)
+    loads_the_kernels.forward_tokens(toks, 0, [n - 1])
+    m = gpu_lib.Transformer.open(folder, dtype=dtype, max_tokens=n)
+    for name, value in (("attn_tiles", 1), ("gemm_split", 0)):
+        m.set_option(name, value)
+    m.forward_tokens(toks, 0, [n - 1])
+    before = torch.cuda.mem_get_info()[0]
+    for name in ("attn_tiles", "gemm_split"):
+        m.set_option(name, -1)
+    assert np.array_equal(m.forward_tokens(toks, 0, [n - 1]), loads_the_kernels.forward_tokens(toks, 0, [n - 1]))
+    assert torch.cuda.mem_get_info()[0] == before
+    m.close()
+    loads_the_kernels.close()
