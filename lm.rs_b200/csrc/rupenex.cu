@@ -82,8 +82,7 @@ template <typename AT, typename WT> class RupenexModel : public DenseModel<AT, W
     unsigned int* ln_counter = nullptr;   // ticket counter of the one-row products that finish with the sublayer's norm
     int max_proj = 0, max_qa = 0, max_att = 0, max_ys = 0, max_H = 0, max_dv = 0, max_act = 0, max_top = 0, max_eff = 0, max_E = 0;
     bool any_shared = false;
-    int ssm_lanes = 0;   // test / measurement override of the scan's lanes per column (0: chosen by the state size)
-    int ssm_cols = 0;    // ... and of its columns per thread (0: chosen by the grid size)
+    int ssm_cols = 0;   // test / measurement override of the scan's columns per thread (0: chosen by the grid size)
 
     size_t n_layers() const override { return layers.size(); }
 
@@ -358,22 +357,17 @@ template <typename AT, typename WT> class RupenexModel : public DenseModel<AT, W
         // (rows per lane, lanes per column) with rows * lanes >= N.  1000 tokens of 64 heads of 64 x 128, one column per thread: 8 rows on 16 lanes
         // 243 us, 16 on 8 246, 32 on 4 240; what decides is how many columns share each read of a token's B and C entries (below): two 171 and
         // 214 (8 and 16 rows), four 166 (8 rows)
-        int lpc = ssm_lanes > 0 ? ssm_lanes : (c.N <= 16 ? 1 : c.N <= 32 ? 2 : c.N <= 64 ? 4 : c.N <= 256 ? 16 : 32);
-        while (lpc < 32 && 32 * lpc < c.N) lpc *= 2;
-        const int nr = 8 * lpc >= c.N ? 8 : (16 * lpc >= c.N ? 16 : 32);
+        const int lpc = c.N <= 16 ? 1 : c.N <= 32 ? 2 : c.N <= 64 ? 4 : c.N <= 256 ? 16 : 32;
+        const int nr = 8 * lpc >= c.N ? 8 : 16;
         int rc = 1;
-#define RP_SCAN(NR_, LPC_) if (nr == NR_ && lpc == LPC_) rc = launch_scan<NR_, LPC_, 1>(st, sp); else
-        // two or four columns per thread; taken when the grid still has a CTA for at least half of the SMs
-        const bool two_ok = (nr == 8 && (lpc == 8 || lpc == 16)) || (nr == 16 && lpc == 8), four_ok = nr == 8 && lpc == 16;
+#define RP_SCAN(NR_, LPC_, CPT_) if (nr == NR_ && lpc == LPC_ && cpt == CPT_) rc = launch_scan<NR_, LPC_, CPT_>(st, sp); else
+        // two or four columns per thread (states of 65 to 128 rows); taken when the grid still has a CTA for at least half of the SMs
         auto ctas = [&](int n) { const int cols = n * (DELTA_THREADS / lpc); return (c.dv + cols - 1) / cols * c.H; };
-        const int cpt = ssm_cols > 0 ? ssm_cols : four_ok && 2 * ctas(4) >= sms ? 4 : two_ok && 2 * ctas(2) >= sms ? 2 : 1;
-        if (cpt == 4 && four_ok) rc = launch_scan<8, 16, 4>(st, sp); else
-        if (cpt == 2 && nr == 8 && lpc == 16) rc = launch_scan<8, 16, 2>(st, sp);
-        else if (cpt == 2 && nr == 16 && lpc == 8) rc = launch_scan<16, 8, 2>(st, sp);
-        else if (cpt == 2 && nr == 8 && lpc == 8) rc = launch_scan<8, 8, 2>(st, sp);
-        else
-        RP_SCAN(8, 1) RP_SCAN(16, 1) RP_SCAN(8, 2) RP_SCAN(16, 2) RP_SCAN(32, 2) RP_SCAN(8, 4) RP_SCAN(16, 4) RP_SCAN(32, 4) RP_SCAN(8, 8) RP_SCAN(16, 8)
-        RP_SCAN(32, 8) RP_SCAN(8, 16) RP_SCAN(16, 16) RP_SCAN(32, 16) RP_SCAN(8, 32) RP_SCAN(16, 32) { error = "no scan kernel for state " + std::to_string(c.N); return 1; }
+        const int cpt = !(nr == 8 && lpc == 16) ? 1 : ssm_cols > 0 ? (ssm_cols >= 4 ? 4 : ssm_cols >= 2 ? 2 : 1) : 2 * ctas(4) >= sms ? 4 : 2 * ctas(2) >= sms ? 2 : 1;
+        RP_SCAN(8, 1, 1) RP_SCAN(16, 1, 1) RP_SCAN(16, 2, 1) RP_SCAN(16, 4, 1) RP_SCAN(8, 16, 1) RP_SCAN(8, 16, 2) RP_SCAN(8, 16, 4) RP_SCAN(16, 16, 1) RP_SCAN(16, 32, 1) {
+            error = "no scan kernel for state " + std::to_string(c.N);
+            return 1;
+        }
 #undef RP_SCAN
         if (rc) return 1;
         GatedGroupNormParams<AT> gp{};
@@ -467,7 +461,6 @@ template <typename AT, typename WT> class RupenexModel : public DenseModel<AT, W
     }
 
     void set_model_option(const char* name, int value) override {
-        if (!strcmp(name, "ssm_lanes")) { ssm_lanes = value; drop_graphs(); }
         if (!strcmp(name, "ssm_cols")) { ssm_cols = value; drop_graphs(); }
     }
     // test access: K and V rows of an attention layer; a state-space layer keeps a state, not rows per position
