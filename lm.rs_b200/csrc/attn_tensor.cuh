@@ -1,6 +1,7 @@
 // attn_tensor.cuh -- attention of many query rows (prompts and long portions) on the 5th-generation tensor cores with operands of full
 // f32 width: every f32 operand is split into three bf16 pieces whose sum is exact (8 + 8 + 8 significant bits), and a product is
-// the six piece products down to 2^-16 of it (what is left out is below 2^-23), each exact in the tensor cores' f32 accumulators.
+// the six piece products down to 2^-16 of it, each exact in the tensor cores' f32 accumulators.  What is left out, twice mid x lo, is at most 2^-22
+// of the product and of either sign (the same error against 64 bits as multiply-adds in f32, or less: figures at the kernels).
 // Same parameters and arithmetic rules as attn_tile_kernel and attn_rows_kernel (dense_ops.cuh).
 #pragma once
 #include "attn_tiles.cuh"
@@ -13,8 +14,8 @@ constexpr int AX_ROWS = 128, AX_KEYS = 128, AX_BOX = 16384, AX_RING = 8 * AX_BOX
 inline int attn_tensor_pad(int d) { return (d + 15) & ~15; }
 inline size_t attn_tensor_smem(int dk) { return 1024 + (size_t)3 * ((dk + 63) / 64) * AX_BOX + AX_RING + 256; }
 
-// x = hi + mid + lo exactly: hi the upper 16 bits (bf16 by truncation: no overflow), mid the rest rounded to bf16, lo what is left (at most 8
-// significant bits).  Two neighbouring elements at a time, packed as the operands hold them (the even one low).
+// x = hi + mid + lo: hi the upper 16 bits (bf16 by truncation: no overflow), mid the rest rounded to bf16 (at most 2^-7 of x), lo what is left (at most
+// 8 significant bits, 2^-16 of x).  Exact from 2^-110 on: of a smaller x the bits below 2^-133, the least a bf16 holds, are lost.  Two neighbouring elements at a time, packed as the operands hold them (the even one low).
 struct Split2 { uint32_t hi, mid, lo; };
 DN_DEVINL Split2 split_bf16x3(float a, float b) {
     const uint32_t ua = __float_as_uint(a) & 0xffff0000u, ub = __float_as_uint(b) & 0xffff0000u;

@@ -88,6 +88,7 @@ inline bool gemm_split_pays(bool glu, int T, int K, int O, int sms) {
 // gemm_form, constants (cycles) fitted to 21 products at 16 tilings each: a 32-wide piece of K takes 800 + 4 N, a CTA 14000 besides and 7000 more when it meets others.
 // us of the choice and of the next best tilings: 301 x 8192 gate/up, K 2048: 112 rows 150, 80 rows 171, 64 rows 197; 301 x 2048, K 8192: 80 rows and K in two 93,
 // 112 and two 106, 112 and four 113; 16 x 4096, K 2048: 16 and four 20, 32 and two 27, 16 37; 200 x 3072, K 3072: 80 and two 41, 112 and two 46, 48 58.
+// The parts of K, and below 512 of K the kernel, depend on the number of rows: the same row in another portion sums in another order.
 struct GemmSplitPlan { int N, splits; };
 inline GemmSplitPlan gemm_split_plan(bool glu, int T, int K, int O, int sms) {
     const long long m_tiles = glu ? (O + 63) / 64 : (O + 127) / 128;

@@ -1,7 +1,7 @@
 // dense_gemm_split.cuh -- many-row products of the float32 operand mode on the 5th-generation tensor cores:
 //     out[T][O] = A[T][K] . W[O][K]^T, all f32, then one of the epilogues of dense_ops.cuh
 // with operands of full f32 width: both are split into three bf16 pieces whose sum is exact (split_bf16x3, attn_tensor.cuh), and a product
-// is the six piece products down to 2^-16 of it, each exact in an f32 accumulator (what is left out is below 2^-23).
+// is the six piece products down to 2^-16 of it, each exact in an f32 accumulator (what is left out is at most 2^-22 of it).
 // Error against 64 bits (normal operands, 2-norm): 1.6e-7 at K 2048 and 2.7e-7 at K 8192, against 4.1e-7 and 8.1e-7 of the multiply-adds of
 // dense_gemm_f32.cuh, which the FMA pipe bounds: 301 x 8192 gate/up, K 2048 520 us there, 150 here (6 x 20.2 GFLOP of pieces: 74 us at the measured bf16
 // peak); 301 x 2048, K 8192 487 and 93; 16 x 4096, K 2048 72 and 20.  What bounds it now: the hand-over of each 32-wide piece of K from the

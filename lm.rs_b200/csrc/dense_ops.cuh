@@ -980,7 +980,7 @@ static __global__ void __launch_bounds__(128) qkv_post_kernel(const QkvPostParam
 // and j + 32 of the tile for each of its rows (K rows padded so that the 16-byte reads of 32 lanes do not collide), an
 // online softmax keeps (max, sum) per row, the probabilities go through shared memory and lane c accumulates output
 // columns c, c + 32, ... .  Tiles start at multiples of 64 keys whatever the portion, so within this kernel a row's arithmetic does
-// not depend on how the prompt was cut; portions that attn_large_tiles sends to attn_tile_kernel sum in another order.  With nsplit > 1 (decode) CTA `split` walks tiles split, split + nsplit, ... and writes
+// not depend on how the prompt was cut; portions that attn_tensor and attn_large_tiles send to the other kernels sum in another order.  With nsplit > 1 (decode) CTA `split` walks tiles split, split + nsplit, ... and writes
 // (max, sum, unnormalised row) to scratch for attn_combine_kernel.
 constexpr int ATT_KT = 64, ATT_WARPS = 4;
 // exp and tanh of the attention inner loop on the special-function unit: ex2.approx is good to about 2e-7 relative, and
