@@ -11,6 +11,7 @@ import torch
 
 import genetar_oracle as G
 import rupenex_oracle as R
+import tudatar_oracle as Tu
 
 pytestmark = pytest.mark.gpu
 
@@ -134,6 +135,32 @@ def test_rows_do_not_see_later_tokens_that_are_no_numbers(gpu_lib, tmp_path):
     toks[at] = 60
     got = m.forward_tokens(toks, 0, list(range(n)))
     assert G.rel_rms(got[:at], want) < 2e-4
+    assert np.isnan(got[at:]).all()
+    m.close()
+
+
+@pytest.mark.parametrize("form", ["kept keys and sinks", "kept keys up to the window", "penalty"])
+def test_windowed_rows_before_a_token_that_is_no_number(gpu_lib, tmp_path, form):
+    """the same for rows with a window, kept first keys, sinks that are on and off, a distance penalty: rows 256 .. 286 are computed again, over the keys they see"""
+    n, at = 320, 287
+    if form == "penalty":
+        O = Tu
+        cfg = Tu.make_config([Tu.window_layer(heads=8, kv_heads=2, dim=12, vdim=20, window=90, mlp=None)])
+    else:
+        O = R
+        cfg = R.make_config([R.attention_layer(heads=8, kv_heads=2, dim=12, vdim=20, size=90, keep_first=20 if form.endswith("sinks") else 250, mlp=None)])
+    W = O.random_weights(cfg, seed=6, gain=2.0)
+    if O is R:
+        W["l0.mix.sink"] = np.array([-np.inf, -3.3895313892515355e38, 0.0, 2.0, -1e30, -np.inf, 5.0, -40.0])
+    toks = np.random.default_rng(3).integers(0, 60, n).tolist()
+    want, _ = O.forward(cfg, W, toks[:at])
+    W["embed"][60] = np.nan
+    toks[at] = 60
+    m = gpu_lib.Transformer.open(O.write_model(str(tmp_path / "m"), cfg, W), dtype="float32", max_tokens=n)
+    m.set_option("attn_tiles", 2)
+    got = m.forward_tokens(toks, 0, list(range(n)))
+    assert O.rel_rms(got[:at], want) < 2e-4
+    assert O.rel_rms(got[256:at], want[256:]) < 2e-4
     assert np.isnan(got[at:]).all()
     m.close()
 
