@@ -205,6 +205,42 @@ DN_DEVINL float moe_combined(const MoeCombineParams& p, int t, int c, float ag =
     }
     return a;
 }
+// the sums of N columns c0, c0 + step, .. of one token: four experts' loads of all of them go out together, the additions are those of moe_combined
+template <int N> DN_DEVINL void moe_combined_cols(const MoeCombineParams& p, int t, int c0, int step, float ag, float (&a)[N]) {
+#pragma unroll
+    for (int i = 0; i < N; i++) { const int c = c0 + i * step; a[i] = p.add && c < p.width ? ag * p.add[(size_t)t * p.width + c] : 0.0f; }
+    for (int k0 = 0; k0 < p.top; k0 += 4) {
+        float w[4], v[4][N];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const size_t pair = (size_t)t * p.top + min(k0 + u, p.top - 1);
+            w[u] = p.wts[pair];
+            const float* row = p.idx && p.idx[pair] >= p.n_real ? p.xin + (size_t)t * p.ld_in : p.y + (p.slot ? (size_t)p.slot[pair] : pair) * p.width;
+#pragma unroll
+            for (int i = 0; i < N; i++) { const int c = c0 + i * step; v[u][i] = c < p.width ? row[c] : 0.0f; }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (k0 + u < p.top)
+#pragma unroll
+                for (int i = 0; i < N; i++) a[i] = fmaf(w[u], v[u][i], a[i]);
+    }
+}
+struct MoeCols {   // one token's sums as the source of a layer norm's row
+    const MoeCombineParams& p;
+    int t;
+    float ag;
+    DN_DEVINL float operator()(int c) const { return moe_combined(p, t, c, ag); }
+    DN_DEVINL void fill(float (&v)[LN_CACHE], int n) const {
+#pragma unroll
+        for (int i0 = 0; i0 < LN_CACHE; i0 += 4) {
+            float a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            if (i0 * (int)blockDim.x < n) moe_combined_cols<4>(p, t, threadIdx.x + i0 * blockDim.x, blockDim.x, ag, a);
+#pragma unroll
+            for (int i = 0; i < 4; i++) v[i0 + i] = a[i];
+        }
+    }
+};
 static __global__ void __launch_bounds__(256) moe_combine_kernel(const MoeCombineParams p) {
     pdl_launch();
     pdl_wait();
@@ -236,7 +272,7 @@ template <typename AT> __global__ void __launch_bounds__(256) moe_combine_layern
     float* xr = p.c.x + (size_t)t * p.c.ldx;
     const float ag = moe_add_gate(p.c, t);
     if (gridDim.y == 1) {
-        layernorm_row<AT>([&](int c) { return moe_combined(p.c, t, c, ag); }, p.c.width, p.w, p.eps, red, xr, p.ls, nullptr, p.h + (size_t)t * p.ldh);
+        layernorm_row<AT>(MoeCols{p.c, t, ag}, p.c.width, p.w, p.eps, red, xr, p.ls, nullptr, p.h + (size_t)t * p.ldh);
         return;
     }
     float* row = p.c.out + (size_t)t * p.c.ldo;
@@ -247,7 +283,7 @@ template <typename AT> __global__ void __launch_bounds__(256) moe_combine_layern
     __syncthreads();
     if (!last) return;
     __threadfence();
-    layernorm_row<AT>([&](int c) { return __ldcg(row + c); }, p.c.width, p.w, p.eps, red, xr, p.ls, nullptr, p.h + (size_t)t * p.ldh);
+    layernorm_row<AT>(L2Cols{row}, p.c.width, p.w, p.eps, red, xr, p.ls, nullptr, p.h + (size_t)t * p.ldh);
     if (threadIdx.x == 0) *p.counter = 0u;
 }
 
