@@ -1134,6 +1134,20 @@ static __global__ void __launch_bounds__(128) ssm_pre_kernel(const SsmPreParams 
     for (int j = 0; j < CONV_MAX_TAPS; j++) w[j] = j < p.taps ? p.wconv[(size_t)c * p.taps + j] : 0.0f;
     const float b = p.bconv ? p.bconv[c] : 0.0f;
     const float* in = p.in + p.c_off;
+    if (p.taps == 4) {   // the usual width: every input is loaded once, four tokens' loads ahead of their stores (1000 tokens of 6144 channels 36.8 us, 15.0 now)
+        float v[7];
+#pragma unroll
+        for (int i = 0; i < 3; i++) v[i] = conv_input(in, p.ld, p.tail, p.C, 4, t0 - 3 + i, c, pos0);
+        for (int t = t0; t < t1; t += 4) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) v[3 + i] = t + i < t1 ? in[(size_t)(t + i) * p.ld + c] : 0.0f;
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (t + i < t1) p.out[(size_t)(t + i) * p.C + c] = silu(fmaf(w[3], v[i + 3], fmaf(w[2], v[i + 2], fmaf(w[1], v[i + 1], fmaf(w[0], v[i], b)))));
+#pragma unroll
+            for (int i = 0; i < 3; i++) v[i] = v[i + 4];
+        }
+    } else
     for (int t = t0; t < t1; t++) {
         float a = b;
 #pragma unroll
@@ -1320,12 +1334,39 @@ template <typename AT> struct GatedGroupNormParams {
     const float* w; float eps;
     AT* out; int ldo;
     int n, groups;
+    int T;                   // > 0: the form of many tokens, a warp per (token, part), grid (T * groups / 8)
 };
+// Many tokens with short parts: a CTA per part had two columns per thread, three barriers and every value computed twice (1000 tokens of 8 parts of 512:
+// 23.6 us, 9.9 now)
+constexpr int GN_CACHE = 16;
+inline bool gated_groupnorm_by_warps(int T, int part) { return T > 1 && part <= 32 * GN_CACHE; }
 template <typename AT> __global__ void __launch_bounds__(256) gated_groupnorm_kernel(const GatedGroupNormParams<AT> p) {
     __shared__ float red[33];
     pdl_launch();
     pdl_wait();
-    const int t = blockIdx.x, gs = p.n / p.groups, c0 = blockIdx.y * gs;
+    const int gs = p.n / p.groups;
+    if (p.T > 0) {   // a warp per part: see gated_groupnorm_by_warps
+        const int lane = threadIdx.x & 31, part = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+        if (part >= p.T * p.groups) return;
+        const int tt = part / p.groups, at = part % p.groups * gs;
+        const float *yr = p.y + (size_t)tt * p.ldy + at, *zr = p.z + (size_t)tt * p.ldz + at;
+        float v[GN_CACHE], z[GN_CACHE], w[GN_CACHE], s = 0.0f;
+#pragma unroll
+        for (int i = 0; i < GN_CACHE; i++) {
+            const int c = lane + 32 * i;
+            v[i] = c < gs ? yr[c] : 0.0f;
+            z[i] = c < gs ? zr[c] : 0.0f;
+            w[i] = c < gs ? p.w[at + c] : 0.0f;
+        }
+#pragma unroll
+        for (int i = 0; i < GN_CACHE; i++) { v[i] *= silu(z[i]); s += v[i] * v[i]; }
+        const float f = 1.0f / sqrtf(warp_sum(s) / (float)gs + p.eps);
+        AT* o = p.out + (size_t)tt * p.ldo + at;
+#pragma unroll
+        for (int i = 0; i < GN_CACHE; i++) if (lane + 32 * i < gs) from_f(o[lane + 32 * i], v[i] * f * w[i]);
+        return;
+    }
+    const int t = blockIdx.x, c0 = blockIdx.y * gs;
     const float* y = p.y + (size_t)t * p.ldy + c0;
     const float* z = p.z + (size_t)t * p.ldz + c0;
     float ss = 0.0f;

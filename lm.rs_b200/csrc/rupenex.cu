@@ -372,7 +372,9 @@ template <typename AT, typename WT> class RupenexModel : public DenseModel<AT, W
         if (rc) return 1;
         GatedGroupNormParams<AT> gp{};
         gp.y = ys; gp.ldy = inner; gp.z = proj; gp.ldz = L.in_rows; gp.w = L.onorm; gp.eps = info.eps; gp.out = att; gp.ldo = inner; gp.n = inner; gp.groups = c.norm_groups;
-        if (launch_k("gated_groupnorm_kernel", st, pdl_now, gated_groupnorm_kernel<AT>, dim3(T, c.norm_groups), dim3(256), 0, gp)) return 1;
+        const bool warps = gated_groupnorm_by_warps(T, inner / c.norm_groups);
+        if (warps) gp.T = T;
+        if (launch_k("gated_groupnorm_kernel", st, pdl_now, gated_groupnorm_kernel<AT>, warps ? dim3((T * c.norm_groups + 7) / 8) : dim3(T, c.norm_groups), dim3(256), 0, gp)) return 1;
         return out_proj(st, T, att, inner, L.wo, L.norm1, L.ls1);
     }
 
@@ -387,6 +389,7 @@ template <typename AT, typename WT> class RupenexModel : public DenseModel<AT, W
         const RpLayerCfg& c = L.c;
         const int n_out = c.E + c.I;
         MoeRouterParams<AT> rp{};
+
         rp.h = h; rp.ld = width; rp.router = L.router; rp.correction = L.correction; rp.E = n_out; rp.top = c.top; rp.width = width; rp.softmax = 1;
         rp.scale = 1.0f; rp.z = rz; rp.idx = eidx; rp.wts = wts;
         if (launch_k("moe_logits_kernel", st, pdl_now, T == 1 ? moe_logits_kernel<AT, true> : moe_logits_kernel<AT, false>, moe_logits_grid(T, n_out), moe_logits_block(T), 0, rp)) return 1;

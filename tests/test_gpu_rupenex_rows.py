@@ -1,0 +1,32 @@
+"""Rows of Rupenex prompts at the edges of their kernels: group norms with parts a warp holds (up to 512 columns) and longer ones, convolutions of four taps
+(a sliding window) and of other widths over runs that end inside a block of four tokens, layer norms of rows a CTA holds in registers (up to 4096
+columns) and longer, and more chosen experts than are loaded at a time.  Against the float64 implementation, 2e-4 as in test_gpu_rupenex.py."""
+import numpy as np
+import pytest
+
+import rupenex_oracle as O
+
+pytestmark = pytest.mark.gpu
+TOL = 2e-4
+# heads, vdim, norm groups (part = heads * vdim / groups), taps, width, tokens
+CASES = [(8, 64, 1, 4, 40, 17), (8, 65, 1, 4, 40, 5), (8, 66, 2, 4, 260, 33), (4, 10, 2, 3, 41, 18), (4, 10, 4, 5, 256, 2), (4, 8, 1, 4, 4096, 3), (4, 8, 1, 2, 4100, 3)]
+
+
+@pytest.mark.parametrize("heads,vdim,groups,taps,width,n", CASES)
+def test_rows_at_the_edges(gpu_lib, tmp_path, heads, vdim, groups, taps, width, n):
+    moe = O.moe(experts=6, identity=2, top=5, ff=24, shared=24)
+    cfg = O.make_config([O.ssm_layer(heads=heads, vdim=vdim, state=12, groups=2, conv=taps, norm_groups=groups, mlp=moe)], width=width, vocab=50)
+    toks = np.random.default_rng(9).integers(0, 50, n).tolist()
+    for seed in range(3, 23):   # weights without a near-tie between experts
+        W = O.random_weights(cfg, seed=seed)
+        if O.clear_choices(cfg, W, toks, 1e-4):
+            break
+    want, _ = O.forward(cfg, W, toks)
+    m = gpu_lib.Transformer.open(O.write_model(str(tmp_path / "m"), cfg, W), dtype="float32", max_tokens=64)
+    got = m.forward_tokens(toks, 0, list(range(n)))
+    assert O.rel_rms(got, want) < TOL
+    if n > 2:   # in two portions: the convolution continues from its tail
+        cut = n // 2
+        parts = np.concatenate([m.forward_tokens(toks[:cut], 0, list(range(cut))), m.forward_tokens(toks[cut:], cut, list(range(n - cut)))])
+        assert O.rel_rms(parts, want) < TOL
+    m.close()
