@@ -106,5 +106,8 @@ inline GemmSplitPlan gemm_split_plan(bool glu, int T, int K, int O, int sms) {
     return best;
 }
 
+// Gated group norms of prompts (mixer_ops.cuh): a warp per (token, part of the row), or a CTA?  A warp holds up to 512 columns.
+inline bool group_norm_by_warps(int T, int part) { return T > 1 && part <= 512; }
+
 }  // namespace dense
 }  // namespace lmrs

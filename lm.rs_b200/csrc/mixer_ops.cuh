@@ -1327,7 +1327,7 @@ template <int NR, int LPC, int CPT> __global__ void __launch_bounds__(DELTA_THRE
 }
 
 // v = y * silu(z); the row is cut into `groups` equal parts, each divided by its own root mean square (eps inside the root),
-// then * w[column]: one CTA per (token, part)
+// then * w[column]: one CTA per (token, part), or a warp (group_norm_by_warps); the same bits either way
 template <typename AT> struct GatedGroupNormParams {
     const float* y; int ldy;
     const float* z; int ldz;
@@ -1336,21 +1336,37 @@ template <typename AT> struct GatedGroupNormParams {
     int n, groups;
     int T;                   // > 0: the form of many tokens, a warp per (token, part), grid (T * groups / 8)
 };
-// Many tokens with short parts: a CTA per part had two columns per thread, three barriers and every value computed twice (1000 tokens of 8 parts of 512:
-// 23.6 us, 9.9 now)
-constexpr int GN_CACHE = 16;
-inline bool gated_groupnorm_by_warps(int T, int part) { return T > 1 && part <= 32 * GN_CACHE; }
+constexpr int GN_CACHE = 16;   // columns a lane of the warp form holds
+// The sum that block_sum makes of 256 threads' values, to the bit, by one warp: v[w] is what thread 32 * w + lane of the block holds.  The eight warp sums are
+// made side by side (each step halves what a lane still carries: 12 shuffles), every addition with the operands it has there.
+DN_DEVINL float block_sum_of_8(float (&v)[8], int lane) {
+#pragma unroll
+    for (int half = 4; half > 0; half >>= 1) {   // lane bits 4, 3, 2 choose among the sums by bits 2, 1, 0 of their number
+        const bool up = lane & (half * 4);
+#pragma unroll
+        for (int w = 0; w < half; w++) {
+            const float other = __shfl_xor_sync(0xffffffffu, up ? v[w] : v[w + half], half * 4);
+            v[w] = (up ? v[w + half] : v[w]) + other;
+        }
+    }
+    float s = v[0];
+#pragma unroll
+    for (int o = 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+#pragma unroll
+    for (int o = 16; o >= 4; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);   // the eight sums, in block_sum's order
+    return s;
+}
 template <typename AT> __global__ void __launch_bounds__(256) gated_groupnorm_kernel(const GatedGroupNormParams<AT> p) {
     __shared__ float red[33];
     pdl_launch();
     pdl_wait();
     const int gs = p.n / p.groups;
-    if (p.T > 0) {   // a warp per part: see gated_groupnorm_by_warps
+    if (p.T > 0) {   // a warp per part: group_norm_by_warps
         const int lane = threadIdx.x & 31, part = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
         if (part >= p.T * p.groups) return;
         const int tt = part / p.groups, at = part % p.groups * gs;
         const float *yr = p.y + (size_t)tt * p.ldy + at, *zr = p.z + (size_t)tt * p.ldz + at;
-        float v[GN_CACHE], z[GN_CACHE], w[GN_CACHE], s = 0.0f;
+        float v[GN_CACHE], z[GN_CACHE], w[GN_CACHE], s[8];
 #pragma unroll
         for (int i = 0; i < GN_CACHE; i++) {
             const int c = lane + 32 * i;
@@ -1359,8 +1375,10 @@ template <typename AT> __global__ void __launch_bounds__(256) gated_groupnorm_ke
             w[i] = c < gs ? p.w[at + c] : 0.0f;
         }
 #pragma unroll
-        for (int i = 0; i < GN_CACHE; i++) { v[i] *= silu(z[i]); s += v[i] * v[i]; }
-        const float f = 1.0f / sqrtf(warp_sum(s) / (float)gs + p.eps);
+        for (int i = 0; i < GN_CACHE; i++) v[i] *= silu(z[i]);
+#pragma unroll
+        for (int i = 0; i < 8; i++) s[i] = fmaf(v[i + 8], v[i + 8], v[i] * v[i]);   // columns c and c + 256: a thread of the block form
+        const float f = 1.0f / sqrtf(block_sum_of_8(s, lane) / (float)gs + p.eps);
         AT* o = p.out + (size_t)tt * p.ldo + at;
 #pragma unroll
         for (int i = 0; i < GN_CACHE; i++) if (lane + 32 * i < gs) from_f(o[lane + 32 * i], v[i] * f * w[i]);

@@ -83,6 +83,7 @@ template <typename AT, typename WT> class RupenexModel : public DenseModel<AT, W
     int max_proj = 0, max_qa = 0, max_att = 0, max_ys = 0, max_H = 0, max_dv = 0, max_act = 0, max_top = 0, max_eff = 0, max_E = 0;
     bool any_shared = false;
     int ssm_cols = 0;   // test / measurement override of the scan's columns per thread (0: chosen by the grid size)
+    int group_norm_warps = 1;   // test / measurement override: 0 = a CTA per part of the group norm in prompts too
 
     size_t n_layers() const override { return layers.size(); }
 
@@ -372,7 +373,7 @@ template <typename AT, typename WT> class RupenexModel : public DenseModel<AT, W
         if (rc) return 1;
         GatedGroupNormParams<AT> gp{};
         gp.y = ys; gp.ldy = inner; gp.z = proj; gp.ldz = L.in_rows; gp.w = L.onorm; gp.eps = info.eps; gp.out = att; gp.ldo = inner; gp.n = inner; gp.groups = c.norm_groups;
-        const bool warps = gated_groupnorm_by_warps(T, inner / c.norm_groups);
+        const bool warps = group_norm_warps && group_norm_by_warps(T, inner / c.norm_groups);
         if (warps) gp.T = T;
         if (launch_k("gated_groupnorm_kernel", st, pdl_now, gated_groupnorm_kernel<AT>, warps ? dim3((T * c.norm_groups + 7) / 8) : dim3(T, c.norm_groups), dim3(256), 0, gp)) return 1;
         return out_proj(st, T, att, inner, L.wo, L.norm1, L.ls1);
@@ -465,6 +466,7 @@ template <typename AT, typename WT> class RupenexModel : public DenseModel<AT, W
 
     void set_model_option(const char* name, int value) override {
         if (!strcmp(name, "ssm_cols")) { ssm_cols = value; drop_graphs(); }
+        else if (!strcmp(name, "group_norm_warps")) group_norm_warps = value;
     }
     // test access: K and V rows of an attention layer; a state-space layer keeps a state, not rows per position
     int read_kv(cudaStream_t st, uint32_t layer, uint32_t pos0, uint32_t n, float* k_out, float* v_out) override {

@@ -30,3 +30,18 @@ def test_rows_at_the_edges(gpu_lib, tmp_path, heads, vdim, groups, taps, width, 
         parts = np.concatenate([m.forward_tokens(toks[:cut], 0, list(range(cut))), m.forward_tokens(toks[cut:], cut, list(range(n - cut)))])
         assert O.rel_rms(parts, want) < TOL
     m.close()
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("heads,vdim,groups,n", [(8, 64, 1, 17), (8, 64, 2, 2), (3, 171, 1, 9), (8, 65, 1, 5), (4, 10, 4, 33), (5, 1, 5, 3)])
+def test_group_norm_sums_in_one_order(gpu_lib, tmp_path, dtype, heads, vdim, groups, n):
+    """a warp per part or a CTA per part: the same bits"""
+    cfg = O.make_config([O.ssm_layer(heads=heads, vdim=vdim, state=8, groups=1, norm_groups=groups, mlp=None)], width=40, vocab=50)
+    toks = np.random.default_rng(4).integers(0, 50, n).tolist()
+    m = gpu_lib.Transformer.open(O.write_model(str(tmp_path / "m"), cfg, O.random_weights(cfg, seed=6)), dtype=dtype, max_tokens=64)
+    got = []
+    for warps in (1, 0):
+        m.set_option("group_norm_warps", warps)
+        got.append(m.forward_tokens(toks, 0, list(range(n))))
+    assert np.array_equal(*got)
+    m.close()
