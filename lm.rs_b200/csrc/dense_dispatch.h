@@ -106,8 +106,11 @@ inline GemmSplitPlan gemm_split_plan(bool glu, int T, int K, int O, int sms) {
     return best;
 }
 
-// Gated group norms of prompts (mixer_ops.cuh): a warp per (token, part of the row), or a CTA?  A warp holds up to 512 columns.
-inline bool group_norm_by_warps(int T, int part) { return T > 1 && part <= 512; }
+// Gated group norms (mixer_ops.cuh): a CTA per (token, part of the row), or a warp, which holds up to 512 columns?  Both make the same bits.  A warp has 16 columns a
+// lane to get through whatever the part's length, so a launch takes 4.2 us at least, a CTA 2.0; what it saves, barriers and values computed twice, counts once
+// the SMs are full.  us, CTA | warp: 1 token of 8 parts of 512 2.8 | 4.7, 16 tokens 3.0 | 4.8, 96 tokens 4.9 | 4.9, 256 tokens 9.1 | 5.8, 1000 tokens 29.8 | 13.4;
+// 1000 tokens of 1 part of 512 5.3 | 4.8, of 8 of 128 15.4 | 12.7, of 32 of 32 45.6 | 44.3; 512 tokens of 2 parts of 256 3.9 | 4.7; 192 tokens of 8 parts of 257 6.0 | 5.5.
+inline bool group_norm_by_warps(int T, int groups, int part) { return part <= 512 && (long long)T * groups * part >= 400000; }
 
 }  // namespace dense
 }  // namespace lmrs

@@ -1327,16 +1327,27 @@ template <int NR, int LPC, int CPT> __global__ void __launch_bounds__(DELTA_THRE
 }
 
 // v = y * silu(z); the row is cut into `groups` equal parts, each divided by its own root mean square (eps inside the root),
-// then * w[column]: one CTA per (token, part), or a warp (group_norm_by_warps); the same bits either way
+// then * w[column].  One CTA per (token, part); prompts with many short parts take the next kernel, which makes the same bits (group_norm_by_warps).
 template <typename AT> struct GatedGroupNormParams {
     const float* y; int ldy;
     const float* z; int ldz;
     const float* w; float eps;
     AT* out; int ldo;
-    int n, groups;
-    int T;                   // > 0: the form of many tokens, a warp per (token, part), grid (T * groups / 8)
+    int T, n, groups;
 };
-constexpr int GN_CACHE = 16;   // columns a lane of the warp form holds
+template <typename AT> __global__ void __launch_bounds__(256) gated_groupnorm_kernel(const GatedGroupNormParams<AT> p) {
+    __shared__ float red[33];
+    pdl_launch();
+    pdl_wait();
+    const int t = blockIdx.x, gs = p.n / p.groups, c0 = blockIdx.y * gs;
+    const float* y = p.y + (size_t)t * p.ldy + c0;
+    const float* z = p.z + (size_t)t * p.ldz + c0;
+    float ss = 0.0f;
+    for (int c = threadIdx.x; c < gs; c += blockDim.x) { const float v = y[c] * silu(z[c]); ss += v * v; }
+    ss = block_sum(ss, red);
+    const float inv = 1.0f / sqrtf(ss / (float)gs + p.eps);
+    for (int c = threadIdx.x; c < gs; c += blockDim.x) from_f(p.out[(size_t)t * p.ldo + c0 + c], y[c] * silu(z[c]) * inv * p.w[c0 + c]);
+}
 // The sum that block_sum makes of 256 threads' values, to the bit, by one warp: v[w] is what thread 32 * w + lane of the block holds.  The eight warp sums are
 // made side by side (each step halves what a lane still carries: 12 shuffles), every addition with the operands it has there.
 DN_DEVINL float block_sum_of_8(float (&v)[8], int lane) {
@@ -1356,42 +1367,33 @@ DN_DEVINL float block_sum_of_8(float (&v)[8], int lane) {
     for (int o = 16; o >= 4; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);   // the eight sums, in block_sum's order
     return s;
 }
-template <typename AT> __global__ void __launch_bounds__(256) gated_groupnorm_kernel(const GatedGroupNormParams<AT> p) {
-    __shared__ float red[33];
+// A warp per (token, part), grid (T * groups / 8), parts of up to 512 columns, held in registers: the kernel above has at most two columns per thread there,
+// three barriers, and computes every value twice.
+constexpr int GN_CACHE = 16;
+template <typename AT> __global__ void __launch_bounds__(256) gated_groupnorm_warps_kernel(const GatedGroupNormParams<AT> p) {
     pdl_launch();
     pdl_wait();
-    const int gs = p.n / p.groups;
-    if (p.T > 0) {   // a warp per part: group_norm_by_warps
-        const int lane = threadIdx.x & 31, part = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-        if (part >= p.T * p.groups) return;
-        const int tt = part / p.groups, at = part % p.groups * gs;
-        const float *yr = p.y + (size_t)tt * p.ldy + at, *zr = p.z + (size_t)tt * p.ldz + at;
-        float v[GN_CACHE], z[GN_CACHE], w[GN_CACHE], s[8];
+    const int gs = p.n / p.groups, lane = threadIdx.x & 31, part = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (part >= p.T * p.groups) return;
+    const int t = part / p.groups, c0 = part % p.groups * gs;
+    const float *y = p.y + (size_t)t * p.ldy + c0, *z = p.z + (size_t)t * p.ldz + c0;
+    float v[GN_CACHE], g[GN_CACHE], w[GN_CACHE], s[8];
 #pragma unroll
-        for (int i = 0; i < GN_CACHE; i++) {
-            const int c = lane + 32 * i;
-            v[i] = c < gs ? yr[c] : 0.0f;
-            z[i] = c < gs ? zr[c] : 0.0f;
-            w[i] = c < gs ? p.w[at + c] : 0.0f;
-        }
-#pragma unroll
-        for (int i = 0; i < GN_CACHE; i++) v[i] *= silu(z[i]);
-#pragma unroll
-        for (int i = 0; i < 8; i++) s[i] = fmaf(v[i + 8], v[i + 8], v[i] * v[i]);   // columns c and c + 256: a thread of the block form
-        const float f = 1.0f / sqrtf(block_sum_of_8(s, lane) / (float)gs + p.eps);
-        AT* o = p.out + (size_t)tt * p.ldo + at;
-#pragma unroll
-        for (int i = 0; i < GN_CACHE; i++) if (lane + 32 * i < gs) from_f(o[lane + 32 * i], v[i] * f * w[i]);
-        return;
+    for (int i = 0; i < GN_CACHE; i++) {
+        const int c = lane + 32 * i;
+        v[i] = c < gs ? y[c] : 0.0f;
+        g[i] = c < gs ? z[c] : 0.0f;
+        w[i] = c < gs ? p.w[c0 + c] : 0.0f;
     }
-    const int t = blockIdx.x, c0 = blockIdx.y * gs;
-    const float* y = p.y + (size_t)t * p.ldy + c0;
-    const float* z = p.z + (size_t)t * p.ldz + c0;
-    float ss = 0.0f;
-    for (int c = threadIdx.x; c < gs; c += blockDim.x) { const float v = y[c] * silu(z[c]); ss += v * v; }
-    ss = block_sum(ss, red);
-    const float inv = 1.0f / sqrtf(ss / (float)gs + p.eps);
-    for (int c = threadIdx.x; c < gs; c += blockDim.x) from_f(p.out[(size_t)t * p.ldo + c0 + c], y[c] * silu(z[c]) * inv * p.w[c0 + c]);
+#pragma unroll
+    for (int i = 0; i < GN_CACHE; i++) v[i] *= silu(g[i]);
+#pragma unroll
+    for (int i = 0; i < 8; i++) s[i] = fmaf(v[i + 8], v[i + 8], v[i] * v[i]);   // columns c and c + 256: a thread of the kernel above
+    const float inv = 1.0f / sqrtf(block_sum_of_8(s, lane) / (float)gs + p.eps);
+    AT* o = p.out + (size_t)t * p.ldo + c0;
+#pragma unroll
+    for (int i = 0; i < GN_CACHE; i++)
+        if (lane + 32 * i < gs) from_f(o[lane + 32 * i], v[i] * inv * w[i]);
 }
 
 }  // namespace dense

@@ -83,7 +83,7 @@ template <typename AT, typename WT> class RupenexModel : public DenseModel<AT, W
     int max_proj = 0, max_qa = 0, max_att = 0, max_ys = 0, max_H = 0, max_dv = 0, max_act = 0, max_top = 0, max_eff = 0, max_E = 0;
     bool any_shared = false;
     int ssm_cols = 0;   // test / measurement override of the scan's columns per thread (0: chosen by the grid size)
-    int group_norm_warps = 1;   // test / measurement override: 0 = a CTA per part of the group norm in prompts too
+    int group_norm_warps = -1;   // test / measurement override: 1 / 0 = a warp / a CTA per part of the group norm, -1 = by size
 
     size_t n_layers() const override { return layers.size(); }
 
@@ -373,9 +373,10 @@ template <typename AT, typename WT> class RupenexModel : public DenseModel<AT, W
         if (rc) return 1;
         GatedGroupNormParams<AT> gp{};
         gp.y = ys; gp.ldy = inner; gp.z = proj; gp.ldz = L.in_rows; gp.w = L.onorm; gp.eps = info.eps; gp.out = att; gp.ldo = inner; gp.n = inner; gp.groups = c.norm_groups;
-        const bool warps = group_norm_warps && group_norm_by_warps(T, inner / c.norm_groups);
-        if (warps) gp.T = T;
-        if (launch_k("gated_groupnorm_kernel", st, pdl_now, gated_groupnorm_kernel<AT>, warps ? dim3((T * c.norm_groups + 7) / 8) : dim3(T, c.norm_groups), dim3(256), 0, gp)) return 1;
+        gp.T = T;
+        const bool warps = group_norm_warps >= 0 ? group_norm_warps && inner / c.norm_groups <= 32 * GN_CACHE : group_norm_by_warps(T, c.norm_groups, inner / c.norm_groups);
+        if (warps ? launch_k("gated_groupnorm_warps_kernel", st, pdl_now, gated_groupnorm_warps_kernel<AT>, dim3((T * c.norm_groups + 7) / 8), dim3(256), 0, gp)
+                  : launch_k("gated_groupnorm_kernel", st, pdl_now, gated_groupnorm_kernel<AT>, dim3(T, c.norm_groups), dim3(256), 0, gp)) return 1;
         return out_proj(st, T, att, inner, L.wo, L.norm1, L.ls1);
     }
 
@@ -390,7 +391,6 @@ template <typename AT, typename WT> class RupenexModel : public DenseModel<AT, W
         const RpLayerCfg& c = L.c;
         const int n_out = c.E + c.I;
         MoeRouterParams<AT> rp{};
-
         rp.h = h; rp.ld = width; rp.router = L.router; rp.correction = L.correction; rp.E = n_out; rp.top = c.top; rp.width = width; rp.softmax = 1;
         rp.scale = 1.0f; rp.z = rz; rp.idx = eidx; rp.wts = wts;
         if (launch_k("moe_logits_kernel", st, pdl_now, T == 1 ? moe_logits_kernel<AT, true> : moe_logits_kernel<AT, false>, moe_logits_grid(T, n_out), moe_logits_block(T), 0, rp)) return 1;
