@@ -91,7 +91,7 @@ int lmrs_b200_forward_tokens(lmrs_b200_t* m, const uint32_t* tokens, size_t n, u
  * portion; "tensor_cores" 0 = many-row products on the CUDA-core kernel even where the tcgen05 kernel applies; "graphs" 0 =
  * decode steps as plain launches instead of CUDA graph replays; "pdl" 1 = decode kernels chained with programmatic
  * dependent launch (on for Genetar, off for the others: where each measures faster), 0 = without; "prompt_pdl" the same for the kernels of
- * a prompt portion (on for Genetar and Tudatar); "mlp_beside" 0 = a Genetar step's feed-forward after its attention instead of beside it; "attn_tiles" 2 / 1 / 0 =
+ * a prompt portion (on for Genetar; without effect for the others, whose prompts are never chained); "mlp_beside" 0 = a Genetar step's feed-forward after its attention instead of beside it; "attn_tiles" 2 / 1 / 0 =
  * attention of several rows on the tensor cores / in 64-row tiles wherever they can run / neither, -1 = by size; "gemm_split" 1 / 0 =
  * float32 products of several rows on the tensor cores wherever they can run / nowhere, -1 = by size; "gemm_form" -1 / 0 / 1 / 2 = tcgen05
  * products of more than 128 rows on one SM per tile / two SMs and 256 columns / 128 columns / 128 columns and K in halves, -2 = by size */

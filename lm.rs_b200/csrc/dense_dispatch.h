@@ -106,6 +106,12 @@ inline GemmSplitPlan gemm_split_plan(bool glu, int T, int K, int O, int sms) {
     return best;
 }
 
+// Are a prompt portion's kernels chained with programmatic dependent launches?  Only where the architecture vouches for its chain (Genetar).  With routed experts
+// they never are: a prompt chained through the grouped product, the experts' sum and the norm behind it into a two-SM product failed to end once in some hundred
+// passes when those row kernels were made faster, for a reason that was not found; the chain as it stood differed from that one in nothing but its timing.  Unchained,
+// 512 tokens of 3 Tudatar layers take 1144 us, chained they took 1060.
+inline bool prompt_chained(int option, int T, bool vouched) { return option != 0 && T > 1 && vouched; }
+
 // Gated group norms (mixer_ops.cuh): a CTA per (token, part of the row), or a warp, which holds up to 512 columns?  Both make the same bits.  A warp has 16 columns a
 // lane to get through whatever the part's length, so a launch takes 4.2 us at least, a CTA 2.0; what it saves, barriers and values computed twice, counts once
 // the SMs are full.  us, CTA | warp: 1 token of 8 parts of 512 2.8 | 4.7, 16 tokens 3.0 | 4.8, 96 tokens 4.9 | 4.9, 256 tokens 9.1 | 5.8, 1000 tokens 29.8 | 13.4;

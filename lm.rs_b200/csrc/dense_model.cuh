@@ -78,9 +78,10 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
     // programmatic dependent launch of the decode chain is an option.  An architecture turns it on where it measures faster (Genetar);
     // chains of many small kernels lose a little (Tudatar, 16 steps of 3 layers: 2.96 -> 3.03 ms)
     int use_graph = 1, use_pdl = 0;
-    // ... and of a prompt portion's.  Most of its kernels are short (512 tokens, 3 layers: 25 of them in 600 us), and the next one's launch, barriers and TMEM
-    // are ready when one ends: 512 tokens, Llama-3.2-1B shapes, Genetar 600 -> 524 us, Tudatar 1125 -> 1037, 2048 tokens of 3B shapes 1602 -> 1584.  Rupenex loses (1084 -> 1105).
+    // ... and of a prompt portion's, where the architecture vouches for it (prompt_chained).  Most of its kernels are short (512 tokens, 3 layers: 25 of them in 600 us),
+    // and the next one's launch, barriers and TMEM are ready when one ends: 512 tokens, Llama-3.2-1B shapes, Genetar 600 -> 524 us, 2048 tokens of 3B shapes 1602 -> 1584.
     int prompt_pdl = 0;
+    bool prompt_chain_ok = false;
     int attn_tiles = -1;   // option: 2 / 1 the tensor-core / the register-tiled attention wherever it can run, 0 neither, -1 by attn_tensor and attn_large_tiles
     int gemm_split = -1;   // option: 1 / 0 float32 products on the tensor cores wherever they can run / nowhere, -1 by gemm_split_pays
     uint16_t* split_planes = nullptr;   // pieces of the running call's f32 operands (attn_tensor.cuh)
@@ -653,7 +654,7 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
                 GCK(cudaMemcpyAsync(d_rows, rows.data(), (size_t)m * 4, cudaMemcpyHostToDevice, st));
                 GCK(cudaStreamSynchronize(st));   // `rows` is a local
             }
-            const Chained chained(*this, T > 1 && prompt_pdl);   // (for this portion's layers and head)
+            const Chained chained(*this, prompt_chained(prompt_pdl, T, prompt_chain_ok));   // (for this portion's layers and head)
             if (run_layers(st, T, ps, pos + (uint32_t)c0)) return 1;
             if (m == 0) continue;
             if (T == 1) {

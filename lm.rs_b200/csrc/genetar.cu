@@ -137,6 +137,7 @@ template <typename AT, typename WT> class GenetarModel : public DenseModel<AT, W
         sms = opt.sms;
         gemm_ctx.sms = opt.sms;
         B::prompt_pdl = 1;
+        B::prompt_chain_ok = true;
         B::use_pdl = 1;   // its decode chain is mostly one-row products that have their first weights in flight while they wait: 370 -> 346 us
                           // per step (6 layers at width 2048, waited for on the host), 96 -> 85 (3 layers at width 256)
         width = (int)cfg.at("width").number(0);

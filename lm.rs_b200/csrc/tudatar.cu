@@ -189,7 +189,6 @@ template <typename AT, typename WT> class TudatarModel : public LatentModel<AT, 
         return 0;
     }
     int load(const std::string& dir, const Json& cfg, const ArchOptions& opt) {
-        B::prompt_pdl = 1;
         sms = opt.sms;
         B::gemm_ctx.sms = opt.sms;
         width = (int)cfg.at("width").number(0);

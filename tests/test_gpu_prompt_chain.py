@@ -1,5 +1,6 @@
 """Prompt portions with their kernels chained by programmatic dependent launch (option "prompt_pdl") and without: the same
-logits to the bit, whole and in portions, for every folder architecture, in both number formats."""
+logits to the bit, whole and in portions, for every folder architecture, in both number formats.  Only Genetar's are chained; for
+the others the option has no effect, and this holds them to giving the same bits pass after pass."""
 import importlib
 
 import numpy as np
