@@ -76,8 +76,8 @@ struct AttnSplitParams {
 };
 static __global__ void __launch_bounds__(256) attn_split_kernel(const AttnSplitParams p) {
     __shared__ float tile[64][65];
-    pdl_launch();
     pdl_wait();
+    pdl_launch();
     const int u = blockIdx.x >> 1, g = blockIdx.y, part = blockIdx.z;
     const int key0 = (u < p.kf ? u : p.first + u - p.kf) * AX_KEYS + (blockIdx.x & 1) * 64;
     float v[8];

@@ -102,8 +102,8 @@ static __global__ void __launch_bounds__(128 * KH, 2) attn_tile_kernel(const Att
         const int j0 = tile * TA_KEYS;
         copy_rows(Vs, VS, 0, p.dv, p.vcache + (size_t)j0 * p.v_ld + (size_t)g * p.dv, p.v_ld, n_keys - j0);
     };
-    pdl_launch();
     pdl_wait();
+    pdl_launch();
     for (int e = threadIdx.x; e < TA_ROWS * (d4 >> 2); e += TA_THREADS) {
         const int r = e / (d4 >> 2), c = e - r * (d4 >> 2);
         const int t = t0 + r / p.HC, hl = h0 + r % p.HC;

@@ -31,8 +31,8 @@ static __global__ void __launch_bounds__(FG_THREADS, 2) gemm_f32_kernel(const Ge
     constexpr int OUT_COLS = GLU ? FG_N / 2 : FG_N, HALF = FG_K / 2;
     constexpr int GROUP = (FG_M + FG_N) * HALF, STAGE = 2 * GROUP;   // floats: [group][A rows | W rows][HALF]
     extern __shared__ __align__(128) float fg_sm[];
-    pdl_launch();
     pdl_wait();
+    pdl_launch();
     GemmTiledParams<float, float> p = pp;
     int row0 = 0;
     if (gridDim.z > 1 || p.grp) {   // as in gemm_tiled_kernel

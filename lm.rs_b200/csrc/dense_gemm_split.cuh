@@ -16,8 +16,8 @@ namespace dense {
 // The rows of A, split once per product: [plane][T][kp], kp = K padded to 8, zeros in the padding
 struct SplitRowsParams { const float* a; int lda, T, K, kp; uint16_t* out; };
 static __global__ void __launch_bounds__(256) split_rows_kernel(const SplitRowsParams p) {
-    pdl_launch();
     pdl_wait();
+    pdl_launch();
     const int pieces = p.kp >> 3;
     const size_t plane = (size_t)p.T * p.kp;
     for (long long e = (long long)blockIdx.x * 256 + threadIdx.x; e < (long long)p.T * pieces; e += (long long)gridDim.x * 256) {
