@@ -477,6 +477,11 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_con
         }
         cluster_sync();   // the sums have arrived
     }
+    // The commits that free the last stages arrive in both CTAs, and nobody else waits for them: none may be on its way to a CTA that has left, where the
+    // successor's barriers would lie.  A lane per stage, beside the epilogue: 0.2 us per product (one lane for all stages, ahead of the split form's
+    // meeting or behind the epilogue: 0.6 and 1.4).
+    if (warp == 0 && mbar_wait_bounded(tfull, 0, abort_flag) && lane < min(p.stages, g1 - g0))
+        mbar_wait_bounded(&empty[lane], ((g1 - g0 - 1 - lane) / p.stages) & 1, abort_flag);
     if (warp >= 2 && ok && m0 < p.T) {   // ---- epilogue: as in the kernel above, 32 x 32 blocks through the idle ring ----
         float* stg = reinterpret_cast<float*>(tiles) + (size_t)(warp - 2) * 32 * 33;
 #pragma unroll 1
