@@ -215,7 +215,7 @@ attn_tensor_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
             bool ok = true;
             auto fetch = [&](const CUtensorMap* map, int x, int dx, int y, int boxes, uint32_t bytes) {
                 const uint32_t s = n & (slots - 1);
-                ok = mbar_wait_bounded(&empty[s], ((n >> slots_log) & 1) ^ 1, abort_flag);
+                ok = mbar_wait_bounded(&empty[s], ((n >> slots_log) & 1) ^ 1, abort_flag, TG_ATTENTION + TG_FREE);
                 if (!ok) return;
                 mbar_expect_tx(&full[s], boxes * bytes);
                 for (int c = 0; c < boxes; c++) tg_tma_load_2d(ring + (s << slot_log) + c * bytes, map, x + c * dx, y, &full[s]);
@@ -235,16 +235,16 @@ attn_tensor_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
             }
             if (*abort_flag) {   // gave up somewhere: let the copies already requested land before shared memory goes away
                 for (uint32_t i = n > slots ? n - slots : 0; i < n; i++)
-                    for (uint32_t w = 0; w < TG_SPIN_LIMIT && !mbar_try_wait(&full[i & (slots - 1)], (i >> slots_log) & 1); w++) {}
+                    mbar_wait_for(&full[i & (slots - 1)], (i >> slots_log) & 1, nullptr);
             }
         } else if (warp == 9) {   // ---- MMA issuer ----
             const uint32_t one = elect_one();
             uint32_t n = 0;   // pieces used
-            bool ok = mbar_wait_bounded(q_ready, 0, abort_flag);
+            bool ok = mbar_wait_bounded(q_ready, 0, abort_flag, TG_ATTENTION + TG_QUERIES);
             // low words of the operand descriptors
             const uint32_t q_lo = (uint32_t)tg_desc_sw128(Qs), ring_lo = (uint32_t)tg_desc_sw128(ring);
             auto ready = [&](uint32_t b) {   // piece b has landed
-                ok = ok && mbar_wait_bounded(&full[b & (slots - 1)], (b >> slots_log) & 1, abort_flag);
+                ok = ok && mbar_wait_bounded(&full[b & (slots - 1)], (b >> slots_log) & 1, abort_flag, TG_ATTENTION + TG_FULL);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 return ok;
             };
@@ -299,8 +299,8 @@ attn_tensor_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
             if (ok) scores(0);
             if (ok && n_walk > 1) scores(1);
             for (int u = 0; u < n_walk && ok; u++) {
-                ok = mbar_wait_bounded(&p_ready[u & 1], (u >> 1) & 1, abort_flag);
-                if (NV > 1 && u > 0) ok = ok && mbar_wait_bounded(pv_free, (u - 1) & 1, abort_flag);
+                ok = mbar_wait_bounded(&p_ready[u & 1], (u >> 1) & 1, abort_flag, TG_ATTENTION + TG_WEIGHTS);
+                if (NV > 1 && u > 0) ok = ok && mbar_wait_bounded(pv_free, (u - 1) & 1, abort_flag, TG_ATTENTION + TG_VALUES_READ);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 if (ok) values(u);
                 if (ok && u + 2 < n_walk) scores(u + 2);
@@ -353,7 +353,7 @@ attn_tensor_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
                 const int b = j0 + 32 * c;
                 return whole ? 0xffffffffu : (bits_from(from - b) | (keep ? bits_to(keep - 1 - b) : 0u)) & (last >= b ? bits_to(last - b) : 0u);
             };
-            ok = mbar_wait_bounded(&s_done[grp], (u >> 1) & 1, abort_flag);
+            ok = mbar_wait_bounded(&s_done[grp], (u >> 1) & 1, abort_flag, TG_ATTENTION + TG_SCORES);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             uint32_t v[32];
@@ -421,7 +421,7 @@ attn_tensor_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
             mbar_arrive(&p_ready[grp]);
             l = l * corr + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
             // ---- the tile's weighted values
-            ok = mbar_wait_bounded(&pv_done[grp], (u >> 1) & 1, abort_flag);
+            ok = mbar_wait_bounded(&pv_done[grp], (u >> 1) & 1, abort_flag, TG_ATTENTION + TG_VALUES);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
@@ -498,7 +498,7 @@ attn_tensor_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(512) : "memory");
     }
-    if (threadIdx.x == 0 && *abort_flag && err) *err = 1;
+    if (threadIdx.x == 0 && *abort_flag && err) *err = *abort_flag;
 }
 
 }  // namespace dense

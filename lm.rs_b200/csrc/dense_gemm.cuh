@@ -11,8 +11,10 @@
 // masks its stores.  What the shape must satisfy: K and lda multiples of 8 elements (16-byte row pitch) and 16-byte
 // aligned bases.  Three stages of 32 KB leave room for two CTAs per SM: one tile's epilogue runs under the other's MMAs.
 // Prompts of more than 128 rows may run on a two-SM form of the same kernel, further down (gemm_form).
-// Every wait is bounded: a wait that runs out raises a flag in mapped host memory, the roles stop, in-flight copies are
-// waited for (bounded again), TMEM is freed and the kernel returns; the next launch reports the flag.
+// Every wait on an mbarrier is bounded in time: one that runs out (TG_WAIT_NS) writes which kernel and which barrier it was to a word in mapped host memory, the
+// roles stop, in-flight copies are waited for (bounded again), TMEM is freed and the kernel returns; the next launch reports the word.  Not bounded are the waits
+// that have no limit to give: tcgen05.alloc (every kernel here frees its columns, and all that can lie on an SM at once fit its 512), the cluster barriers
+// (every thread of every CTA comes to each of them, after a give-up too) and griddepcontrol.wait (for the end of the kernel before).
 #pragma once
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -33,24 +35,46 @@ constexpr int TG_M = 128, TG_N = 128, TG_KB = 128 /* bytes of K per stage */, TG
 constexpr int TG_A_BYTES = TG_M * TG_KB, TG_B_BYTES = TG_N * TG_KB, TG_STAGE_BYTES = TG_A_BYTES + TG_B_BYTES;
 constexpr int TG_THREADS = 64 + 128;
 constexpr size_t TG_SMEM = 1024 + (size_t)TG_STAGES * TG_STAGE_BYTES + 256;
-constexpr uint32_t TG_SPIN_LIMIT = 1u << 24;   // try_wait calls (each suspends for a while) before a wait gives up
+constexpr uint32_t TG_WAIT_NS = 2000000000u;   // how long a wait may take ...
+constexpr uint32_t TG_LEAST_TRIES = 4096;      // ... after it has looked this often (a context that was switched out for a while may not have)
+// what a wait was for, in the status word: kernel * 256 + barrier
+enum { TG_ONE_CTA = 1 << 8, TG_PAIR = 2 << 8, TG_ATTENTION = 3 << 8, TG_F32 = 4 << 8,
+       TG_FREE = 1, TG_FULL, TG_SUMS, TG_SUMS_READ, TG_ROWS_FREE, TG_ROWS_FULL, TG_SPLIT_FREE, TG_SPLIT_FULL, TG_QUERIES, TG_SCORES, TG_WEIGHTS, TG_VALUES, TG_VALUES_READ };
+inline std::string tg_gave_up(int status) {
+    static const char* kernels[] = {"a tensor-core kernel", "gemm_bf16_tc_kernel", "gemm_bf16_pair_kernel", "attn_tensor_kernel", "gemm_split_kernel"};
+    static const char* waits[] = {"one of its barriers", "a free stage", "a stage's copies", "the sums", "its sums to be read", "a free stage of rows", "a stage of rows",
+                                  "room for split weights", "split weights", "the split queries", "scores", "softmax weights", "weighted values", "weighted values to be read"};
+    const int k = status >> 8, w = status & 255;
+    return std::string(k >= 1 && k <= 4 ? kernels[k] : kernels[0]) + " gave up waiting for " + (w >= 1 && w <= 13 ? waits[w] : waits[0]) + " (device status " + std::to_string(status) + ")";
+}
 
 struct TcGemmParams {
     int T, K, O;
     EpiParams<__nv_bfloat16> e;
-    int* err;   // mapped host word: set to 1 when a wait ran out
+    int* err;   // mapped host word: set when a wait ran out (tg_gave_up)
     // grouped form (one matrix per expert over rows sorted by expert): blockIdx.z = group z owns rows grp[z] .. grp[z+1] of A and
     // of the output and rows z*O .. z*O+O of the weight tensor map; null: one matrix for all T rows
     const int* grp;
     int stages;   // two-SM kernel: stages of its ring
 };
 
-DN_DEVINL bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-    for (uint32_t i = 0; i < TG_SPIN_LIMIT; i++) {
+DN_DEVINL uint32_t now_ns() { uint32_t t; asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(t)); return t; }
+DN_DEVINL bool mbar_wait_for(uint64_t* bar, uint32_t parity, const volatile int* abort_flag) {
+    for (uint32_t i = 0; i < TG_LEAST_TRIES; i++) {   // (each try suspends for a while)
         if (mbar_try_wait(bar, parity)) return true;
-        if (*abort_flag) return false;
+        if (abort_flag && *abort_flag) return false;
     }
-    *abort_flag = 1;
+    const uint32_t from = now_ns();
+    do {
+        if (mbar_try_wait(bar, parity)) return true;
+        if (abort_flag && *abort_flag) return false;
+    } while (now_ns() - from < TG_WAIT_NS);
+    return false;
+}
+// `what`: the status word of a wait that runs out.  It stops the CTA's other roles
+DN_DEVINL bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int what) {
+    if (mbar_wait_for(bar, parity, abort_flag)) return true;
+    if (!*abort_flag) *abort_flag = what;
     return false;
 }
 DN_DEVINL void tg_tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
@@ -234,7 +258,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
             int issued = 0;
             for (int g = 0; g < KS; g++) {
                 const int s = g % TG_STAGES;
-                if (!mbar_wait_bounded(&empty[s], ((g / TG_STAGES) & 1) ^ 1, abort_flag)) break;
+                if (!mbar_wait_bounded(&empty[s], ((g / TG_STAGES) & 1) ^ 1, abort_flag, TG_ONE_CTA + TG_FREE)) break;
                 uint8_t* a_t = tiles + (size_t)s * TG_STAGE_BYTES;
                 mbar_expect_tx(&full[s], STAGE_TX);
                 tg_tma_load_2d(a_t, &tm_a, g * TG_KB, m0, &full[s]);
@@ -248,7 +272,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
             }
             if (*abort_flag) {   // gave up somewhere: let the copies already requested land before shared memory goes away
                 for (int g = issued > TG_STAGES ? issued - TG_STAGES : 0; g < issued; g++)
-                    for (uint32_t i = 0; i < TG_SPIN_LIMIT && !mbar_try_wait(&full[g % TG_STAGES], (g / TG_STAGES) & 1); i++) {}
+                    mbar_wait_for(&full[g % TG_STAGES], (g / TG_STAGES) & 1, nullptr);
             }
         }
     } else if (warp == 1) {
@@ -258,7 +282,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
         const uint32_t one = elect_one(), idesc = tg_idesc<BN>(), t_lo = (uint32_t)tg_desc_sw128(tiles);
         bool ok = true, landed = false;
         for (int g = 0, s = 0, round = 0; g < KS; g++) {
-            ok = landed || mbar_wait_bounded(&full[s], round & 1, abort_flag);
+            ok = landed || mbar_wait_bounded(&full[s], round & 1, abort_flag, TG_ONE_CTA + TG_FULL);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t da = t_lo + s * (TG_STAGE_BYTES >> 4), db = da + (TG_A_BYTES >> 4);   // 16 bf16 = 32 bytes along K inside the swizzle atom
@@ -280,7 +304,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
         // per row, loads of the residual batched eight rows ahead of their stores.
         const int quad = warp & 3;
         float* stg = reinterpret_cast<float*>(tiles) + (size_t)(warp - 2) * 32 * 33;
-        const bool ok = mbar_wait_bounded(tfull, 0, abort_flag);
+        const bool ok = mbar_wait_bounded(tfull, 0, abort_flag, TG_ONE_CTA + TG_SUMS);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (ok) {
 #pragma unroll 1
@@ -307,7 +331,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(BN) : "memory");
     }
-    if (threadIdx.x == 0 && *abort_flag && p.err) *p.err = 1;
+    if (threadIdx.x == 0 && *abort_flag && p.err) *p.err = *abort_flag;
 }
 
 // ---- two SMs on one tile (tcgen05 cta_group::2): prompts of more than 128 rows ----------------------------------------------------
@@ -410,7 +434,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_con
         if (lane == 0) {   // ---- TMA producer: this CTA's rows of A and of W ----
             int issued = 0;
             for (int g = g0, s = 0, round = 0; g < g1; g++) {
-                if (!mbar_wait_bounded(&empty[s], (round & 1) ^ 1, abort_flag)) break;
+                if (!mbar_wait_bounded(&empty[s], (round & 1) ^ 1, abort_flag, TG_PAIR + TG_FREE)) break;
                 uint8_t* a_t = tiles + (size_t)s * STAGE;
                 if (side == 0) mbar_expect_tx(&full[s], 2 * STAGE);   // both CTAs' bytes
                 const uint32_t bar = cluster_addr(&full[s], rank & ~1u);
@@ -422,7 +446,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_con
             }
             if (*abort_flag && side == 0) {   // gave up somewhere: let the copies already requested land before shared memory goes away
                 for (int i = issued > p.stages ? issued - p.stages : 0; i < issued; i++)
-                    for (uint32_t w = 0; w < TG_SPIN_LIMIT && !mbar_try_wait(&full[i % p.stages], (i / p.stages) & 1); w++) {}
+                    mbar_wait_for(&full[i % p.stages], (i / p.stages) & 1, nullptr);
             }
         }
     } else if (warp == 1) {
@@ -432,7 +456,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_con
             const uint16_t mask = (uint16_t)(3u << (rank & ~1u));
             bool ok = true, landed = false;
             for (int i = 0, s = 0, round = 0; i < g1 - g0; i++) {
-                ok = landed || mbar_wait_bounded(&full[s], round & 1, abort_flag);
+                ok = landed || mbar_wait_bounded(&full[s], round & 1, abort_flag, TG_PAIR + TG_FULL);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t da = t_lo + s * (STAGE >> 4), db = da + (TG_A_BYTES >> 4);
@@ -455,7 +479,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_con
     float4* recv = reinterpret_cast<float4*>(tiles + 4 * 32 * 33 * 4);   // SPLIT: the other pair's sums, [chunk][gate | up][8][row]
     bool ok = true;
     if (warp >= 2) {
-        ok = mbar_wait_bounded(tfull, 0, abort_flag);
+        ok = mbar_wait_bounded(tfull, 0, abort_flag, TG_PAIR + TG_SUMS);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     }
     if constexpr (SPLIT > 1) {
@@ -480,8 +504,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_con
     // The commits that free the last stages arrive in both CTAs, and nobody else waits for them: none may be on its way to a CTA that has left, where the
     // successor's barriers would lie.  A lane per stage, beside the epilogue: 0.2 us per product (one lane for all stages, ahead of the split form's
     // meeting or behind the epilogue: 0.6 and 1.4).
-    if (warp == 0 && mbar_wait_bounded(tfull, 0, abort_flag) && lane < min(p.stages, g1 - g0))
-        mbar_wait_bounded(&empty[lane], ((g1 - g0 - 1 - lane) / p.stages) & 1, abort_flag);
+    if (warp == 0 && mbar_wait_bounded(tfull, 0, abort_flag, TG_PAIR + TG_SUMS) && lane < min(p.stages, g1 - g0))
+        mbar_wait_bounded(&empty[lane], ((g1 - g0 - 1 - lane) / p.stages) & 1, abort_flag, TG_PAIR + TG_FREE);
     if (warp >= 2 && ok && m0 < p.T) {   // ---- epilogue: as in the kernel above, 32 x 32 blocks through the idle ring ----
         float* stg = reinterpret_cast<float*>(tiles) + (size_t)(warp - 2) * 32 * 33;
 #pragma unroll 1
@@ -526,7 +550,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_con
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(BN) : "memory");
     }
-    if (threadIdx.x == 0 && *abort_flag && p.err) *p.err = 1;
+    if (threadIdx.x == 0 && *abort_flag && p.err) *p.err = *abort_flag;
 }
 
 // ---- host side ------------------------------------------------------------------------------------------------------------
@@ -605,7 +629,7 @@ inline int dense_gemm_launch(DenseGemmCtx& c, cudaStream_t st, int T, const AT* 
         tg_init(c);
         if (!c.enc) return -1;
         if ((reinterpret_cast<uintptr_t>(a) & 15) || (reinterpret_cast<uintptr_t>(w) & 15) || (w2 && (reinterpret_cast<uintptr_t>(w2) & 15))) return -1;
-        if (*c.h_err) { err = "a tensor-core matrix product gave up waiting on one of its barriers (device status flag set)"; return 1; }
+        if (*c.h_err) { err = tg_gave_up(*c.h_err); return 1; }
         constexpr bool GLU = EPI == EPI_GLU;
         int form = GEMM_ONE_CTA;   // two-SM tiles: ungrouped products of more than 128 rows
         if (n_groups == 0 && T > 128 && (T + 255) / 256 <= 65535) {

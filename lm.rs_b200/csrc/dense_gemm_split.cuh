@@ -104,14 +104,14 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
             for (int h = h0; h < h1 && ok; h++) {
                 if (!(h & 1)) {
                     const int i = (h - h0) >> 1, s = i % x_slots;
-                    ok = mbar_wait_bounded(&x_empty[s], ((i / x_slots) & 1) ^ 1, abort_flag);
+                    ok = mbar_wait_bounded(&x_empty[s], ((i / x_slots) & 1) ^ 1, abort_flag, TG_F32 + TG_ROWS_FREE);
                     if (!ok) break;
                     mbar_expect_tx(&x_full[s], 3 * x_bytes);
                     for (int pl = 0; pl < 3; pl++) tg_tma_load_2d(x_ring + s * x_slot + pl * x_bytes, &tm_x, h * 64, pl * p.T + t0, &x_full[s]);
                     hx = h + 2;
                 }
                 const int i = h - h0, s = i % FX_W_SLOTS;
-                ok = mbar_wait_bounded(&w_empty[s], ((i / FX_W_SLOTS) & 1) ^ 1, abort_flag);
+                ok = mbar_wait_bounded(&w_empty[s], ((i / FX_W_SLOTS) & 1) ^ 1, abort_flag, TG_F32 + TG_FREE);
                 if (!ok) break;
                 mbar_expect_tx(&w_full[s], FX_W_SLOT);
                 tg_tma_load_2d(w_ring + s * FX_W_SLOT, &tm_w, h * 128, n0, &w_full[s]);
@@ -120,9 +120,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
             }
             if (*abort_flag) {   // gave up somewhere: let the copies already requested land before shared memory goes away
                 for (int i = max(0, hw - h0 - FX_W_SLOTS); i < hw - h0; i++)
-                    for (uint32_t w = 0; w < TG_SPIN_LIMIT && !mbar_try_wait(&w_full[i % FX_W_SLOTS], (i / FX_W_SLOTS) & 1); w++) {}
+                    mbar_wait_for(&w_full[i % FX_W_SLOTS], (i / FX_W_SLOTS) & 1, nullptr);
                 for (int i = max(0, ((hx - h0) >> 1) - x_slots); i < (hx - h0) >> 1; i++)
-                    for (uint32_t w = 0; w < TG_SPIN_LIMIT && !mbar_try_wait(&x_full[i % x_slots], (i / x_slots) & 1); w++) {}
+                    mbar_wait_for(&x_full[i % x_slots], (i / x_slots) & 1, nullptr);
             }
         } else if (warp == 13) {   // ---- MMA issuer ----
             const uint32_t one = elect_one();
@@ -132,9 +132,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
             uint32_t acc_small = 0;
             for (int i = 0; i < h1 - h0; i++) {
                 const int j = i >> 2, as = i & (a_slots - 1), xi = i >> 1, xs = xi % x_slots;
-                if (!(i & 3) && j >= 2) ok = mbar_wait_bounded(&d_empty[j & 1], ((j >> 1) & 1) ^ 1, abort_flag);
-                if (!(i & 1)) ok = ok && mbar_wait_bounded(&x_full[xs], (xi / x_slots) & 1, abort_flag);
-                ok = ok && (landed || mbar_wait_bounded(&a_full[as], (a_slots == 4 ? i >> 2 : i >> 1) & 1, abort_flag));
+                if (!(i & 3) && j >= 2) ok = mbar_wait_bounded(&d_empty[j & 1], ((j >> 1) & 1) ^ 1, abort_flag, TG_F32 + TG_SUMS_READ);
+                if (!(i & 1)) ok = ok && mbar_wait_bounded(&x_full[xs], (xi / x_slots) & 1, abort_flag, TG_F32 + TG_ROWS_FULL);
+                ok = ok && (landed || mbar_wait_bounded(&a_full[as], (a_slots == 4 ? i >> 2 : i >> 1) & 1, abort_flag, TG_F32 + TG_SPLIT_FULL));
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t d = tmem + (j & 1) * DN, a = tmem + a_at + as * 48;
@@ -165,7 +165,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         bool ok = true;
         for (int i = grp; i < h1 - h0 && ok; i += 2) {
             const int s = i % FX_W_SLOTS, as = i & (a_slots - 1), ai = a_slots == 4 ? i >> 2 : i >> 1;
-            ok = mbar_wait_bounded(&w_full[s], (i / FX_W_SLOTS) & 1, abort_flag);
+            ok = mbar_wait_bounded(&w_full[s], (i / FX_W_SLOTS) & 1, abort_flag, TG_F32 + TG_FULL);
             if (!ok) break;
             const uint8_t* src = w_ring + s * FX_W_SLOT + row * 128;
             float4 v[8];
@@ -180,7 +180,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
                 pl[k][0][e + 1] = y.hi; pl[k][1][e + 1] = y.mid; pl[k][2][e + 1] = y.lo;
             }
             mbar_arrive(&w_empty[s]);
-            ok = mbar_wait_bounded(&a_empty[as], (ai & 1) ^ 1, abort_flag);
+            ok = mbar_wait_bounded(&a_empty[as], (ai & 1) ^ 1, abort_flag, TG_F32 + TG_SPLIT_FREE);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
@@ -212,7 +212,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         };
         bool ok = true;
         for (int j = 0; j < c1 - c0 && ok; j++) {
-            ok = mbar_wait_bounded(&d_full[j & 1], (j >> 1) & 1, abort_flag);
+            ok = mbar_wait_bounded(&d_full[j & 1], (j >> 1) & 1, abort_flag, TG_F32 + TG_SUMS);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             add((j & 1) * DN);
@@ -296,7 +296,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(512) : "memory");
     }
-    if (threadIdx.x == 0 && *abort_flag && p.err) *p.err = 1;
+    if (threadIdx.x == 0 && *abort_flag && p.err) *p.err = *abort_flag;
 }
 
 // ---- host side ----
@@ -307,7 +307,7 @@ inline int gemm_split_launch(DenseGemmCtx& c, cudaStream_t st, const GemmTiledPa
     constexpr bool GLU = EPI == EPI_GLU;
     tg_init(c);
     if (!c.enc) return -1;
-    if (*c.h_err) { err = "a tensor-core kernel gave up waiting on one of its barriers (device status flag set)"; return 1; }
+    if (*c.h_err) { err = tg_gave_up(*c.h_err); return 1; }
     GemmSplitParams p{};
     p.T = q.T; p.K = q.K; p.O = q.O; p.N = plan.N; p.n_tiles = (q.T + plan.N - 1) / plan.N; p.splits = plan.splits;
     p.a = q.a; p.lda = q.lda; p.w = q.w; p.w2 = q.w2; p.e = q.e; p.err = c.d_err;

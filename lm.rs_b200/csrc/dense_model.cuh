@@ -485,7 +485,7 @@ template <typename AT, typename WT> class DenseModel : public ArchModel {
     int launch_attn_tensor(cudaStream_t st, AttnRowsParams<AT> p) {
         dense::tg_init(gemm_ctx);
         if (!gemm_ctx.enc) return -1;
-        if (*gemm_ctx.h_err) { error = "a tensor-core kernel gave up waiting on one of its barriers (device status flag set)"; return 1; }
+        if (*gemm_ctx.h_err) { error = dense::tg_gave_up(*gemm_ctx.h_err); return 1; }
         const int kv_mul = p.H / p.G, chunks = (kv_mul + p.HC - 1) / p.HC, pos0 = (int)p.ps.pos, dkp = attn_tensor_pad(p.dk), dvp = attn_tensor_pad(p.dv);
         p.TQ = std::max(1, AX_ROWS / p.HC);
         p.async = p.dk % 4 == 0 && p.dv % 4 == 0 && p.k_ld % 4 == 0 && p.v_ld % 4 == 0;
