@@ -1134,7 +1134,9 @@ static __global__ void __launch_bounds__(128) ssm_pre_kernel(const SsmPreParams 
     for (int j = 0; j < CONV_MAX_TAPS; j++) w[j] = j < p.taps ? p.wconv[(size_t)c * p.taps + j] : 0.0f;
     const float b = p.bconv ? p.bconv[c] : 0.0f;
     const float* in = p.in + p.c_off;
-    if (p.taps == 4) {   // the usual width: every input is loaded once, four tokens' loads ahead of their stores (1000 tokens of 6144 channels 36.8 us, 15.0 now)
+    // Four taps, the width of the models with such layers: every input is loaded once, four tokens' loads ahead of their stores.  Other widths load an input once per
+    // tap.  us, that | this: 1000 tokens of 5120 channels 36.0 | 16.8, 16 tokens 15.1 | 5.2, one 2.0 | 1.7.
+    if (p.taps == 4) {
         float v[7];
 #pragma unroll
         for (int i = 0; i < 3; i++) v[i] = conv_input(in, p.ld, p.tail, p.C, 4, t0 - 3 + i, c, pos0);
@@ -1147,8 +1149,7 @@ static __global__ void __launch_bounds__(128) ssm_pre_kernel(const SsmPreParams 
 #pragma unroll
             for (int i = 0; i < 3; i++) v[i] = v[i + 4];
         }
-    } else
-    for (int t = t0; t < t1; t++) {
+    } else for (int t = t0; t < t1; t++) {
         float a = b;
 #pragma unroll
         for (int j = 0; j < CONV_MAX_TAPS; j++)
@@ -1171,7 +1172,7 @@ static __global__ void __launch_bounds__(128) ssm_pre_kernel(const SsmPreParams 
 // that B and C entries are read with 16-byte shared-memory loads; a thread may own CPT adjacent columns, which share those reads.  Per token and row: S <- decay * S + (dt x_j) B_i, and
 // y_j += S C_i; a reduction across the lpc lanes, eight tokens at a time (block_sums), then + D x_j.  Two rows go through one instruction.  What bounds it:
 // one or two warps per scheduler that issue every 3.8 cycles, waiting for shared memory and for their own results (1000 tokens of 64 heads of 64 x 128: 251 us with a
-// reduction per token, 214 without, 171 with 16 lanes per column instead of 8, 166 with four columns per thread instead of two).  Tokens are staged DELTA_TB at a time by cp.async, the
+// reduction per token, 214 without, 171 with 16 lanes per column instead of 8, 163 with four columns per thread instead of two).  Tokens are staged DELTA_TB at a time by cp.async, the
 // next block in flight while this one is used.  The order of every sum is fixed, so a token's result does not depend on the
 // portion it arrives in.  The state is read at the start (zeros when the step starts at position 0) and written back at
 // the end.

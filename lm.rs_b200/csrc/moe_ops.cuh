@@ -205,7 +205,9 @@ DN_DEVINL float moe_combined(const MoeCombineParams& p, int t, int c, float ag =
     }
     return a;
 }
-// the sums of N columns c0, c0 + step, .. of one token: four experts' loads of all of them go out together, the additions are those of moe_combined
+// the sums of N columns c0, c0 + step, .. of one token: four experts' loads of all of them go out together, the additions are those of moe_combined.  The last
+// expert fills the places of four that there are none for; leaving those loads out is no faster.  1000 tokens of 2048 columns through the norm, us, expert after
+// expert | here: 1 chosen 20.4 | 12.4, 2 23.5 | 12.4, 4 21.9 | 12.6, 5 26.0 | 16.2, 8 38.0 | 18.7; 2 tokens, 5 chosen 11.9 | 5.4; 256 columns, 5 chosen 10.2 | 9.8.
 template <int N> DN_DEVINL void moe_combined_cols(const MoeCombineParams& p, int t, int c0, int step, float ag, float (&a)[N]) {
 #pragma unroll
     for (int i = 0; i < N; i++) { const int c = c0 + i * step; a[i] = p.add && c < p.width ? ag * p.add[(size_t)t * p.width + c] : 0.0f; }
